@@ -32,7 +32,8 @@ struct Builder {
   // FP64 -> FP32 (nearest) and FP32 -> FP64 conversions with the CvtDesc index map
   void cvt_f32(const std::vector<CvtDesc>& v);
   void widen(const std::vector<CvtDesc>& v);
-  void qr(const std::vector<QRDesc>& v);
+  // sequential: the row-sequential kernel (qr_sequential.cu)
+  void qr(const std::vector<QRDesc>& v, bool sequential = false);
   void qapply(const std::vector<QApplyDesc>& v);
   void jacobi(const std::vector<JacobiDesc>& v);
   void trunc(const std::vector<TruncDesc>& v, double tol, long long rmax);

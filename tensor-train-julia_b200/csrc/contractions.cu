@@ -410,7 +410,7 @@ void rand_rounding_general(ttc_context* c, int m, const double* alpha, const ttc
         B.gemm({gd(rh * n, s, q, Yc[j], 1, (long long)rh * n, W[j][k + 1], 1, q, Z, 1, (long long)rh * n, ws,
                    j == 0 ? 0.0 : 1.0)});
       }
-      B.qr({{rh * n, s, Z, rh * n, Q, rh * n, nullptr, 0, Tws}});
+      B.qr({{rh * n, s, Z, rh * n, Q, rh * n, nullptr, 0, Tws}}, true);
       const int yc = Y->capr(0, k);
       B.copy({cd3(Q, Y->core(0, k), rh, n, rhn, 1, rh, (long long)rh * n, 1, yc, (long long)yc * n)});
       std::vector<GemmDesc> gp, gu, gv;

@@ -189,7 +189,7 @@ void hadamard_rounding_host(ttc_context* c, int m, const ttc_ttv* ys, const int6
       double* Q = B.wd((size_t)rh * n * rhn);
       double* Tws = B.wd(qr_tws_h(rh * n, s));
       B.gemm({gd(rh * n, s, (int)R, Yc, 1, (long long)rh * n, W[k + 1], 1, R, Z, 1, (long long)rh * n, ws)});
-      B.qr({{rh * n, s, Z, rh * n, Q, rh * n, nullptr, 0, Tws}});
+      B.qr({{rh * n, s, Z, rh * n, Q, rh * n, nullptr, 0, Tws}}, true);
       const int yc = Y->capr(0, k);
       B.copy({cd3(Q, Y->core(0, k), rh, n, rhn, 1, rh, (long long)rh * n, 1, yc, (long long)yc * n)});
       // Qy[(l1, l2), rho'] = sum_{rho, z} y_k[rho, z, (l1, l2)] Q[rho, z, rho']

@@ -40,6 +40,8 @@ struct QRDesc {
 };
 constexpr int QR_MAX_M = 1536;
 void launch_qr(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, int* d_flags);
+// The same factorisation with every sum over all rows in one order (qr_sequential.cu).
+void launch_qr_seq(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, int* d_flags);
 
 // B <- Q B with Q = H_1 ... H_K the Householder factor a QR launch left in A (reflectors below
 // the diagonal, T factors in Tws): B is m x nb (ld ldb); columns >= *n_dev (when given) are

@@ -7,10 +7,9 @@
 // the sketch rank exceeds the TT rank, and zero-padded cores give exactly zero columns;
 // Householder returns an orthonormal Q for any input, like LAPACK.
 //
-// Layout: panels of NB = 16 columns are factored in shared memory (reflectors with the
-// LAPACK dlarfg convention beta = -sign(alpha)*||x||), the block reflector
-// I - V T V^T (dlarft) is applied to the trailing columns by warps that own two
-// columns each (V is read from shared memory once per pair of columns), and Q is formed
+// Layout: panels of NB = 16 columns are factored in registers (reflectors with the LAPACK dlarfg
+// convention beta = -sign(alpha)*||x||), the block reflector I - V T V^T (dlarft) is applied to
+// the trailing columns in octets of 8, several warps sharing an octet's rows, and Q is formed
 // backwards from the stored panels (dorgqr).
 //
 // One thread-block cluster of C CTAs per problem.  Every CTA factors each panel itself
@@ -18,8 +17,21 @@
 // (8o .. 8o+7) of the trailing update and of Q are owned by CTA o mod C, so a column is always
 // updated by the same CTA.  The block reflectors are applied on the FP64 tensor cores
 // (mma.sync m8n8k4).  A cluster barrier (release/acquire at cluster scope) after each
-// panel's trailing update makes the next panel visible to every CTA.  CTA 0 writes the
-// factored panels and the T factors, which the Q formation reads after one more barrier.
+// panel's trailing update makes the next panel visible to every CTA.  The CTAs write the
+// factored panel's columns in turn and CTA 0 the T factors, which the Q formation reads after one
+// more barrier.
+//
+// What bounds it: the chain of column steps (n of them, one barrier each), so a step is kept
+// short: the columns of the panel stay in registers, the reflector column is published once in
+// shared memory with its leading rows zeroed (no row masks in the dot products and updates), and
+// the scalars of a reflector (one reciprocal square root and one reciprocal, no branch) are computed
+// while the dot products are reduced.  Cycles per column step on one SM, with a square root and two
+// divisions in every warp and the columns in shared memory before: 64 rows 2020, now 790; 256 rows
+// 2290 and 1020; 512 rows 5600 and 1600.  One problem with Q: 128 x 64 126 us before and 69 now,
+// 256 x 256 530 and 320, 512 x 256 870 and 468; the QRs of a 60-TT rounding 36.7 and 24.6 ms.
+// The rest is the trailing update and the Q formation, on 8-column octets held in registers from the
+// first product to the second (read and written once; 0.33 and 0.52 of 2.5 M cycles for 512 x 256
+// before, 0.14 and 0.17 now).
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -31,47 +43,11 @@ namespace cg = cooperative_groups;
 namespace ttc {
 namespace {
 constexpr int NB = 16;
-constexpr int NT = 512;
-constexpr int NW = NT / 32;
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
-}
-
-// Block-wide sum; `red` holds NW doubles.  All threads get the result.
-__device__ double block_sum(double v, double* red) {
-  v = warp_sum(v);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  double s = 0.0;
-#pragma unroll
-  for (int i = 0; i < NW; ++i) s += red[i];
-  return s;
-}
-
-// Copy `cols` columns of `rows` doubles (one warp per column, lanes over rows, four loads in
-// flight per lane); returns whether a non-finite value was copied.
-__device__ __forceinline__ bool copy_cols(double* __restrict__ dst, long long dld, const double* __restrict__ src,
-                                          long long sld, int rows, int cols) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  bool bad = false;
-  for (int c = warp; c < cols; c += NW) {
-    const double* sc = src + (long long)c * sld;
-    double* dc = dst + (long long)c * dld;
-    for (int r0 = lane; r0 < rows; r0 += 128) {
-      double v[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) v[u] = (r0 + 32 * u < rows) ? sc[r0 + 32 * u] : 0.0;
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (r0 + 32 * u < rows) { dc[r0 + 32 * u] = v[u]; bad |= !isfinite(v[u]); }
-    }
-  }
-  return bad;
 }
 
 // D += A B on the FP64 tensor-core path (mma.sync m8n8k4): per lane a = A[lane>>2][lane&3],
@@ -82,204 +58,466 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
                : "d"(a), "d"(b));
 }
 
-// Reflector entry V[l][r] of the panel (unit diagonal and zeros above it implied).
-__device__ __forceinline__ double vref(const double* V, int mp_ld, int jb, int mp, int l, int r) {
-  if (l >= jb || r >= mp || r < l) return 0.0;
-  return (r == l) ? 1.0 : V[l * mp_ld + r];
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
+
+// Rows r and r + 1 (r even) of a column with mp rows, zero where masked; one 16-byte load when the
+// column is 16-byte aligned (vec).
+__device__ __forceinline__ void load2(double (&v)[2], const double* col, int r, int mp, bool on, bool vec) {
+  if (on && vec && r + 1 < mp) {
+    const double2 t = *reinterpret_cast<const double2*>(col + r);
+    v[0] = t.x; v[1] = t.y;
+  } else {
+    v[0] = (on && r < mp) ? col[r] : 0.0;
+    v[1] = (on && r + 1 < mp) ? col[r + 1] : 0.0;
+  }
+}
+__device__ __forceinline__ void store2(const double (&v)[2], double* col, int r, int mp, bool on, bool vec) {
+  if (on && vec && r + 1 < mp) {
+    *reinterpret_cast<double2*>(col + r) = make_double2(v[0], v[1]);
+  } else {
+    if (on && r < mp) col[r] = v[0];
+    if (on && r + 1 < mp) col[r + 1] = v[1];
+  }
+}
+__device__ __forceinline__ bool vec_ok(const double* p, int ld) {
+  return ((reinterpret_cast<uintptr_t>(p) & 15) == 0) && ((ld & 1) == 0);
 }
 
-// Apply (I - V T^T V^T) [trans=1] or (I - V T V^T) [trans=0] to columns [c_begin, c_end) of
-// the global matrix M (rows r0..m-1, ld), with V (mp x jb) in shared memory (column-major,
-// stride mp_ld = 4 mod 16 for conflict-free fragment loads) and T (jb x jb) in shared memory.
-// One warp per octet of 8 columns; octet o belongs to CTA o mod csize.  Both products run on
-// the FP64 tensor cores: W (16 x 8) = V^T C accumulated over 4-row steps, U = T^T W (or T W)
-// through a per-warp scratch Ws (16 x 8), then C -= V U per 8-row tile.
-__device__ void apply_block_reflector(double* M, int ld, int r0, int m, int c_begin, int c_end,
-                                      const double* V, int mp_ld, int jb, const double* T, bool trans,
-                                      int crank, int csize, double* Wscr) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qr = lane >> 2, qc = lane & 3;
-  const int mp = m - r0;
-  double* Ws = Wscr + warp * 128;
+// 1 / sqrt(x) for normal positive x below 2^1000: the hardware's approximation (relative error below
+// 2^-19) and one step of the third-order iteration y (1 + e/2 + 3 e^2 / 8), e = 1 - x y^2 (Householder's
+// method), whose remainder 5 e^3 / 16 is below 2^-55: four dependent operations.
+__device__ __forceinline__ double rsqrt_normal(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+// 1 / x for normal x away from the ends of the range: the hardware's approximation and y (1 + e + e^2),
+// e = 1 - x y (remainder e^3).
+__device__ __forceinline__ double rcp_normal(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
+// The reflectors V of a panel in shared memory: column l at l * panel_ld(mp), its rows in groups of
+// eight whose two halves are swapped in the columns with bit 1 of l set.  With a column stride of
+// 8 mod 16 doubles the fragment loads of both passes of apply_block meet no bank twice.  The unit
+// diagonal and the zeros above it and below row mp (to the next multiple of 8) are stored.
+__host__ __device__ __forceinline__ int panel_ld(int mp) {
+  const int r = (mp + 7) & ~7;
+  return (r & 15) ? r : r + 8;
+}
+__device__ __forceinline__ int panel_at(int l, int r, int ld) { return l * ld + (r ^ (((l >> 1) & 1) << 2)); }
+
+// Shared-memory doubles before the panel: T, the scalars, two NB x NB tables and the exchange
+// buffer of apply_block.
+template <int NW>
+constexpr int kExchange = (NW <= 8 ? 2 : 1) * NW * 128;
+template <int NW>
+constexpr int kFixed = 3 * NB * NB + 4 * NB + kExchange<NW>;
+
+// Apply (I - V T^T V^T) [trans] or (I - V T V^T) to columns [c_begin, c_end) and rows r0 .. r0 + mp - 1
+// of the global matrix M, with V (16 columns) in shared memory at p_off as above, T[col * 16 + row] at the
+// start of shared memory and the exchange buffer behind it.  G
+// warps share an octet of 8 columns, warp g its 8-row tiles g, g + G, ..., which it holds in
+// registers from the first pass to the second, so the columns are read and written once.  Both
+// passes run on the FP64 tensor cores, transposed:
+//   pass 1  W^T (8 x 16) += C^T V   (K = 4 rows of a tile at a time, rows 2 qc + s in step s)
+//   U^T = W^T T or W^T T^T, whose column order gives lane qc the entries 4 s + qc of pass 2
+//   pass 2  C^T (8 x 8 rows) -= U^T V^T
+// Rows mp must not exceed 8 G MAXT.
+template <int NW, int G, int MAXT>
+__device__ __noinline__ void apply_block_g(double* M, int ld, int r0, int mp, int c_begin, int c_end, int p_off,
+                                           bool trans, int crank, int csize) {
+  extern __shared__ __align__(16) double sm[];
+  const double* T = sm;
+  double* Wx = sm + NB * NB;
+  const double* P = sm + p_off;
+  const int mp_ld = panel_ld(mp);
+  constexpr int NG = NW / G;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, qr = lane >> 2, qc = lane & 3;
+  const int grp = warp / G, gw = warp % G;
+  const bool vec = vec_ok(M + r0, ld);
   const int o_begin = c_begin >> 3, o_end = (c_end + 7) >> 3;
   const int o_first = o_begin + ((crank - o_begin) % csize + csize) % csize;
-  for (int o = o_first + warp * csize; o < o_end; o += NW * csize) {
-    const int c0 = 8 * o;
-    // pass 1: W = V^T C; B fragment = C[r][c0 + qr]
-    const int cb = c0 + qr;
-    const bool cb_ok = (cb >= c_begin && cb < c_end);
-    const double* colb = M + (long long)(cb_ok ? cb : c_begin) * ld + r0;
-    // 32-row chunks, the next chunk's loads in flight while the current one is multiplied;
-    // even and odd k-steps accumulate into separate tiles (four independent MMA chains)
-    double w00 = 0.0, w01 = 0.0, w10 = 0.0, w11 = 0.0, x00 = 0.0, x01 = 0.0, x10 = 0.0, x11 = 0.0;
-    double ba[8], bn[8];
-    auto load8 = [&](double (&bb)[8], int k0) {
+  if (o_first + grp * csize >= o_end) return;
+  // B fragments of the U product: T[l][sigma] (trans) or T[sigma][l], l = 8 h + 2 qc + e,
+  // sigma = (qr >> 1) + 4 (qr & 1) + 8 h2
+  double tf[2][2][2];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int r = k0 + 4 * u + qc;
-        bb[u] = (cb_ok && r < mp) ? colb[r] : 0.0;
-      }
-    };
-    auto mma8 = [&](const double (&bb)[8], int k0) {
+  for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (int u = 0; u < 8; u += 2) {
-        const int r = k0 + 4 * u + qc;
-        dmma(w00, w01, vref(V, mp_ld, jb, mp, qr, r), bb[u]);
-        dmma(w10, w11, vref(V, mp_ld, jb, mp, 8 + qr, r), bb[u]);
-        dmma(x00, x01, vref(V, mp_ld, jb, mp, qr, r + 4), bb[u + 1]);
-        dmma(x10, x11, vref(V, mp_ld, jb, mp, 8 + qr, r + 4), bb[u + 1]);
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+      for (int h2 = 0; h2 < 2; ++h2) {
+        const int l = 8 * h + 2 * qc + e, sg = (qr >> 1) + 4 * (qr & 1) + 8 * h2;
+        tf[h][e][h2] = trans ? T[sg * NB + l] : T[l * NB + sg];
       }
-    };
-    load8(ba, 0);
-    for (int k0 = 0;; k0 += 64) {
-      const bool more1 = k0 + 32 < mp;
-      if (more1) load8(bn, k0 + 32);
-      mma8(ba, k0);
-      if (!more1) break;
-      const bool more2 = k0 + 64 < mp;
-      if (more2) load8(ba, k0 + 64);
-      mma8(bn, k0 + 32);
-      if (!more2) break;
+  const double* p1 = P + qr * mp_ld + ((2 * qc) ^ (((qr >> 1) & 1) << 2));   // pass 1: columns qr, qr + 8
+  const double* p2 = P + qc * mp_ld + (qr ^ (((qc >> 1) & 1) << 2));         // pass 2: columns 4 s + qc
+  int it = 0;
+  for (int o = o_first + grp * csize; o < o_end; o += NG * csize, ++it) {
+    const int c = 8 * o + qr;
+    const bool cok = (c >= c_begin && c < c_end);
+    double* col = M + (long long)(cok ? c : c_begin) * ld + r0;
+    double cc[MAXT][2];
+#pragma unroll
+    for (int t = 0; t < MAXT; ++t) load2(cc[t], col, 8 * (gw + G * t) + 2 * qc, mp, cok, vec);
+    double w[2][2][2] = {};
+#pragma unroll
+    for (int t = 0; t < MAXT; ++t) {
+      const int rt = 8 * (gw + G * t);
+      if (rt < mp) {
+        const double2 v0 = *reinterpret_cast<const double2*>(p1 + rt);
+        const double2 v1 = *reinterpret_cast<const double2*>(p1 + 8 * mp_ld + rt);
+        dmma(w[0][0][0], w[0][0][1], cc[t][0], v0.x);
+        dmma(w[1][0][0], w[1][0][1], cc[t][0], v1.x);
+        dmma(w[0][1][0], w[0][1][1], cc[t][1], v0.y);
+        dmma(w[1][1][0], w[1][1][1], cc[t][1], v1.y);
+      }
     }
-    w00 += x00; w01 += x01; w10 += x10; w11 += x11;
-    Ws[qr * 8 + 2 * qc] = w00;
-    Ws[qr * 8 + 2 * qc + 1] = w01;
-    Ws[(8 + qr) * 8 + 2 * qc] = w10;
-    Ws[(8 + qr) * 8 + 2 * qc + 1] = w11;
-    __syncwarp();
-    // U = T^T W or T W (T upper triangular); this lane needs -U[4s + qc][qr], s = 0..3
-    double ub[4];
+    double ws[2][2];
 #pragma unroll
-    for (int sidx = 0; sidx < 4; ++sidx) {
-      const int l = 4 * sidx + qc;
-      double u = 0.0;
-      if (l < jb) {
-        if (trans) {
-          for (int i = 0; i <= l; ++i) u = fma(T[l * NB + i], Ws[i * 8 + qr], u);
-        } else {
-          for (int i = l; i < jb; ++i) u = fma(T[i * NB + l], Ws[i * 8 + qr], u);
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) ws[h][e] = w[h][0][e] + w[h][1][e];
+    if (G > 1) {   // add the G partial products in the same order in every warp
+      double* X = Wx + ((NW <= 8) ? (it & 1) * NW * 128 : 0) + grp * G * 128;
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        *reinterpret_cast<double2*>(X + gw * 128 + h * 64 + lane * 2) = make_double2(ws[h][0], ws[h][1]);
+      asm volatile("bar.sync %0, %1;\n" ::"r"(1 + grp), "n"(G * 32) : "memory");
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        double2 a = *reinterpret_cast<const double2*>(X + h * 64 + lane * 2);
+#pragma unroll
+        for (int g = 1; g < G; ++g) {
+          const double2 b = *reinterpret_cast<const double2*>(X + g * 128 + h * 64 + lane * 2);
+          a.x += b.x; a.y += b.y;
         }
+        ws[h][0] = a.x; ws[h][1] = a.y;
       }
-      ub[sidx] = -u;
+      // with one buffer, every read is done before the next octet's writes
+      if (NW > 8) asm volatile("bar.sync %0, %1;\n" ::"r"(1 + grp), "n"(G * 32) : "memory");
     }
-    __syncwarp();   // Ws is rewritten for the next octet
-    // pass 2: C[rt..rt+7][c0..c0+7] -= V[rt.., 0..15] U
-    const int ca = c0 + 2 * qc;
-    const bool ok0 = (ca >= c_begin && ca < c_end), ok1 = (ca + 1 >= c_begin && ca + 1 < c_end);
-    double* col0 = M + (long long)(ok0 ? ca : c_begin) * ld + r0;
-    double* col1 = M + (long long)(ok1 ? ca + 1 : c_begin) * ld + r0;
-    // 32-row sets of four 8-row tiles, the next set's loads in flight while the current one is
-    // multiplied and stored
-    double da0[4], da1[4], dn0[4], dn1[4];
-    auto load4 = [&](double (&d0)[4], double (&d1)[4], int rt0) {
+    double u[2][2] = {};
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int r = rt0 + 8 * u + qr;
-        const bool rok = r < mp;
-        d0[u] = (ok0 && rok) ? col0[r] : 0.0;
-        d1[u] = (ok1 && rok) ? col1[r] : 0.0;
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int h2 = 0; h2 < 2; ++h2) dmma(u[h2][0], u[h2][1], ws[h][e], tf[h][e][h2]);
+#pragma unroll
+    for (int t = 0; t < MAXT; ++t) {
+      const int rt = 8 * (gw + G * t);
+      if (rt < mp) {
+#pragma unroll
+        for (int s = 0; s < 4; ++s) dmma(cc[t][0], cc[t][1], -u[s >> 1][s & 1], p2[4 * s * mp_ld + rt]);
+        store2(cc[t], col, rt + 2 * qc, mp, cok, vec);
       }
-    };
-    auto upd4 = [&](double (&d0)[4], double (&d1)[4], int rt0) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int r = rt0 + 8 * u + qr;
-#pragma unroll
-        for (int sidx = 0; sidx < 4; ++sidx) dmma(d0[u], d1[u], vref(V, mp_ld, jb, mp, 4 * sidx + qc, r), ub[sidx]);
-        if (ok0 && r < mp) col0[r] = d0[u];
-        if (ok1 && r < mp) col1[r] = d1[u];
-      }
-    };
-    load4(da0, da1, 0);
-    for (int rt0 = 0;; rt0 += 64) {
-      const bool more1 = rt0 + 32 < mp;
-      if (more1) load4(dn0, dn1, rt0 + 32);
-      upd4(da0, da1, rt0);
-      if (!more1) break;
-      const bool more2 = rt0 + 64 < mp;
-      if (more2) load4(da0, da1, rt0 + 64);
-      upd4(dn0, dn1, rt0 + 32);
-      if (!more2) break;
     }
   }
+}
+
+// Warps per octet by the panel's rows: 16 tiles of 8 rows per warp at most.
+template <int NW>
+__device__ __forceinline__ void apply_block(double* M, int ld, int r0, int mp, int c_begin, int c_end, int p_off,
+                                            bool trans, int crank, int csize) {
+  if constexpr (NW <= 8) {
+    if (mp <= 256) apply_block_g<NW, 4, 8>(M, ld, r0, mp, c_begin, c_end, p_off, trans, crank, csize);
+    else apply_block_g<NW, 4, 16>(M, ld, r0, mp, c_begin, c_end, p_off, trans, crank, csize);
+  } else {
+    if (mp <= 512) apply_block_g<NW, 8, 8>(M, ld, r0, mp, c_begin, c_end, p_off, trans, crank, csize);
+    else if (mp <= 1024) apply_block_g<NW, 8, 16>(M, ld, r0, mp, c_begin, c_end, p_off, trans, crank, csize);
+    else apply_block_g<NW, 16, 12>(M, ld, r0, mp, c_begin, c_end, p_off, trans, crank, csize);
+  }
+}
+
+// A stored panel (R in and above its diagonal, the reflectors below) into shared memory as V.
+template <int NW>
+__device__ __forceinline__ void load_panel_v(double* P, int mp_ld, const double* A, int lda, int mp, int jb) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool vec = vec_ok(A, lda);
+  const int mp8 = (mp + 7) & ~7;
+#pragma unroll
+  for (int q = 0; q < NB / NW; ++q) {
+    const int c = warp + NW * q;
+    const double* col = A + (long long)c * lda;
+    for (int b = 2 * lane; b < mp8; b += 512) {
+      double v[8][2];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) load2(v[i], col, b + 64 * i, mp, c < jb, vec);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int r = b + 64 * i;
+        if (i == 0 && r < NB) {
+          if (r <= c) v[i][0] = (r == c && c < jb) ? 1.0 : 0.0;
+          if (r + 1 <= c) v[i][1] = (r + 1 == c && c < jb) ? 1.0 : 0.0;
+        }
+        if (r < mp8) *reinterpret_cast<double2*>(P + panel_at(c, r, mp_ld)) = make_double2(v[i][0], v[i][1]);
+      }
+    }
+  }
+}
+
+// Shared-memory tables of a panel's factorisation.
+struct PanelSm {
+  double *T, *sv, *tau, *pub, *gs, *xl, *Wx, *P;
+};
+template <int NW>
+__device__ __forceinline__ PanelSm panel_sm(double* sm) {
+  PanelSm S;
+  S.T = sm;                          // NB*NB
+  S.Wx = S.T + NB * NB;              // exchange buffer of apply_block
+  S.gs = S.Wx + kExchange<NW>;       // NB*NB  x_l . x_i below row i (l < i), unscaled; then V^T V
+  S.xl = S.gs + NB * NB;             // NB*NB  x_l[i] (l < i), unscaled
+  S.sv = S.xl + NB * NB;             // NB     reflector scales 1/(alpha - beta)
+  S.tau = S.sv + NB;                 // NB
+  S.pub = S.tau + NB;                // 2*NB   alpha and squared norm below the diagonal of the published columns
+  S.P = S.pub + 2 * NB;              // panel, 16 columns of panel_ld(mp)
+  return S;
+}
+
+// The reflector of a column step from the published alpha and s = ||x||^2: with norm = ||(alpha, x)||,
+// beta = -sign(alpha) norm, v = [alpha - beta; x] and g = |alpha| + norm, H = I - v v^T / (norm g), that
+// is c -= ws v with ws = (v^T c) rn rg.  H = I (nz false) when x = 0 or the squared norm is subnormal
+// (a column of norm below 2e-154, whose square would carry no digits).
+struct Reflector {
+  double alpha, norm, rn, rg;
+  bool nz;
+  __device__ __forceinline__ explicit Reflector(double2 as) {
+    const double n2 = fma(as.x, as.x, as.y);
+    alpha = as.x;
+    nz = as.y != 0.0 && n2 >= 2.2250738585072014e-308;
+    rn = rsqrt_normal(n2);
+    norm = n2 * rn;
+    rg = rcp_normal(fabs(as.x) + norm);
+  }
+  __device__ __forceinline__ double u() const { return copysign(fabs(alpha) + norm, alpha); }        // alpha - beta
+  __device__ __forceinline__ double tau() const { return nz ? fma(fabs(alpha), rn, 1.0) : 0.0; }     // (beta - alpha) / beta
+  __device__ __forceinline__ double scale() const { return nz ? copysign(rg, alpha) : 0.0; }         // 1 / (alpha - beta)
+  __device__ __forceinline__ double beta() const { return nz ? -copysign(norm, alpha) : alpha; }
+};
+
+// T from the products gs, xl and the scales, by one warp.  G = V^T V (l < i): v_l[i] = scal_l x_l[i],
+// v_i[i] = 1, rows below i scaled by both.  T forward (dlarft): T[r][l] = -tau_l sum_{r <= k < l} T[r][k]
+// G[k][l], T[l][l] = tau_l; lane r holds row r and adds T[r][l] G[l][j] to every later column's sum at
+// once.  Loads, chain and stores are kept apart, so that no load waits for a store.
+template <int NW>
+__device__ __forceinline__ void form_t(const PanelSm& S, int jb, double* Tg) {
+  const int lane = threadIdx.x & 31, r = lane & 15;
+  double a[NB];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int e = lane + 32 * k, l = e >> 4, i = e & 15;
+    a[k] = (l < i && i < jb) ? S.sv[l] * fma(S.sv[i], S.gs[e], S.xl[e]) : 0.0;
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) S.gs[lane + 32 * k] = a[k];
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < NB; ++j) a[j] = 0.0;
+  double2 g[NB / 2], gn[NB / 2];
+  const double2* gr = reinterpret_cast<const double2*>(S.gs);
+#pragma unroll
+  for (int k = 0; k < NB / 2; ++k) g[k] = gr[k];
+  double tl = S.tau[0];
+#pragma unroll
+  for (int l = 0; l < NB; ++l) {
+    double tn = 0.0;
+    if (l + 1 < NB) {                          // row l + 1 while row l is used
+      tn = S.tau[l + 1];
+#pragma unroll
+      for (int k = (l + 2) / 2; k < NB / 2; ++k) gn[k] = gr[(l + 1) * (NB / 2) + k];
+    }
+    a[l] = (r == l) ? tl : (r < l ? -tl * a[l] : 0.0);
+#pragma unroll
+    for (int j = l + 1; j < NB; ++j) a[j] = fma(a[l], (j & 1) ? g[j / 2].y : g[j / 2].x, a[j]);
+#pragma unroll
+    for (int k = 0; k < NB / 2; ++k) g[k] = gn[k];
+    tl = tn;
+  }
+  if (lane < NB) {
+#pragma unroll
+    for (int l = 0; l < NB; ++l) S.T[l * NB + r] = a[l];
+    if (Tg) {
+#pragma unroll
+      for (int l = 0; l < NB; ++l) Tg[l * NB + r] = a[l];
+    }
+  }
+}
+
+// One panel: A points at its first diagonal entry, mp rows, jb <= 16 columns.  A column belongs to LPC
+// lanes of a warp, lane hl holding its rows 2 LPC i + 2 hl + {0, 1} in registers (mp <= 2 LPC RI); a
+// warp has CW adjacent columns, side by side (LPC = 32 / CW) or CPW to a lane (LPC = 32).
+// Column step jj: the reflector column x = column jj below row jj lies in shared memory, zero in the
+// rows <= jj and beyond mp, with its squared norm and alpha.  Every column forms x . c; the columns
+// c > jj then take the reflector (x unscaled), for c < jj the product is an entry of V^T V.  The warp of
+// column jj + 1 publishes that column and its squared norm.  The reflectors are scaled, and T formed,
+// after the last step.
+template <int NW, int LPC, int RI>
+__device__ __noinline__ bool factor_panel(double* A, int lda, int mp, int jb, int crank, int csize, double* Tws) {
+  extern __shared__ __align__(16) double sm[];
+  const PanelSm S = panel_sm<NW>(sm);
+  const int mp_ld = panel_ld(mp);
+  constexpr int CW = NB / NW, CPW = CW * LPC / 32, CH = 2 * LPC, XLD = CH * RI;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, hl = lane & (LPC - 1);
+  const int c0 = warp * CW + lane / LPC;      // column q of this lane: c0 + q
+  const bool vec = vec_ok(A, lda);
+  double* X = S.P;                            // two published columns (the panel region is free until the end)
+  double cr[CPW][RI][2];
+#pragma unroll
+  for (int q = 0; q < CPW; ++q)
+#pragma unroll
+    for (int i = 0; i < RI; ++i)
+      load2(cr[q][i], A + (long long)(c0 + q) * lda, CH * i + 2 * hl, mp, c0 + q < jb, vec);
+  int hi = 0;
+#pragma unroll
+  for (int q = 0; q < CPW; ++q)
+#pragma unroll
+    for (int i = 0; i < RI; ++i)
+      hi = max(hi, max(__double2hiint(cr[q][i][0]) & 0x7fffffff, __double2hiint(cr[q][i][1]) & 0x7fffffff));
+  __syncwarp();
+  cluster_arrive();                           // this CTA has read the panel (waited for before it is overwritten)
+
+  // column j = c0 + q of some lanes of this warp
+  auto publish = [&](const double (&v)[RI][2], int j, bool me) {
+    double* x = X + (j & 1) * XLD + 2 * hl;
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    {
+      const int r = 2 * hl;
+      const double v0 = (r > j) ? v[0][0] : 0.0, v1 = (r + 1 > j) ? v[0][1] : 0.0;
+      if (me) *reinterpret_cast<double2*>(x) = make_double2(v0, v1);
+      if (me && hl < NB / 2) *reinterpret_cast<double2*>(S.xl + j * NB + 2 * hl) = make_double2(v0, v1);
+      a[0] = v0 * v0; a[1] = v1 * v1;
+    }
+#pragma unroll
+    for (int i = 1; i < RI; ++i) {
+      if (me) *reinterpret_cast<double2*>(x + CH * i) = make_double2(v[i][0], v[i][1]);
+      a[2 * (i & 1)] = fma(v[i][0], v[i][0], a[2 * (i & 1)]);
+      a[2 * (i & 1) + 1] = fma(v[i][1], v[i][1], a[2 * (i & 1) + 1]);
+    }
+    double s = RI > 1 ? (a[0] + a[1]) + (a[2] + a[3]) : a[0] + a[1];
+#pragma unroll
+    for (int o = LPC / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (me && hl == (j >> 1)) *reinterpret_cast<double2*>(S.pub + 2 * j) = make_double2((j & 1) ? v[0][1] : v[0][0], s);
+  };
+  if (warp == 0) publish(cr[0], 0, c0 == 0);
+
+  // unrolled by two (the parity of jj is then fixed): in full, the loop outgrows the instruction cache
+#pragma unroll 2
+  for (int jj = 0; jj < NB; ++jj) {
+    if (jj >= jb) break;
+    __syncthreads();
+    const double* x = X + (jj & 1) * XLD + 2 * hl;
+    const double2 as = *reinterpret_cast<const double2*>(S.pub + 2 * jj);
+    constexpr bool KEEP = (1 + CPW) * RI <= 16;   // x stays in registers from the product to the update
+    double xr[KEEP ? RI : 1][2];
+    double acc[CPW][4] = {};
+#pragma unroll
+    for (int i = 0; i < RI; ++i) {
+      if (!KEEP && i > 0 && i % 4 == 0) asm volatile("" ::: "memory");   // bounds the loads hoisted at once
+      const double2 t = *reinterpret_cast<const double2*>(x + CH * i);
+      if (KEEP) { xr[i][0] = t.x; xr[i][1] = t.y; }
+#pragma unroll
+      for (int q = 0; q < CPW; ++q) {
+        acc[q][2 * (i & 1)] = fma(t.x, cr[q][i][0], acc[q][2 * (i & 1)]);
+        acc[q][2 * (i & 1) + 1] = fma(t.y, cr[q][i][1], acc[q][2 * (i & 1) + 1]);
+      }
+    }
+    double d[CPW];
+#pragma unroll
+    for (int q = 0; q < CPW; ++q)
+      d[q] = RI > 1 ? (acc[q][0] + acc[q][1]) + (acc[q][2] + acc[q][3]) : acc[q][0] + acc[q][1];
+    const Reflector H(as);                    // the scalars, without branches, beside the reduction of the products
+#pragma unroll
+    for (int o = LPC / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int q = 0; q < CPW; ++q) d[q] += __shfl_xor_sync(0xffffffffu, d[q], o);
+#pragma unroll
+    for (int q = 0; q < CPW; ++q)
+      if (c0 + q < jj && hl == 0) S.gs[(c0 + q) * NB + jj] = d[q];
+    if (warp * CW + CW - 1 > jj) {            // a column of this warp is not finished
+      const double u = H.u(), rr = H.rn * H.rg;
+#pragma unroll
+      for (int q = 0; q < CPW; ++q) {
+        const int c = c0 + q;
+        const double cj = __shfl_sync(0xffffffffu, (jj & 1) ? cr[q][0][1] : cr[q][0][0], (lane & ~(LPC - 1)) | (jj >> 1));
+        const bool on = c > jj && H.nz;
+        const double ws = on ? rr * fma(u, cj, d[q]) : 0.0;
+#pragma unroll
+        for (int i = 0; i < RI; ++i) {
+          if (!KEEP && i % 4 == 0) asm volatile("" ::: "memory");
+          double x0, x1;
+          if (KEEP) { x0 = xr[i][0]; x1 = xr[i][1]; }
+          else {
+            const double2 t2 = *reinterpret_cast<const double2*>(x + CH * i);
+            x0 = t2.x; x1 = t2.y;
+          }
+          cr[q][i][0] = fma(-ws, x0, cr[q][i][0]);
+          cr[q][i][1] = fma(-ws, x1, cr[q][i][1]);
+        }
+        if (on && hl == (jj >> 1)) {
+          const double w = fma(-ws, u, cj);
+          if (jj & 1) cr[q][0][1] = w; else cr[q][0][0] = w;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < CPW; ++q)
+        if (warp == (jj + 1) / CW && jj + 1 < jb && (CPW == 1 || c0 + q == jj + 1))
+          publish(cr[q], jj + 1, CPW > 1 || c0 == jj + 1);
+    }
+  }
+  __syncthreads();
+  cluster_wait();                             // every CTA holds the panel: it may be overwritten
+  double sc[CPW], bc[CPW];
+#pragma unroll
+  for (int q = 0; q < CPW; ++q) {
+    const int c = c0 + q;
+    const Reflector H(*reinterpret_cast<const double2*>(S.pub + 2 * min(c, jb - 1)));
+    sc[q] = (c < jb) ? H.scale() : 0.0;
+    bc[q] = H.beta();
+    if (hl == 0) { S.sv[c] = sc[q]; S.tau[c] = (c < jb) ? H.tau() : 0.0; }
+  }
+  __syncthreads();
+  const int mp8 = (mp + 7) & ~7;
+#pragma unroll
+  for (int q = 0; q < CPW; ++q) {
+    const int c = c0 + q;
+    const bool own = c < jb, out = own && (c % csize == crank);
+#pragma unroll
+    for (int i = 0; i < RI; ++i) {
+      const int r = CH * i + 2 * hl;
+      double v[2], g[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        v[e] = cr[q][i][e] * sc[q];
+        g[e] = v[e];
+        if (i == 0 && r + e <= c) {           // on and above the diagonal: R in global memory, V in the panel
+          g[e] = (r + e == c) ? bc[q] : cr[q][i][e];
+          v[e] = (r + e == c && own) ? 1.0 : 0.0;
+        }
+      }
+      if (r < mp8) *reinterpret_cast<double2*>(S.P + panel_at(c, r, mp_ld)) = make_double2(v[0], v[1]);
+      store2(g, A + (long long)c * lda, r, mp, out, vec);
+    }
+  }
+  if (warp == 0) form_t<NW>(S, jb, (crank == 0) ? Tws : nullptr);   // its columns' registers are free by now
+  __syncthreads();
+  return hi >= 0x7ff00000;
 }
 }  // namespace
 
-// Column steps of a panel held in registers (panel rows mp <= 32 * RMAX): warp w keeps panel
-// column (w + 1) mod NW, lane l its rows l + 32 i, for the whole panel.  Step jj reads only the
-// reflector column x = P[:, jj] and its diagonal from shared memory: the warps of the columns
-// c > jj apply reflector jj to their column (x unscaled, as in the shared-memory loop below),
-// the warps of the finished columns c < jj form x_c . x_jj below row jj for V^T V, and the warp
-// of column jj + 1 returns its squared norm below the diagonal and publishes the column to P,
-// where it is the next step's reflector.  Every column reaches P at the step that finishes it.
-template <int RMAX>
-__device__ __forceinline__ void panel_steps_regs(double* P, int mp, int mp_ld, int jb, double* nrm2, double* tau,
-                                                 double* sv, double* bet, double* gs) {
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int c = (warp + 1) % NW;
-  const bool own = c < jb;
-  double* pc = P + c * mp_ld;
-  double cr[RMAX];
-#pragma unroll
-  for (int i = 0; i < RMAX; ++i) {
-    const int r = lane + 32 * i;
-    cr[i] = (own && r < mp) ? pc[r] : 0.0;
-  }
-  for (int jj = 0; jj < jb; ++jj) {
-    const double s = nrm2[jj & 1];
-    const double alpha = P[jj * mp_ld + jj];
-    double beta, t, scal;
-    if (s == 0.0) { t = 0.0; beta = alpha; scal = 0.0; }
-    else {
-      beta = -copysign(sqrt(fma(alpha, alpha, s)), alpha);
-      t = (beta - alpha) / beta;
-      scal = 1.0 / (alpha - beta);
-    }
-    const double* x = P + jj * mp_ld;
-    if (own && c != jj) {
-      double dd[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-      for (int i = 0; i < RMAX; ++i) {
-        const int r = lane + 32 * i;
-        const double xv = (r > jj && r < mp) ? x[r] : 0.0;
-        dd[i & 3] = fma(xv, cr[i], dd[i & 3]);
-      }
-      const double d = warp_sum((dd[0] + dd[1]) + (dd[2] + dd[3]));
-      if (c < jj) {
-        if (lane == 0) gs[c * NB + jj] = d;
-      } else {
-        const double cj = __shfl_sync(0xffffffffu, cr[0], jj);   // row jj < 32: lane jj, i = 0
-        const double w = fma(scal, d, cj) * t;                   // tau v^T c
-        const double ws = w * scal;
-        double qq[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-        for (int i = 0; i < RMAX; ++i) {
-          const int r = lane + 32 * i;
-          if (r > jj && r < mp) {
-            cr[i] = fma(-ws, x[r], cr[i]);
-            if (r > jj + 1) qq[i & 3] = fma(cr[i], cr[i], qq[i & 3]);
-          }
-        }
-        if (lane == jj) cr[0] = cj - w;
-        if (c == jj + 1) {
-          const double q = warp_sum((qq[0] + qq[1]) + (qq[2] + qq[3]));
-          if (lane == 0) nrm2[(jj + 1) & 1] = q;
-#pragma unroll
-          for (int i = 0; i < RMAX; ++i) {
-            const int r = lane + 32 * i;
-            if (r < mp) pc[r] = cr[i];
-          }
-        }
-      }
-    }
-    if (tid == 0) { tau[jj] = t; sv[jj] = scal; bet[jj] = beta; }
-    __syncthreads();
-  }
-}
-
 // T layout in shared memory: T[col * NB + row] (upper triangular).
-__global__ void __launch_bounds__(NT, 1) householder_qr_kernel(const QRDesc* __restrict__ descs, int csize, int* flags) {
-  extern __shared__ double sm[];
+template <int NW>
+__global__ void __launch_bounds__(NW * 32, NW <= 8 ? 2 : 1)
+    householder_qr_kernel(const QRDesc* __restrict__ descs, int csize, int* flags) {
+  extern __shared__ __align__(16) double sm[];
   cg::cluster_group cluster = cg::this_cluster();
   const int crank = (int)cluster.block_rank();
   const QRDesc D = descs[blockIdx.x / csize];
@@ -288,157 +526,41 @@ __global__ void __launch_bounds__(NT, 1) householder_qr_kernel(const QRDesc* __r
   // R (Kc x D.n) and Q (D.m x Kc)
   const int m = dev_bound(D.m, D.m_dev, D.m_mult), n = dev_bound(D.n, D.n_dev, D.n_mult);
   const int K = min(m, n), Kc = min(D.m, D.n);
-  double* T = sm;                    // NB*NB
-  double* tau = T + NB * NB;         // NB
-  double* red = tau + NB;            // NW
-  double* sv = red + NW;             // NB   reflector scales 1/(alpha - beta)
-  double* bet = sv + NB;             // NB   betas (diagonal of R)
-  double* nrm2 = bet + NB;           // 2    squared norm below the diagonal of the next column
-  double* gs = nrm2 + 2;             // NB*NB  x_l . x_i below row i (l < i), unscaled
-  double* xl_i = gs + NB * NB;       // NB*NB  x_l[i] (l < i), unscaled
-  double* G = xl_i + NB * NB;        // NB*NB  (V^T V)
-  double* Wscr = G + NB * NB;        // NW*128  per-warp 16 x 8 scratch of the reflector products
-  double* P = Wscr + NW * 128;       // panel, (mp_ld x NB), mp_ld = 4 mod 16
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const PanelSm S = panel_sm<NW>(sm);
+  const int tid = threadIdx.x;
   double* A = D.A;
   const int lda = D.lda;
   bool nonfinite = false;
 
   for (int j0 = 0; j0 < K; j0 += NB) {
-    const int jb = min(NB, K - j0);
-    const int mp = m - j0;
-    const int mp_ld = mp + ((4 - mp) & 15);
-    // 1. load panel
-    nonfinite |= copy_cols(P, mp_ld, A + (long long)j0 * lda + j0, lda, mp, jb);
-    __syncthreads();
-    // 2. factor panel, one CTA barrier per column: reflector jj (dlarfg: beta =
-    //    -sign(alpha) ||(alpha, x)||, tau = (beta - alpha)/beta, v = [1; x/(alpha - beta)]) is
-    //    applied to columns c > jj with x unscaled; the warp that updates column jj+1 also
-    //    returns its squared norm below the diagonal for the next reflector.  The reflector
-    //    columns are scaled, and the betas stored, after the loop.
-    {
-      double s0 = 0.0;
-      for (int r = 1 + tid; r < mp; r += NT) { const double x = P[r]; s0 = fma(x, x, s0); }
-      s0 = block_sum(s0, red);
-      if (tid == 0) nrm2[0] = s0;
-      __syncthreads();
+    const int jb = min(NB, K - j0), mp = m - j0;
+    double* Ap = A + (long long)j0 * lda + j0;
+    double* Tws = D.Tws ? D.Tws + (j0 / NB) * NB * NB : nullptr;
+    // registers per lane for the panel's own row count (uniform across the cluster)
+    if constexpr (NW <= 8) {
+      if (mp <= 64) nonfinite |= factor_panel<NW, 16, 2>(Ap, lda, mp, jb, crank, csize, Tws);
+      else if (mp <= 128) nonfinite |= factor_panel<NW, 16, 4>(Ap, lda, mp, jb, crank, csize, Tws);
+      else if (mp <= 256) nonfinite |= factor_panel<NW, 32, 4>(Ap, lda, mp, jb, crank, csize, Tws);
+      else nonfinite |= factor_panel<NW, 32, 8>(Ap, lda, mp, jb, crank, csize, Tws);
+    } else {
+      if (mp <= 128) nonfinite |= factor_panel<NW, 32, 2>(Ap, lda, mp, jb, crank, csize, Tws);
+      else if (mp <= 256) nonfinite |= factor_panel<NW, 32, 4>(Ap, lda, mp, jb, crank, csize, Tws);
+      else if (mp <= 512) nonfinite |= factor_panel<NW, 32, 8>(Ap, lda, mp, jb, crank, csize, Tws);
+      else if (mp <= 1024) nonfinite |= factor_panel<NW, 32, 16>(Ap, lda, mp, jb, crank, csize, Tws);
+      else nonfinite |= factor_panel<NW, 32, 24>(Ap, lda, mp, jb, crank, csize, Tws);
     }
-    // the panel's own row count picks the column-step routine (uniform across the cluster):
-    // registers up to 512 rows, else the shared-memory loop below (the register column and the
-    // loads in flight no longer fit 128 registers at 24 rows per lane)
-    if (mp <= 256) panel_steps_regs<8>(P, mp, mp_ld, jb, nrm2, tau, sv, bet, gs);
-    else if (mp <= 512) panel_steps_regs<16>(P, mp, mp_ld, jb, nrm2, tau, sv, bet, gs);
-    else for (int jj = 0; jj < jb; ++jj) {
-      const double s = nrm2[jj & 1];
-      const double alpha = P[jj * mp_ld + jj];
-      double beta, t, scal;
-      if (s == 0.0) { t = 0.0; beta = alpha; scal = 0.0; }
-      else {
-        beta = -copysign(sqrt(fma(alpha, alpha, s)), alpha);
-        t = (beta - alpha) / beta;
-        scal = 1.0 / (alpha - beta);
-      }
-      const double* x = P + jj * mp_ld;
-      // slot k of warp k mod NW: column k < jj gives x_k . x_jj below row jj (for V^T V),
-      // column k + 1 > jj gets the reflector
-      for (int k = warp; k < jb - 1; k += NW) {
-        if (k < jj) {
-          const double* pl = P + k * mp_ld;
-          double g = 0.0, g2 = 0.0;
-          for (int r = jj + 1 + lane; r < mp; r += 64) {
-            g = fma(pl[r], x[r], g);
-            if (r + 32 < mp) g2 = fma(pl[r + 32], x[r + 32], g2);
-          }
-          g = warp_sum(g + g2);
-          if (lane == 0) gs[k * NB + jj] = g;
-          continue;
-        }
-        const int c = k + 1;
-        double* pc = P + c * mp_ld;
-        const double cj = pc[jj];
-        double d = 0.0, d2 = 0.0;       // two chains
-        for (int r = jj + 1 + lane; r < mp; r += 64) {
-          d = fma(x[r], pc[r], d);
-          if (r + 32 < mp) d2 = fma(x[r + 32], pc[r + 32], d2);
-        }
-        d = warp_sum(d + d2);
-        const double w = fma(scal, d, cj) * t;     // tau v^T c
-        const double ws = w * scal;
-        double q = 0.0, q2 = 0.0;
-        for (int r = jj + 1 + lane; r < mp; r += 64) {
-          const double u = fma(-ws, x[r], pc[r]);
-          pc[r] = u;
-          if (r > jj + 1) q = fma(u, u, q);
-          if (r + 32 < mp) {
-            const double u2 = fma(-ws, x[r + 32], pc[r + 32]);
-            pc[r + 32] = u2;
-            q2 = fma(u2, u2, q2);
-          }
-        }
-        q += q2;
-        if (c == jj + 1) {
-          q = warp_sum(q);
-          if (lane == 0) nrm2[(jj + 1) & 1] = q;
-        }
-        if (lane == 0) pc[jj] = cj - w;
-      }
-      if (tid == 0) { tau[jj] = t; sv[jj] = scal; bet[jj] = beta; }
-      __syncthreads();
-    }
-    for (int e = tid; e < NB * NB; e += NT) {        // unscaled x_l[i] for V^T V
-      const int i = e / NB, l = e - i * NB;
-      if (l < i && i < jb) xl_i[l * NB + i] = P[l * mp_ld + i];
-    }
-    __syncthreads();
-    for (int c = warp; c < jb; c += NW) {
-      double* pc = P + c * mp_ld;
-      const double sc = sv[c];
-      for (int r = c + 1 + lane; r < mp; r += 32) pc[r] *= sc;
-      if (lane == 0) pc[c] = bet[c];
-    }
-    __syncthreads();
-    // 3. T factor.  G = V^T V (l < i) from the dot products of the panel loop:
-    //    v_l[i] = scal_l x_l[i], v_i[i] = 1, rows below i scaled by both (x unscaled there);
-    //    then T from T^{-1} + T^{-T} = V^T V (compact WY): T^{-1} = striu(G) + diag(1/tau), so
-    //    T[r][j] = -tau_r sum_{r < l <= j} G[r][l] T[l][j], T[j][j] = tau_j; lane j of warp 0
-    //    back-substitutes column j in registers (a zero tau gives a zero row, as in dlarft).
-    for (int e = tid; e < NB * NB; e += NT) {
-      const int i = e / NB, l = e - i * NB;
-      if (l < i) G[i * NB + l] = (i < jb) ? sv[l] * fma(sv[i], gs[l * NB + i], xl_i[l * NB + i]) : 0.0;
-    }
-    __syncthreads();
-    if (warp == 0 && lane < NB) {
-      const int j = lane;
-      double tc[NB];
-#pragma unroll
-      for (int k = 0; k < NB; ++k) tc[k] = (k == j && j < jb) ? tau[k] : 0.0;
-#pragma unroll
-      for (int r = NB - 2; r >= 0; --r) {
-        double a2 = 0.0;
-#pragma unroll
-        for (int l = r + 1; l < NB; ++l) a2 = fma(G[l * NB + r], tc[l], a2);
-        if (r < j && j < jb) tc[r] = -tau[r] * a2;
-      }
-#pragma unroll
-      for (int k = 0; k < NB; ++k) T[j * NB + k] = tc[k];
-    }
-    __syncthreads();
-    // 4. trailing update with H^T = I - V T^T V^T (this CTA's column octets)
-    if (j0 + jb < n) apply_block_reflector(A, lda, j0, m, j0 + jb, n, P, mp_ld, jb, T, true, crank, csize, Wscr);
-    // 5. CTA 0 writes back the panel and keeps T
-    if (crank == 0) {
-      copy_cols(A + (long long)j0 * lda + j0, lda, P, mp_ld, mp, jb);
-      if (D.Tws)
-        for (int e = tid; e < NB * NB; e += NT) D.Tws[(j0 / NB) * NB * NB + e] = T[e];
-    }
-    cluster.sync();   // trailing columns and the panel visible to every CTA
+    // trailing update with H^T = I - V T^T V^T (this CTA's column octets)
+    if (j0 + jb < n) apply_block<NW>(A, lda, j0, mp, j0 + jb, n, (int)(S.P - sm), true, crank, csize);
+    __syncwarp();
+    cluster_arrive();   // trailing columns and the panel visible to every CTA
+    cluster_wait();
   }
-  if (nonfinite && crank == 0 && threadIdx.x == 0) atomicOr(flags, DFLAG_NONFINITE);
+  if (nonfinite && crank == 0) atomicOr(flags, DFLAG_NONFINITE);
 
   // R = upper triangle of A[0:Kc, 0:D.n] (zero outside the factored block)
   if (D.R) {
-    for (int j = (int)(threadIdx.x >> 5) + NW * crank; j < D.n; j += NW * csize)
-      for (int i = (int)(threadIdx.x & 31); i < Kc; i += 32) {
+    for (int j = (tid >> 5) + NW * crank; j < D.n; j += NW * csize)
+      for (int i = tid & 31; i < Kc; i += 32) {
         const double v = (i <= j) ? A[(long long)j * lda + i] : 0.0;
         if (D.r_trans) D.R[(long long)i * D.ldr + j] = v;
         else D.R[(long long)j * D.ldr + i] = v;
@@ -450,95 +572,103 @@ __global__ void __launch_bounds__(NT, 1) householder_qr_kernel(const QRDesc* __r
   // and updates only its own column octets, so the panels need no barrier between them.
   // The reflectors act on rows < m; identity columns c >= K are untouched unless a column
   // bound leaves some of them with c < m.
-  for (int c = 0; c < Kc; ++c) {
+  for (int c = tid >> 5; c < Kc; c += NW) {
     if (((c >> 3) % csize) != crank) continue;
-    for (int i = tid; i < D.m; i += NT) D.Q[(long long)c * D.ldq + i] = (i == c) ? 1.0 : 0.0;
+    for (int i = tid & 31; i < D.m; i += 32) D.Q[(long long)c * D.ldq + i] = (i == c) ? 1.0 : 0.0;
   }
-  __syncthreads();
   const int qc_end = (n < D.n) ? Kc : K;
   const int npan = (K + NB - 1) / NB;
   for (int p = npan - 1; p >= 0; --p) {
-    const int j0 = p * NB, jb = min(NB, K - j0), mp = m - j0, mp_ld = mp + ((4 - mp) & 15);
-    copy_cols(P, mp_ld, A + (long long)j0 * lda + j0, lda, mp, jb);
-    for (int e = tid; e < NB * NB; e += NT) T[e] = D.Tws[p * NB * NB + e];
+    const int j0 = p * NB, jb = min(NB, K - j0), mp = m - j0, mp_ld = panel_ld(mp);
+    __syncthreads();    // the identity columns, then the previous panel's products
+    load_panel_v<NW>(S.P, mp_ld, A + (long long)j0 * lda + j0, lda, mp, jb);
+    for (int e = tid; e < NB * NB; e += NW * 32) S.T[e] = D.Tws[p * NB * NB + e];
     __syncthreads();
-    apply_block_reflector(D.Q, D.ldq, j0, m, j0, qc_end, P, mp_ld, jb, T, false, crank, csize, Wscr);
-    __syncthreads();
+    apply_block<NW>(D.Q, D.ldq, j0, mp, j0, qc_end, (int)(S.P - sm), false, crank, csize);
   }
 }
 
 // B <- Q B from the stored panels, backwards (as the Q formation, but from B instead of the
 // identity and over all its columns).  CTA problem / csize owns the column octets o with
 // o mod csize == CTA rank; the panels are only read, so no CTA waits for another.
-__global__ void __launch_bounds__(NT, 1) householder_apply_q_kernel(const QApplyDesc* __restrict__ descs, int csize) {
-  extern __shared__ double sm[];
+template <int NW>
+__global__ void __launch_bounds__(NW * 32, NW <= 8 ? 2 : 1)
+    householder_apply_q_kernel(const QApplyDesc* __restrict__ descs, int csize) {
+  extern __shared__ __align__(16) double sm[];
   const int crank = (int)(blockIdx.x % csize);
   const QApplyDesc D = descs[blockIdx.x / csize];
   const int m = dev_bound(D.m, D.m_dev, D.m_mult), K = min(D.K, m);   // H_k = I for k >= m
   if (m <= 0 || K <= 0 || D.nb <= 0) return;
   const int nb = D.n_dev ? min(D.nb, *D.n_dev) : D.nb;
   if (nb <= 0) return;
-  double* T = sm;                    // NB*NB
-  double* Wscr = T + NB * NB;        // NW*128
-  double* P = Wscr + NW * 128;       // panel, (mp_ld x NB)
+  double* T = sm;                                  // NB*NB, then the exchange buffer of apply_block
+  double* P = T + NB * NB + kExchange<NW>;         // panel
   const int tid = threadIdx.x;
   const int npan = (K + NB - 1) / NB;
   for (int p = npan - 1; p >= 0; --p) {
-    const int j0 = p * NB, jb = min(NB, K - j0), mp = m - j0, mp_ld = mp + ((4 - mp) & 15);
-    copy_cols(P, mp_ld, D.A + (long long)j0 * D.lda + j0, D.lda, mp, jb);
-    for (int e = tid; e < NB * NB; e += NT) T[e] = D.Tws[p * NB * NB + e];
+    const int j0 = p * NB, jb = min(NB, K - j0), mp = m - j0, mp_ld = panel_ld(mp);
     __syncthreads();
-    apply_block_reflector(D.B, D.ldb, j0, m, 0, nb, P, mp_ld, jb, T, false, crank, csize, Wscr);
+    load_panel_v<NW>(P, mp_ld, D.A + (long long)j0 * D.lda + j0, D.lda, mp, jb);
+    for (int e = tid; e < NB * NB; e += NW * 32) T[e] = D.Tws[p * NB * NB + e];
     __syncthreads();
+    apply_block<NW>(D.B, D.ldb, j0, mp, 0, nb, (int)(P - sm), false, crank, csize);
   }
 }
 
-void launch_qr_apply(const QApplyDesc* d_descs, int count, int max_m, cudaStream_t s) {
-  if (count <= 0) return;
-  TTC_REQUIRE(max_m <= QR_MAX_M, TTC_EDIM, "qr apply: row count exceeds the supported maximum (1536)");
-  const size_t smem = sizeof(double) * (NB * NB + NW * 128 + (size_t)(max_m + 15) * NB);
+namespace {
+// Rows up to which the eight-warp kernels (two CTAs per SM) hold a panel's registers and tiles.
+constexpr int kSmallM = 512;
+
+template <int NW>
+size_t qr_smem(int max_m) {
+  return sizeof(double) * (kFixed<NW> + (size_t)NB * panel_ld(std::max(max_m, 1)));
+}
+template <int NW>
+size_t qr_apply_smem(int max_m) {
+  return sizeof(double) * (NB * NB + kExchange<NW> + (size_t)NB * panel_ld(std::max(max_m, 1)));
+}
+
+template <int NW>
+void launch_qr_apply_t(const QApplyDesc* d_descs, int count, int max_m, cudaStream_t s) {
+  constexpr int lim = NW <= 8 ? kSmallM : QR_MAX_M;
+  const size_t smem = qr_apply_smem<NW>(max_m);
   static PerDeviceOnce attr_once;
   int dev = 0;
   TTC_CUDA(cudaGetDevice(&dev));
   attr_once.run(dev, [] {
-    TTC_CUDA(cudaFuncSetAttribute(householder_apply_q_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(sizeof(double) * (NB * NB + NW * 128 + (size_t)(QR_MAX_M + 15) * NB))));
+    TTC_CUDA(cudaFuncSetAttribute(householder_apply_q_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)qr_apply_smem<NW>(lim)));
   });
-  const int nsm = current_sm_count();
   int per_sm = 1;
-  TTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, householder_apply_q_kernel, NT, smem));
-  const int csize = std::min(8, std::max(1, nsm * std::max(1, per_sm) / count));
-  householder_apply_q_kernel<<<(unsigned)(count * csize), NT, smem, s>>>(d_descs, csize);
+  TTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, householder_apply_q_kernel<NW>, NW * 32, smem));
+  const int csize = std::min(8, std::max(1, current_sm_count() * std::max(1, per_sm) / count));
+  householder_apply_q_kernel<NW><<<(unsigned)(count * csize), NW * 32, smem, s>>>(d_descs, csize);
   TTC_CHECK_LAUNCH();
 }
 
-namespace {
-size_t qr_smem(int max_m) {
-  return sizeof(double) * (NB * NB * 4 + 3 * NB + NW + 2 + NW * 128 + (size_t)(max_m + 15) * NB);
-}
-
-constexpr int kQrWaves = 2;
-void launch_qr_cfg(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, int* d_flags) {
-  const size_t smem = qr_smem(max_m);
+template <int NW>
+void launch_qr_t(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, int* d_flags) {
+  constexpr int lim = NW <= 8 ? kSmallM : QR_MAX_M;
+  const size_t smem = qr_smem<NW>(max_m);
   static PerDeviceOnce attr_once;
   int dev = 0;
   TTC_CUDA(cudaGetDevice(&dev));
   attr_once.run(dev, [] {
-    TTC_CUDA(cudaFuncSetAttribute(householder_qr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)qr_smem(QR_MAX_M)));
+    TTC_CUDA(cudaFuncSetAttribute(householder_qr_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)qr_smem<NW>(lim)));
   });
-  const int nsm = current_sm_count();
-  // CTAs per problem: up to two waves of the resident-CTA slots of the GPU (the planner puts the
+  // CTAs per problem: one wave of the resident-CTA slots of the two-per-SM kernel (a CTA's column steps
+  // run beside its neighbour's products), two waves of the one-per-SM kernel (the planner puts the
   // largest problems first, so the second wave holds the short ones), at most 8 (portable cluster)
   int per_sm = 1;
-  TTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, householder_qr_kernel, NT, smem));
-  const int slots = nsm * std::max(1, per_sm);
-  int c = std::min(8, std::max(1, kQrWaves * slots / count));
+  TTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, householder_qr_kernel<NW>, NW * 32, smem));
+  const int slots = current_sm_count() * std::max(2, per_sm);
+  const int c = std::min(8, std::max(1, slots / count));
   int csize = 1;
   while (csize * 2 <= c) csize *= 2;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(count * csize));
-  cfg.blockDim = dim3(NT);
+  cfg.blockDim = dim3(NW * 32);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
@@ -548,15 +678,26 @@ void launch_qr_cfg(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, 
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  TTC_CUDA(cudaLaunchKernelEx(&cfg, householder_qr_kernel, d_descs, csize, d_flags));
+  TTC_CUDA(cudaLaunchKernelEx(&cfg, householder_qr_kernel<NW>, d_descs, csize, d_flags));
   TTC_CHECK_LAUNCH();
 }
 }  // namespace
 
+void launch_qr_apply(const QApplyDesc* d_descs, int count, int max_m, cudaStream_t s) {
+  if (count <= 0) return;
+  TTC_REQUIRE(max_m <= QR_MAX_M, TTC_EDIM, "qr apply: row count exceeds the supported maximum (1536)");
+  if (max_m <= kSmallM) launch_qr_apply_t<8>(d_descs, count, max_m, s);
+  else launch_qr_apply_t<16>(d_descs, count, max_m, s);
+}
+
 void launch_qr(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, int* d_flags) {
   if (count <= 0) return;
   TTC_REQUIRE(max_m <= QR_MAX_M, TTC_EDIM, "qr: row count exceeds the supported maximum (1536)");
-  launch_qr_cfg(d_descs, count, max_m, s, d_flags);
+  // Launches of few problems (every CTA has an SM to itself) and panels beyond 256 rows take sixteen
+  // warps: one problem 512 x 256 with Q 468 us (584 with eight), 276 x 138 203 (213), 256 x 256 363 (320)
+  const bool alone = max_m > 256 && 8LL * count <= current_sm_count();
+  if (max_m <= kSmallM && !alone) launch_qr_t<8>(d_descs, count, max_m, s, d_flags);
+  else launch_qr_t<16>(d_descs, count, max_m, s, d_flags);
 }
 
 }  // namespace ttc

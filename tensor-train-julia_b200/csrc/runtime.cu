@@ -144,7 +144,10 @@ static void launch_op(ttc_context* c, const Plan& p, const Op& op) {
     const unsigned char* d = p.d_blob + op.off;
     switch (op.kind) {
       case OP_GEMM: launch_gemm_f64((const GemmDesc*)d, op.count, op.total, s); break;
-      case OP_QR: launch_qr((const QRDesc*)d, op.count, op.a, s, c->d_flags); break;
+      case OP_QR:
+        if (op.total) launch_qr_seq((const QRDesc*)d, op.count, op.a, s, c->d_flags);
+        else launch_qr((const QRDesc*)d, op.count, op.a, s, c->d_flags);
+        break;
       case OP_QAPPLY: launch_qr_apply((const QApplyDesc*)d, op.count, op.a, s); break;
       case OP_JACOBI:
         launch_jacobi((const JacobiDesc*)d, op.count, op.a, op.b, op.total != 0, s, c->d_flags, op.iw, (int)op.rmax);
@@ -487,7 +490,7 @@ void Builder::widen(const std::vector<CvtDesc>& v) {
   Op op; op.kind = OP_WIDEN; op.off = plan->push(v); op.count = (int)v.size(); op.total = mx;
   plan->ops.push_back(op);
 }
-void Builder::qr(const std::vector<QRDesc>& v) {
+void Builder::qr(const std::vector<QRDesc>& v, bool sequential) {
   if (v.empty()) return;
   int mm = 0, nn = 0;
   for (auto& d : v) {
@@ -513,6 +516,7 @@ void Builder::qr(const std::vector<QRDesc>& v) {
     return qr_flops(a.m, a.n, a.Q != nullptr) > qr_flops(b.m, b.n, b.Q != nullptr);
   });
   Op op; op.kind = OP_QR; op.off = plan->push(w); op.count = (int)w.size(); op.a = mm; op.b = nn;
+  op.total = sequential ? 1 : 0;
   for (auto& d : w) op.flops += qr_flops(d.m, d.n, d.Q != nullptr);
   plan->ops.push_back(op);
 }
