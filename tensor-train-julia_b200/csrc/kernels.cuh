@@ -21,6 +21,9 @@ __device__ __forceinline__ int dev_bound(int cap, const int* p, int mult) {
   return p ? min(cap, max(0, mult * *p)) : cap;
 }
 
+// Dynamic shared memory that keeps a second CTA off an SM (227 KB at most per SM and CTA).
+constexpr size_t kLoneCtaSmem = 116 * 1024;
+
 // ---- batched Householder QR (qr_householder.cu)
 // A (m x n, col-major, lda) is overwritten.  Q (m x K, ldq) and R (K x n, ldr),
 // K = min(m, n), like LAPACK geqrf + orgqr (Julia `qr`, `Matrix(F.Q)`, `F.R`).

@@ -63,27 +63,30 @@ __device__ __forceinline__ void cluster_arrive() {
 }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
 
-// Rows r and r + 1 (r even) of a column with mp rows, zero where masked; one 16-byte load when the
-// column is 16-byte aligned (vec).
-__device__ __forceinline__ void load2(double (&v)[2], const double* col, int r, int mp, bool on, bool vec) {
-  if (on && vec && r + 1 < mp) {
-    const double2 t = *reinterpret_cast<const double2*>(col + r);
+// Rows r and r + 1 (r even) of a column with mp rows, zero where masked.  VEC: one 16-byte access; the
+// columns are 16-byte aligned and mp is even (vec_ok).
+template <bool VEC>
+__device__ __forceinline__ void load2(double (&v)[2], const double* col, int r, int mp, bool on) {
+  if (VEC) {
+    double2 t = make_double2(0.0, 0.0);
+    if (on && r < mp) t = *reinterpret_cast<const double2*>(col + r);
     v[0] = t.x; v[1] = t.y;
   } else {
     v[0] = (on && r < mp) ? col[r] : 0.0;
     v[1] = (on && r + 1 < mp) ? col[r + 1] : 0.0;
   }
 }
-__device__ __forceinline__ void store2(const double (&v)[2], double* col, int r, int mp, bool on, bool vec) {
-  if (on && vec && r + 1 < mp) {
-    *reinterpret_cast<double2*>(col + r) = make_double2(v[0], v[1]);
+template <bool VEC>
+__device__ __forceinline__ void store2(const double (&v)[2], double* col, int r, int mp, bool on) {
+  if (VEC) {
+    if (on && r < mp) *reinterpret_cast<double2*>(col + r) = make_double2(v[0], v[1]);
   } else {
     if (on && r < mp) col[r] = v[0];
     if (on && r + 1 < mp) col[r + 1] = v[1];
   }
 }
-__device__ __forceinline__ bool vec_ok(const double* p, int ld) {
-  return ((reinterpret_cast<uintptr_t>(p) & 15) == 0) && ((ld & 1) == 0);
+__device__ __forceinline__ bool vec_ok(const double* p, int ld, int mp) {
+  return ((reinterpret_cast<uintptr_t>(p) & 15) == 0) && (((ld | mp) & 1) == 0);
 }
 
 // 1 / sqrt(x) for normal positive x below 2^1000: the hardware's approximation (relative error below
@@ -142,7 +145,7 @@ __device__ __noinline__ void apply_block_g(double* M, int ld, int r0, int mp, in
   constexpr int NG = NW / G;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, qr = lane >> 2, qc = lane & 3;
   const int grp = warp / G, gw = warp % G;
-  const bool vec = vec_ok(M + r0, ld);
+  const bool vec = vec_ok(M + r0, ld, mp);
   const int o_begin = c_begin >> 3, o_end = (c_end + 7) >> 3;
   const int o_first = o_begin + ((crank - o_begin) % csize + csize) % csize;
   if (o_first + grp * csize >= o_end) return;
@@ -166,20 +169,25 @@ __device__ __noinline__ void apply_block_g(double* M, int ld, int r0, int mp, in
     const bool cok = (c >= c_begin && c < c_end);
     double* col = M + (long long)(cok ? c : c_begin) * ld + r0;
     double cc[MAXT][2];
+    if (vec) {
 #pragma unroll
-    for (int t = 0; t < MAXT; ++t) load2(cc[t], col, 8 * (gw + G * t) + 2 * qc, mp, cok, vec);
+      for (int t = 0; t < MAXT; ++t) load2<true>(cc[t], col, 8 * (gw + G * t) + 2 * qc, mp, cok);
+    } else {
+#pragma unroll
+      for (int t = 0; t < MAXT; ++t) load2<false>(cc[t], col, 8 * (gw + G * t) + 2 * qc, mp, cok);
+    }
     double w[2][2][2] = {};
 #pragma unroll
     for (int t = 0; t < MAXT; ++t) {
+      // leave the loop: multiplications predicated off would take the tensor core's time all the same
       const int rt = 8 * (gw + G * t);
-      if (rt < mp) {
-        const double2 v0 = *reinterpret_cast<const double2*>(p1 + rt);
-        const double2 v1 = *reinterpret_cast<const double2*>(p1 + 8 * mp_ld + rt);
-        dmma(w[0][0][0], w[0][0][1], cc[t][0], v0.x);
-        dmma(w[1][0][0], w[1][0][1], cc[t][0], v1.x);
-        dmma(w[0][1][0], w[0][1][1], cc[t][1], v0.y);
-        dmma(w[1][1][0], w[1][1][1], cc[t][1], v1.y);
-      }
+      if (rt >= mp) break;
+      const double2 v0 = *reinterpret_cast<const double2*>(p1 + rt);
+      const double2 v1 = *reinterpret_cast<const double2*>(p1 + 8 * mp_ld + rt);
+      dmma(w[0][0][0], w[0][0][1], cc[t][0], v0.x);
+      dmma(w[1][0][0], w[1][0][1], cc[t][0], v1.x);
+      dmma(w[0][1][0], w[0][1][1], cc[t][1], v0.y);
+      dmma(w[1][1][0], w[1][1][1], cc[t][1], v1.y);
     }
     double ws[2][2];
 #pragma unroll
@@ -215,11 +223,11 @@ __device__ __noinline__ void apply_block_g(double* M, int ld, int r0, int mp, in
 #pragma unroll
     for (int t = 0; t < MAXT; ++t) {
       const int rt = 8 * (gw + G * t);
-      if (rt < mp) {
+      if (rt >= mp) break;
 #pragma unroll
-        for (int s = 0; s < 4; ++s) dmma(cc[t][0], cc[t][1], -u[s >> 1][s & 1], p2[4 * s * mp_ld + rt]);
-        store2(cc[t], col, rt + 2 * qc, mp, cok, vec);
-      }
+      for (int s = 0; s < 4; ++s) dmma(cc[t][0], cc[t][1], -u[s >> 1][s & 1], p2[4 * s * mp_ld + rt]);
+      if (vec) store2<true>(cc[t], col, rt + 2 * qc, mp, cok);
+      else store2<false>(cc[t], col, rt + 2 * qc, mp, cok);
     }
   }
 }
@@ -242,7 +250,7 @@ __device__ __forceinline__ void apply_block(double* M, int ld, int r0, int mp, i
 template <int NW>
 __device__ __forceinline__ void load_panel_v(double* P, int mp_ld, const double* A, int lda, int mp, int jb) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool vec = vec_ok(A, lda);
+  const bool vec = vec_ok(A, lda, mp);
   const int mp8 = (mp + 7) & ~7;
 #pragma unroll
   for (int q = 0; q < NB / NW; ++q) {
@@ -250,8 +258,13 @@ __device__ __forceinline__ void load_panel_v(double* P, int mp_ld, const double*
     const double* col = A + (long long)c * lda;
     for (int b = 2 * lane; b < mp8; b += 512) {
       double v[8][2];
+      if (vec) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) load2(v[i], col, b + 64 * i, mp, c < jb, vec);
+        for (int i = 0; i < 8; ++i) load2<true>(v[i], col, b + 64 * i, mp, c < jb);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) load2<false>(v[i], col, b + 64 * i, mp, c < jb);
+      }
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int r = b + 64 * i;
@@ -368,14 +381,22 @@ __device__ __noinline__ bool factor_panel(double* A, int lda, int mp, int jb, in
   constexpr int CW = NB / NW, CPW = CW * LPC / 32, CH = 2 * LPC, XLD = CH * RI;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, hl = lane & (LPC - 1);
   const int c0 = warp * CW + lane / LPC;      // column q of this lane: c0 + q
-  const bool vec = vec_ok(A, lda);
+  const bool vec = vec_ok(A, lda, mp);
   double* X = S.P;                            // two published columns (the panel region is free until the end)
   double cr[CPW][RI][2];
+  if (vec) {
 #pragma unroll
-  for (int q = 0; q < CPW; ++q)
+    for (int q = 0; q < CPW; ++q)
 #pragma unroll
-    for (int i = 0; i < RI; ++i)
-      load2(cr[q][i], A + (long long)(c0 + q) * lda, CH * i + 2 * hl, mp, c0 + q < jb, vec);
+      for (int i = 0; i < RI; ++i)
+        load2<true>(cr[q][i], A + (long long)(c0 + q) * lda, CH * i + 2 * hl, mp, c0 + q < jb);
+  } else {
+#pragma unroll
+    for (int q = 0; q < CPW; ++q)
+#pragma unroll
+      for (int i = 0; i < RI; ++i)
+        load2<false>(cr[q][i], A + (long long)(c0 + q) * lda, CH * i + 2 * hl, mp, c0 + q < jb);
+  }
   int hi = 0;
 #pragma unroll
   for (int q = 0; q < CPW; ++q)
@@ -504,7 +525,8 @@ __device__ __noinline__ bool factor_panel(double* A, int lda, int mp, int jb, in
         }
       }
       if (r < mp8) *reinterpret_cast<double2*>(S.P + panel_at(c, r, mp_ld)) = make_double2(v[0], v[1]);
-      store2(g, A + (long long)c * lda, r, mp, out, vec);
+      if (vec) store2<true>(g, A + (long long)c * lda, r, mp, out);
+      else store2<false>(g, A + (long long)c * lda, r, mp, out);
     }
   }
   if (warp == 0) form_t<NW>(S, jb, (crank == 0) ? Tws : nullptr);   // its columns' registers are free by now
@@ -637,12 +659,13 @@ void launch_qr_apply_t(const QApplyDesc* d_descs, int count, int max_m, cudaStre
   TTC_CUDA(cudaGetDevice(&dev));
   attr_once.run(dev, [] {
     TTC_CUDA(cudaFuncSetAttribute(householder_apply_q_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)qr_apply_smem<NW>(lim)));
+                                  (int)std::max(qr_apply_smem<NW>(lim), kLoneCtaSmem)));
   });
   int per_sm = 1;
   TTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, householder_apply_q_kernel<NW>, NW * 32, smem));
   const int csize = std::min(8, std::max(1, current_sm_count() * std::max(1, per_sm) / count));
-  householder_apply_q_kernel<NW><<<(unsigned)(count * csize), NW * 32, smem, s>>>(d_descs, csize);
+  const size_t smem_l = count * csize <= current_sm_count() ? std::max(smem, kLoneCtaSmem) : smem;
+  householder_apply_q_kernel<NW><<<(unsigned)(count * csize), NW * 32, smem_l, s>>>(d_descs, csize);
   TTC_CHECK_LAUNCH();
 }
 
@@ -655,7 +678,7 @@ void launch_qr_t(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, in
   TTC_CUDA(cudaGetDevice(&dev));
   attr_once.run(dev, [] {
     TTC_CUDA(cudaFuncSetAttribute(householder_qr_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)qr_smem<NW>(lim)));
+                                  (int)std::max(qr_smem<NW>(lim), kLoneCtaSmem)));
   });
   // CTAs per problem: one wave of the resident-CTA slots of the two-per-SM kernel (a CTA's column steps
   // run beside its neighbour's products), two waves of the one-per-SM kernel (the planner puts the
@@ -669,7 +692,8 @@ void launch_qr_t(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, in
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(count * csize));
   cfg.blockDim = dim3(NW * 32);
-  cfg.dynamicSmemBytes = smem;
+  // one CTA per SM while there are SMs for all
+  cfg.dynamicSmemBytes = count * csize <= current_sm_count() ? std::max(smem, kLoneCtaSmem) : smem;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;

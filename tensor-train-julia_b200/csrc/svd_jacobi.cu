@@ -517,9 +517,10 @@ __global__ void __launch_bounds__(NT, RMAX <= 8 ? 2 : 1)
 // streams a block through shared memory, reduces three dot products across the warp and waits at a
 // barrier, and measured per step that is several thousand cycles, 70 % of the kernel.  Here a CTA
 // takes its block pair (32 column slots: block I in slots 0-15, block J in 16-31) and
-//   1. forms the 32 x 32 Gram matrix G = S^T S on the FP64 tensor cores (mma.sync m8n8k4);
+//   1. forms the 32 x 32 Gram matrix G = S^T S on the FP64 tensor cores (mma.sync m8n8k4), the ten
+//      tiles on and above the diagonal, each quarter of the rows by two warps;
 //   2. runs the Jacobi rotations on G instead of on the columns (two-sided: G <- J^T G J, with the
-//      rotations accumulated in V, V <- V J), 16 disjoint pairs per inner round and two barriers
+//      rotations accumulated in V, V <- V J), 16 disjoint pairs per inner round and one barrier
 //      per round, on 32-element rows instead of m-row columns;
 //   3. applies V to the columns with the tensor cores again (S V, m x 32 x 32), writing the result
 //      straight back to the problem's columns in global memory.
@@ -537,58 +538,49 @@ __global__ void __launch_bounds__(NT, RMAX <= 8 ? 2 : 1)
 // blocks); in the later rounds only the 256 cross pairs (inner round s pairs slot p with
 // 16 + (p + s) mod 16).  A sweep thus visits every column pair once, and it converges when no CTA of
 // the cluster rotated anything during a whole sweep.
+// What bounds it: the inner rounds' chain of instructions, then the two products.  Cycles per visit of
+// one 248 x 248 problem (eight CTAs) before and now: inner rounds 15200 and 9100, Gram matrix 6200 and
+// 3600, S V 6600 and 5800; one such problem 1.54 and 1.09 ms, 60 of them 4.53 and 3.11 ms.
 namespace {
 constexpr int GLD = 36;          // leading dimension of G and V in shared memory (= 4 mod 16: no bank conflicts)
+constexpr int GSZ = 32 * GLD;
+constexpr int kGramPart = 640;   // the ten 8 x 8 tiles on and above the diagonal of a 32 x 32 Gram matrix
 
-// Rotation of one pair in an inner round, split by who reads it: RotA (slots, cosine, sine; read by
-// every role) and RotB (t = s / c and the pair's entries of G before the round; read by the threads
-// that update the diagonal or compute the next round's rotations).
-struct __align__(16) RotA {
-  double c, s;
-  int i, j, on, pad;
-};
-struct __align__(16) RotB {
-  double t, gii, gjj, gij;
-};
-
-// Shared-memory doubles of a launch of jacobi_block_kernel: S (32 slots of stride ms), G, V and the
-// column norms (n); the active-column list (n ints) follows.
+// Shared-memory doubles of a launch of jacobi_block_kernel: S (32 slots of stride ms), the two copies of
+// G and V (together also the four partial Gram matrices) and the column norms (n); the active-column
+// list (n ints) follows.
 __host__ __device__ __forceinline__ size_t block_dyn_doubles(int ms, int n) {
-  return (size_t)32 * ms + 2 * 32 * GLD + (size_t)n;
+  return (size_t)32 * ms + (GSZ + 4 * kGramPart) + (size_t)n;
 }
 
 __device__ __forceinline__ void cp_async8(double* dst, const double* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
 }
-
-// Pairing of inner round r: the circle method over the 32 slots (full) or the cross pairs
-// (p, 16 + (p + r) mod 16).  Partner of slot x and the index of its pair.
-__device__ __forceinline__ void inner_partner(int x, int r, bool full, int& y, int& pidx) {
-  if (full) {
-    const int pos = (x == 0) ? 0 : ((x - 1 - r) % 31 + 31) % 31 + 1;
-    y = rr_player(31 - pos, r, 32);
-    pidx = min(pos, 31 - pos);
-  } else if (x < 16) {
-    y = 16 + ((x + r) & 15);
-    pidx = x;
-  } else {
-    pidx = (x - 16 - r) & 15;
-    y = pidx;
-  }
+__device__ __forceinline__ void cp_async16(double* dst, const double* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
 }
 
-// make_rot without branches (the same operations; a pair that does not rotate gets c = 1, s = t = 0),
-// for the inner rounds' critical path.
+// 1 / sqrt(x) for normal positive x: the hardware's approximation (relative error below 2^-19) and one
+// third-order step y (1 + e/2 + 3 e^2 / 8), e = 1 - x y^2 (Householder's method; remainder 5 e^3 / 16).
+__device__ __forceinline__ double rsqrt_normal(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
+// make_rot without branches on scaled values, for the inner rounds' critical path: a pair that does not
+// rotate gets c = 1, s = t = 0.
 __device__ __forceinline__ Rot make_rot_nb(double alpha, double beta, double gamma, const RotCfg& q) {
-  alpha *= q.sc; beta *= q.sc; gamma *= q.sc;
-  const double g2 = gamma * gamma;
+  const double g2 = gamma * gamma, d = beta - alpha;
+  const double rh = rsqrt_normal(fma(d, d, 4.0 * g2));
   const bool ap = (alpha > q.zthr) && (beta > q.zthr) && (g2 > q.tol2 * alpha * beta);
-  const double d = beta - alpha;
-  const double rh = rsqrt(fma(d, d, 4.0 * g2));
   const double c2 = fma(0.5 * fabs(d), rh, 0.5);
-  const double rc = rsqrt(c2);
-  const double s = copysign(1.0, d) * gamma * rh * rc;
+  const double gs = copysign(1.0, d) * (gamma * rh);
+  const double rc = rsqrt_normal(c2);
+  const double s = gs * rc;
   Rot r;
   r.c = ap ? c2 * rc : 1.0;
   r.s = ap ? s : 0.0;
@@ -597,172 +589,176 @@ __device__ __forceinline__ Rot make_rot_nb(double alpha, double beta, double gam
   return r;
 }
 
-// Rotation of slots x, y from their entries of G, written with i = min(x, y), j = max(x, y); returns
-// whether it rotates.
-__device__ __forceinline__ bool set_pair(RotA& PA, RotB& PB, int x, int y, double gxx, double gyy, double gxy,
-                                         const RotCfg& q) {
-  const int i = min(x, y), j = max(x, y);
-  const double gii = (x < y) ? gxx : gyy, gjj = (x < y) ? gyy : gxx;
-  const Rot R = make_rot_nb(gii, gjj, gxy, q);
-  PA.c = R.c; PA.s = R.s; PA.i = i; PA.j = j; PA.on = R.apply ? 1 : 0;
-  PB.t = R.t; PB.gii = gii; PB.gjj = gjj; PB.gij = gxy;
-  return R.apply;
+// Entry (i, j) of a symmetric matrix of which the part i < j is kept.
+__device__ __forceinline__ int sym(int i, int j) { return min(i, j) + max(i, j) * GLD; }
+
+// Next slot of a circle-method position: slots 1 .. 31 move round, slot 0 stays.
+__device__ __forceinline__ int rr_next(int x) { return x == 0 ? 0 : (x == 31 ? 1 : x + 1); }
+
+__device__ __forceinline__ double flip(double v, int mask) {   // v with the sign bit xor mask
+  return __hiloint2double(__double2hiint(v) ^ mask, __double2loint(v));
 }
 
-// The 2 x 2 block of G in rows (A.i, A.j) and columns (B.i, B.j) after the round's rotations:
-// rows i' = c i - s j, j' = s i + c j by A, then the same on the columns by B.
-__device__ __forceinline__ void rotate_block(const RotA& A, const RotA& B, double& b00, double& b01, double& b10,
-                                             double& b11) {
-  if (A.on) {
-    const double u0 = A.c * b00 - A.s * b10, v0 = fma(A.s, b00, A.c * b10);
-    const double u1 = A.c * b01 - A.s * b11, v1 = fma(A.s, b01, A.c * b11);
-    b00 = u0; b10 = v0; b01 = u1; b11 = v1;
-  }
-  if (B.on) {
-    const double u0 = B.c * b00 - B.s * b01, v0 = fma(B.s, b00, B.c * b01);
-    const double u1 = B.c * b10 - B.s * b11, v1 = fma(B.s, b10, B.c * b11);
-    b00 = u0; b01 = v0; b10 = u1; b11 = v1;
-  }
+// The barrier of an inner round: the warps arrive from the code of their roles.
+__device__ __forceinline__ void round_barrier() {
+  __syncwarp();
+  asm volatile("bar.sync 1, %0;\n" ::"n"(NT) : "memory");
 }
 
-// rotate_block without branches: a pair that does not rotate has c = 1, s = 0 exactly, which leaves
-// finite entries unchanged bit for bit.
-__device__ __forceinline__ void rotate_block_nb(const RotA& A, const RotA& B, double& b00, double& b01, double& b10,
-                                                double& b11) {
-  const double u0 = A.c * b00 - A.s * b10, v0 = fma(A.s, b00, A.c * b10);
-  const double u1 = A.c * b01 - A.s * b11, v1 = fma(A.s, b01, A.c * b11);
-  b00 = B.c * u0 - B.s * u1; b01 = fma(B.s, u0, B.c * u1);
-  b10 = B.c * v0 - B.s * v1; b11 = fma(B.s, v0, B.c * v1);
-}
-
-// V's rows in registers (thread = row): the rotations of inner round R, whose slots are known at
-// compile time, applied to the row.
-__host__ __device__ constexpr int rr_slot(int pos, int round) { return pos == 0 ? 0 : ((pos - 1 + round) % 31) + 1; }
-template <int R, bool FULL>
-__device__ __forceinline__ void v_apply(double (&v)[32], const RotA* P) {
-  // a pair that does not rotate has c = 1, s = 0 exactly (make_rot), so every pair is applied
-  // without a branch and all sixteen loads are issued first
-  double c[16], s[16];
-#pragma unroll
-  for (int p = 0; p < 16; ++p) {   // (c, s) are the first 16 bytes of a 16-byte aligned RotA
-    const double2 cs = *reinterpret_cast<const double2*>(&P[p].c);
-    c[p] = cs.x; s[p] = cs.y;
-  }
-#pragma unroll
-  for (int p = 0; p < 16; ++p) {
-    const int x = FULL ? rr_slot(p, R) : p, y = FULL ? rr_slot(31 - p, R) : 16 + ((p + R) & 15);
-    const int i = x < y ? x : y, j = x < y ? y : x;
-    const double a = v[i], b = v[j];
-    v[i] = c[p] * a - s[p] * b;
-    v[j] = fma(s[p], a, c[p] * b);
-  }
-}
-#define TTC_VCASE(R) \
-  case R: v_apply<R, FULL>(v, P); break;
+// The inner rounds on G: nr rounds of 16 disjoint pairs, pair p of round r being the slots at positions p
+// and 31 - p of the circle method (FULL, 31 rounds: all pairs), or p and 16 + (p + r) mod 16 (16 rounds:
+// the pairs across the blocks).  One barrier per round, the roles dealt by warps:
+//  * warps 0, 1, 2 and 4 rotate the 120 off-diagonal 2 x 2 blocks of G (pairs p < q, a thread each) from
+//    one copy of G into the other, so that the pre-round entries stay readable for the whole round;
+//  * lanes 0-15 of warp 7 carry the pairs' own off-diagonal entries over (OFF: zero after a rotation);
+//  * warps 5 and 6 rotate V, two lanes to a row, in registers ordered by position (shifted by one place
+//    per round: one loop body instead of one per round, which had outgrown the instruction cache);
+//  * warp 3, the critical path, with its scheduler almost to itself, computes the rotations of round r + 1, one pair a lane: its slots u, v were paired with u', v' in round r, so after round r
+//      G[u,v] = c_u (c_v G[u,v] + s_v G[u,v']) + s_u (c_v G[u',v] + s_v G[u',v'])
+//    with the signed sines of u and v (new u = c_u u + s_u u'), and G[u,u], G[v,v] are what the rotations
+//    of round r left (alpha - t gamma, beta + t gamma).
+// A pair's rotation is kept by pair index: CSP = (c, s of its first slot; the second has -s), DG = the
+// two diagonal entries after it.  The place of u and v in round r (pair, side) is the same in every
+// round.  Returns whether a pair rotated after round 0 (warp 3's lanes).
 template <bool FULL>
-__device__ __forceinline__ void v_round(double (&v)[32], const RotA* P, int r) {
-  switch (r) {
-    TTC_VCASE(0) TTC_VCASE(1) TTC_VCASE(2) TTC_VCASE(3) TTC_VCASE(4) TTC_VCASE(5) TTC_VCASE(6) TTC_VCASE(7)
-    TTC_VCASE(8) TTC_VCASE(9) TTC_VCASE(10) TTC_VCASE(11) TTC_VCASE(12) TTC_VCASE(13) TTC_VCASE(14) TTC_VCASE(15)
-    default:
-      if constexpr (FULL) {
-        switch (r) {
-          TTC_VCASE(16) TTC_VCASE(17) TTC_VCASE(18) TTC_VCASE(19) TTC_VCASE(20) TTC_VCASE(21) TTC_VCASE(22)
-          TTC_VCASE(23) TTC_VCASE(24) TTC_VCASE(25) TTC_VCASE(26) TTC_VCASE(27) TTC_VCASE(28) TTC_VCASE(29)
-          TTC_VCASE(30)
-          default: break;
-        }
-      }
-      break;
-  }
-}
-#undef TTC_VCASE
-
-// One inner round r on G with the rotations (cA, cB) computed from G before the round, in one
-// barrier interval, the roles dealt by warps (a warp whose lanes take different roles runs the roles
-// one after another, and warps w and w + 4 share a scheduler):
-//  * warps 0-2 and lanes 0-23 of warp 4 apply the rotations to the 120 off-diagonal 2 x 2 blocks
-//    (pair p rows, pair q columns, p < q; table blk) of G <- J^T G J, and lanes 0-15 of warp 5 to
-//    the 16 diagonal blocks;
-//  * warp 6 applies them to V, whose rows it holds in registers (thread = row);
-//  * lanes 0-15 of warp 3, the round's critical path, with its scheduler to itself (warp 7 idles),
-//    compute the rotations of round r + 1 into (nA, nB), one pair each:
-//    the pair's two slots lie in two different pairs of round r (a round robin never repeats a pair
-//    in consecutive rounds), so its three entries after this round follow from the pre-round block
-//    of those pairs and their rotations, evaluated with the same operations as the block update.
-template <bool FULL>
-__device__ __forceinline__ void gram_round(double* G, double (&vrow)[32], const RotA* cA, const RotB* cB, RotA* nA,
-                                           RotB* nB, const unsigned char* blk, const unsigned long long* sched, int r, int nr,
-                                           const RotCfg& q, int* s_rot, unsigned long long& pre) {
+__device__ __forceinline__ bool inner_rounds(double* G, double* V, double2 (*CSP)[16], double (*DG)[32], double (*OFF)[16],
+                                             const RotCfg& q) {
+  constexpr int NR = FULL ? 31 : 16;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (warp < 3 || (warp == 4 && lane < 24)) {
+  bool any = false;
+  if (warp < 3 || warp == 4) {
     const int bk = warp < 3 ? tid : 96 + lane;
-    const RotA A = cA[blk[2 * bk]], B = cA[blk[2 * bk + 1]];
-    if (A.on || B.on) {
-      double b00 = G[A.i + B.i * GLD], b01 = G[A.i + B.j * GLD];
-      double b10 = G[A.j + B.i * GLD], b11 = G[A.j + B.j * GLD];
-      rotate_block(A, B, b00, b01, b10, b11);
-      G[A.i + B.i * GLD] = b00; G[B.i + A.i * GLD] = b00;
-      G[A.i + B.j * GLD] = b01; G[B.j + A.i * GLD] = b01;
-      G[A.j + B.i * GLD] = b10; G[B.i + A.j * GLD] = b10;
-      G[A.j + B.j * GLD] = b11; G[B.j + A.j * GLD] = b11;
-    }
-  } else if (warp == 5 && lane < 16) {
-    const RotA A = cA[lane];
-    if (A.on) {
-      const RotB Bd = cB[lane];
-      G[A.i * (GLD + 1)] = Bd.gii - Bd.t * Bd.gij;
-      G[A.j * (GLD + 1)] = Bd.gjj + Bd.t * Bd.gij;
-      G[A.i + A.j * GLD] = 0.0;
-      G[A.j + A.i * GLD] = 0.0;
-    }
-  } else if (warp == 6) {
-    v_round<FULL>(vrow, cA, r);
-  } else if (warp == 3 && lane < 16) {
-    if (r + 1 < nr) {
-      const int p = lane;
-      // pair p of round r + 1 = (u, v); u lies in pair ia, v in pair ib of round r (ia < ib, the
-      // block update's orientation), whose slots (Ai, Aj), (Bi, Bj) the schedule fixes
-      int ia, ib, Ai, Aj, Bi, Bj, u, v;
-      if (FULL) {
-        const unsigned long long e = pre;   // schedule entry of round r + 1, loaded a round earlier
-        if (r + 2 < nr) pre = sched[(r + 2) * 16 + p];
-        ia = e & 15; ib = (e >> 4) & 15; Ai = (e >> 8) & 31; Aj = (e >> 13) & 31;
-        Bi = (e >> 18) & 31; Bj = (e >> 23) & 31; u = (e >> 28) & 31; v = (e >> 33) & 31;
-      } else {
-        // (p, 16 + (p + r + 1) mod 16): p lies in pair p, the other slot in pair p + 1 (mod 16)
-        const int a = p, b = (p + 1) & 15, ya = 16 + ((p + r) & 15), yb = 16 + ((p + 1 + r) & 15);
-        const bool sw = a > b;
-        ia = sw ? b : a; ib = sw ? a : b;
-        Ai = ia; Aj = sw ? yb : ya; Bi = ib; Bj = sw ? ya : yb;
-        u = sw ? yb : p; v = sw ? p : yb;
+    int p = 0, rem = min(bk, 119);
+    while (rem >= 15 - p) { rem -= 15 - p; ++p; }
+    const int pq = p + 1 + rem;
+    const bool on = bk < 120;
+    int x = p, y = pq, x1 = FULL ? 31 - p : 16 + p, y1 = FULL ? 31 - pq : 16 + pq;
+#pragma unroll 2
+    for (int r = 0; r < NR; ++r) {
+      const double* Gc = G + (r & 1) * GSZ;
+      double* Gn = G + ((r & 1) ^ 1) * GSZ;
+      const double2 A = CSP[r & 1][p], B = CSP[r & 1][pq];
+      const int i00 = FULL ? sym(x, y) : x + y * GLD, i01 = FULL ? sym(x, y1) : x + y1 * GLD;
+      const int i10 = FULL ? sym(x1, y) : y + x1 * GLD, i11 = sym(x1, y1);
+      const double g00 = Gc[i00], g01 = Gc[i01], g10 = Gc[i10], g11 = Gc[i11];
+      const double u0 = fma(A.y, g10, A.x * g00), v0 = fma(-A.y, g00, A.x * g10);
+      const double u1 = fma(A.y, g11, A.x * g01), v1 = fma(-A.y, g01, A.x * g11);
+      if (on) {
+        Gn[i00] = fma(B.y, u1, B.x * u0);
+        Gn[i01] = fma(-B.y, u0, B.x * u1);
+        Gn[i10] = fma(B.y, v1, B.x * v0);
+        Gn[i11] = fma(-B.y, v0, B.x * v1);
       }
-      double b00 = G[Ai + Bi * GLD], b01 = G[Ai + Bj * GLD];
-      double b10 = G[Aj + Bi * GLD], b11 = G[Aj + Bj * GLD];
-      const RotA A = cA[ia], B = cA[ib];
-      const RotB AB = cB[ia], BB = cB[ib];
-      rotate_block_nb(A, B, b00, b01, b10, b11);
-      // a pair that does not rotate has t = 0: its diagonal stays as it is
-      const double guv = (u == Ai) ? ((v == Bi) ? b00 : b01) : ((v == Bi) ? b10 : b11);
-      const double guu = (u == Ai) ? AB.gii - AB.t * AB.gij : AB.gjj + AB.t * AB.gij;
-      const double gvv = (v == Bi) ? BB.gii - BB.t * BB.gij : BB.gjj + BB.t * BB.gij;
-      if (set_pair(nA[p], nB[p], u, v, guu, gvv, guv, q)) *s_rot = 1;
+      if (FULL) { x = rr_next(x); x1 = rr_next(x1); y = rr_next(y); y1 = rr_next(y1); }
+      else { x1 = x1 == 31 ? 16 : x1 + 1; y1 = y1 == 31 ? 16 : y1 + 1; }
+      round_barrier();
+    }
+  } else if (warp == 5 || warp == 6) {
+    // row = 16 (warp - 5) + lane mod 16; lane half h holds the pairs 8 h .. 8 h + 7: v[k] the first slot of
+    // pair 8 h + k, w[k] the second one (FULL: at positions 31 - 8 h - k)
+    const int h = lane >> 4, row = 16 * (warp - 5) + (lane & 15);
+    double v[8], w[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      v[k] = (8 * h + k == row) ? 1.0 : 0.0;
+      w[k] = ((FULL ? 31 - 8 * h - k : 16 + 8 * h + k) == row) ? 1.0 : 0.0;
+    }
+    for (int r = 0; r < NR; ++r) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const double2 A = CSP[r & 1][8 * h + k];
+        const double a = v[k], b = w[k];
+        v[k] = fma(A.y, b, A.x * a);
+        w[k] = fma(-A.y, a, A.x * b);
+      }
+      // one place on: position j takes the slot at j + 1 (FULL: 1 .. 31, else 16 .. 31 in a circle); one
+      // slot crosses between the lane halves each way
+      if (FULL) {
+        const double out = __shfl_xor_sync(0xffffffffu, h ? v[0] : w[7], 16), first = v[1];
+#pragma unroll
+        for (int k = 0; k < 7; ++k)
+          if (k > 0) v[k] = v[k + 1];
+        if (h) v[0] = first;
+        v[7] = h ? w[7] : out;                  // position 15 takes 16, position 7 takes 8
+#pragma unroll
+        for (int k = 7; k > 0; --k) w[k] = w[k - 1];
+        w[0] = h ? out : first;                 // position 23 takes 24, position 31 takes 1
+      } else {
+        const double out = __shfl_xor_sync(0xffffffffu, w[0], 16);
+#pragma unroll
+        for (int k = 0; k < 7; ++k) w[k] = w[k + 1];
+        w[7] = out;
+      }
+      round_barrier();
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      V[row + (8 * h + k) * GLD] = v[k];
+      V[row + (FULL ? 31 - 8 * h - k : 16 + 8 * h + k) * GLD] = w[k];
+    }
+  } else if (warp == 3) {
+    const int p = lane & 15;
+    int u, v, u1, v1, ia, ib, da, db, ma, mb;   // slots in round r + 1 and their partners in round r
+    const int neg = (int)0x80000000;
+    if (FULL) {
+      u = (p == 0) ? 0 : p + 1;  v = (p == 0) ? 1 : 32 - p;                 // round 1
+      u1 = (p == 0) ? 31 : 30 - p;                                          // partners in round 0
+      v1 = (p == 0) ? 30 : p - 1;
+      const int pu = (p == 0) ? 0 : p + 1, pv = (p == 0) ? 1 : 32 - p;      // positions in round r
+      ia = min(pu, 31 - pu); ma = pu > 15 ? neg : 0; da = 2 * ia + (pu > 15);
+      ib = min(pv, 31 - pv); mb = pv > 15 ? neg : 0; db = 2 * ib + (pv > 15);
+    } else {
+      u = p; v = 16 + ((p + 1) & 15); u1 = 16 + p; v1 = (p + 1) & 15;
+      ia = p; ma = 0; da = 2 * p;
+      ib = (p + 1) & 15; mb = neg; db = 2 * ib + 1;
+    }
+#pragma unroll 2
+    for (int r = 0; r < NR; ++r) {
+      if (r + 1 < NR) {
+        const double* Gc = G + (r & 1) * GSZ;
+        const double2 A = CSP[r & 1][ia], B = CSP[r & 1][ib];
+        const double al = DG[r & 1][da], be = DG[r & 1][db];
+        const int j00 = FULL ? sym(u, v) : u + v * GLD, j01 = sym(u, v1);
+        const int j10 = sym(u1, v), j11 = FULL ? sym(u1, v1) : v1 + u1 * GLD;
+        const double g00 = Gc[j00], g01 = Gc[j01], g10 = Gc[j10], g11 = Gc[j11];
+        const double su = flip(A.y, ma), sv = flip(B.y, mb);
+        const double t1 = fma(sv, g01, B.x * g00), t2 = fma(sv, g11, B.x * g10);
+        const double ga = fma(su, t2, A.x * t1);
+        const Rot R = make_rot_nb(al, be, ga, q);
+        if (lane < 16) {
+          CSP[(r & 1) ^ 1][p] = make_double2(R.c, -R.s);
+          *reinterpret_cast<double2*>(&DG[(r & 1) ^ 1][2 * p]) = make_double2(fma(-R.t, ga, al), fma(R.t, ga, be));
+          OFF[(r & 1) ^ 1][p] = R.apply ? 0.0 : ga;
+        }
+        any |= R.apply;
+        if (FULL) { u = rr_next(u); v = rr_next(v); u1 = rr_next(u1); v1 = rr_next(v1); }
+        else { v = v == 31 ? 16 : v + 1; u1 = u1 == 31 ? 16 : u1 + 1; }
+      }
+      round_barrier();
+    }
+  } else {
+    const int p = lane & 15;
+    int x = p, x1 = FULL ? 31 - p : 16 + p;
+    for (int r = 0; r < NR; ++r) {
+      if (lane < 16) G[((r & 1) ^ 1) * GSZ + sym(x, x1)] = OFF[r & 1][p];
+      if (FULL) { x = rr_next(x); x1 = rr_next(x1); }
+      else x1 = x1 == 31 ? 16 : x1 + 1;
+      round_barrier();
     }
   }
-  __syncthreads();
+  return any;
 }
 }  // namespace
 
 __global__ void __launch_bounds__(NT, 2)
     jacobi_block_kernel(const JacobiDesc* __restrict__ descs, const int* __restrict__ order, int csize, int* flags,
                         int max_sweeps) {
-  extern __shared__ double sm[];
+  extern __shared__ __align__(16) double sm[];
   __shared__ int s_any, s_nact;
   __shared__ double s_red[NW];
-  __shared__ RotA s_ra[2][16];
-  __shared__ RotB s_rb[2][16];
-  __shared__ unsigned char s_blk[2 * 120];
-  __shared__ unsigned long long s_sched[31 * 16];   // full inner sweep: pair p of round r, see gram_round
+  __shared__ double2 s_csp[2][16];
+  __shared__ __align__(16) double s_dg[2][32];
+  __shared__ double s_off[2][16];
   __shared__ int s_rot;
   cg::cluster_group cluster = cg::this_cluster();
   const int crank = (int)cluster.block_rank();
@@ -772,11 +768,14 @@ __global__ void __launch_bounds__(NT, 2)
   const int m = max(1, dev_bound(D.m, D.m_dev, D.m_mult)), n = D.n;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, qr = lane >> 2, qc = lane & 3;
   const int ms = smem_stride(m);
+  const int m4 = (m + 3) & ~3;                  // rows m .. m4 - 1 of S are zero
   double* S = sm;
-  double* G = S + (size_t)32 * ms;
-  double* V = G + 32 * GLD;
-  double* nrm = V + 32 * GLD;
+  double* G = S + (size_t)32 * ms;              // G[0]; the partial Gram matrices lie behind it, over G[1] and V
+  double* part = G + GSZ;
+  double* V = G + 2 * GSZ;
+  double* nrm = G + GSZ + 4 * kGramPart;
   int* act = reinterpret_cast<int*>(sm + block_dyn_doubles(ms, n));
+  const bool vec = ((D.ldx & 1) == 0) && ((reinterpret_cast<uintptr_t>(D.X) & 15) == 0);
 
   // column norms and ||X||_F^2: scale and numerical-zero threshold, as in jacobi_svd_kernel
   {
@@ -792,30 +791,6 @@ __global__ void __launch_bounds__(NT, 2)
     if (lane == 0) s_red[warp] = a;
   }
   if (tid == 0) s_any = 0;
-  if (tid < 120) {   // the off-diagonal 2 x 2 blocks (p, q), p < q, of an inner round
-    int p = 0, rem = tid;
-    while (rem >= 15 - p) { rem -= 15 - p; ++p; }
-    s_blk[2 * tid] = (unsigned char)p;
-    s_blk[2 * tid + 1] = (unsigned char)(p + 1 + rem);
-  }
-  for (int e = tid; e < 31 * 16; e += NT) {
-    const int r = e >> 4, p = e & 15;
-    unsigned long long w = 0;
-    if (r > 0) {
-      const int x = rr_player(p, r, 32), y = rr_player(31 - p, r, 32);
-      int xp, a, yp, b;
-      inner_partner(x, r - 1, true, xp, a);
-      inner_partner(y, r - 1, true, yp, b);
-      const bool sw = a > b;
-      const int ia = sw ? b : a, ib = sw ? a : b;
-      const int u = sw ? y : x, up = sw ? yp : xp, v = sw ? x : y, vp = sw ? xp : yp;
-      w = (unsigned long long)ia | ((unsigned long long)ib << 4) | ((unsigned long long)min(u, up) << 8) |
-          ((unsigned long long)max(u, up) << 13) | ((unsigned long long)min(v, vp) << 18) |
-          ((unsigned long long)max(v, vp) << 23) | ((unsigned long long)u << 28) | ((unsigned long long)v << 33);
-    }
-    s_sched[e] = w;
-  }
-
   __syncthreads();
   double fro2 = 0.0;
 #pragma unroll
@@ -846,6 +821,9 @@ __global__ void __launch_bounds__(NT, 2)
   const int ne = nblk + (nblk & 1);
   cluster.sync();   // every CTA of the cluster runs before the first distributed-shared-memory access
 
+  // Gram tiles (a, b), a <= b, of 8 x 8 entries: five of them for each of the two warps that share a
+  // quarter of the rows
+  const int kq = ((m4 + 15) / 16) * 4, kbeg = min(m4, (warp >> 1) * kq), kend = min(m4, kbeg + kq);
   int* any0 = cluster.map_shared_rank(&s_any, 0);
   bool converged = false;
   int sweep = 0;
@@ -861,114 +839,144 @@ __global__ void __launch_bounds__(NT, 2)
           bj = -1;
         }
         const int cI = min(16, na - bi * 16), cJ = bj >= 0 ? min(16, na - bj * 16) : 0;
-        // load the valid slots: a warp per slot, lanes over rows, every copy in flight at once
-        for (int slot = warp; slot < 32; slot += NW) {
-          const bool inI = slot < 16;
-          const int k = inI ? slot : slot - 16;
-          if (k >= (inI ? cI : cJ)) continue;
-          const double* src = D.X + (long long)act[(inI ? bi : bj) * 16 + k] * D.ldx;
+        auto valid = [&](int slot) { return slot < 16 ? slot < cI : slot - 16 < cJ; };
+        // load the valid slots: a warp per slot, lanes over rows, every copy in flight at once; the other
+        // slots, and the rows up to a multiple of four, are zero
+#pragma unroll
+        for (int k4 = 0; k4 < 32 / NW; ++k4) {
+          const int slot = warp + NW * k4;
           double* dst = S + (size_t)slot * ms;
-          for (int r = lane; r < m; r += 32) cp_async8(dst + r, src + r);
+          if (valid(slot)) {
+            const double* src = D.X + (long long)act[slot < 16 ? bi * 16 + slot : bj * 16 + slot - 16] * D.ldx;
+            if (vec) {
+              for (int r = 2 * lane; r + 1 < m; r += 64) cp_async16(dst + r, src + r);
+              if ((m & 1) && lane == 0) cp_async8(dst + m - 1, src + m - 1);
+            } else {
+              for (int r = lane; r < m; r += 32) cp_async8(dst + r, src + r);
+            }
+            if (m + lane < m4) dst[m + lane] = 0.0;
+          } else {
+            for (int r = lane; r < m4; r += 32) dst[r] = 0.0;
+          }
         }
         asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
         __syncthreads();
-        auto valid = [&](int slot) { return slot < 16 ? slot < cI : slot - 16 < cJ; };
-        // G = S^T S: 16 tiles of 8 x 8, tiles warp and warp + 8 of each warp in one K loop, two
-        // accumulator chains per tile
+        // G = S^T S, scaled: the upper ten tiles, each quarter of the rows by two warps
         {
-          const int t0 = warp, t1 = warp + NW;
-          const int ca0 = 8 * (t0 >> 2) + qr, cb0 = 8 * (t0 & 3) + qr;
-          const int ca1 = 8 * (t1 >> 2) + qr, cb1 = 8 * (t1 & 3) + qr;
-          const bool va0 = valid(ca0), vb0 = valid(cb0), va1 = valid(ca1), vb1 = valid(cb1);
-          const double* Sa0 = S + (size_t)ca0 * ms;
-          const double* Sb0 = S + (size_t)cb0 * ms;
-          const double* Sa1 = S + (size_t)ca1 * ms;
-          const double* Sb1 = S + (size_t)cb1 * ms;
-          double g[4][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
-          for (int k0 = 0; k0 < m; k0 += 8) {
-            const int k = k0 + qc, k2 = k0 + 4 + qc;
-            const bool in1 = k < m, in2 = k2 < m;
-            dmma(g[0][0], g[0][1], (va0 && in1) ? Sa0[k] : 0.0, (vb0 && in1) ? Sb0[k] : 0.0);
-            dmma(g[1][0], g[1][1], (va0 && in2) ? Sa0[k2] : 0.0, (vb0 && in2) ? Sb0[k2] : 0.0);
-            dmma(g[2][0], g[2][1], (va1 && in1) ? Sa1[k] : 0.0, (vb1 && in1) ? Sb1[k] : 0.0);
-            dmma(g[3][0], g[3][1], (va1 && in2) ? Sa1[k2] : 0.0, (vb1 && in2) ? Sb1[k2] : 0.0);
-          }
-          G[ca0 + (8 * (t0 & 3) + 2 * qc) * GLD] = g[0][0] + g[1][0];
-          G[ca0 + (8 * (t0 & 3) + 2 * qc + 1) * GLD] = g[0][1] + g[1][1];
-          G[ca1 + (8 * (t1 & 3) + 2 * qc) * GLD] = g[2][0] + g[3][0];
-          G[ca1 + (8 * (t1 & 3) + 2 * qc + 1) * GLD] = g[2][1] + g[3][1];
+          const double* Sq = S + qr * ms + qc;
+          const int hw = warp & 1;
+          double g[5][2] = {};
+          // four K steps' fragments in flight; the two halves of the tiles in loops of their own (a branch
+          // inside the loop is turned into predicated multiplications, which take the tensor core's time
+          // all the same: 5400 cycles against 2870 at 256 rows)
+          auto loop = [&](auto step) {
+            int k = kbeg;
+            for (; k + 16 <= kend; k += 16) {
+              double f[4][4];
+#pragma unroll
+              for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int t = 0; t < 4; ++t) f[u][t] = Sq[8 * t * ms + k + 4 * u];
+#pragma unroll
+              for (int u = 0; u < 4; ++u) step(f[u][0], f[u][1], f[u][2], f[u][3]);
+            }
+            for (; k < kend; k += 4) step(Sq[k], Sq[8 * ms + k], Sq[16 * ms + k], Sq[24 * ms + k]);
+          };
+          if (hw == 0)
+            loop([&](double f0, double f1, double f2, double f3) {
+              dmma(g[0][0], g[0][1], f0, f0);
+              dmma(g[1][0], g[1][1], f0, f1);
+              dmma(g[2][0], g[2][1], f0, f2);
+              dmma(g[3][0], g[3][1], f0, f3);
+              dmma(g[4][0], g[4][1], f1, f1);
+            });
+          else
+            loop([&](double, double f1, double f2, double f3) {
+              dmma(g[0][0], g[0][1], f1, f2);
+              dmma(g[1][0], g[1][1], f1, f3);
+              dmma(g[2][0], g[2][1], f2, f2);
+              dmma(g[3][0], g[3][1], f2, f3);
+              dmma(g[4][0], g[4][1], f3, f3);
+            });
+          double* pt = part + (warp >> 1) * kGramPart + hw * 320 + lane * 2;
+#pragma unroll
+          for (int t = 0; t < 5; ++t) *reinterpret_cast<double2*>(pt + 64 * t) = make_double2(g[t][0], g[t][1]);
+        }
+        __syncthreads();
+        for (int e = tid; e < kGramPart; e += NT) {
+          const double v = ((part[e] + part[kGramPart + e]) + (part[2 * kGramPart + e] + part[3 * kGramPart + e])) * q.sc;
+          const int t = e >> 6, l = (e & 63) >> 1;
+          const int a = t < 4 ? 0 : (t < 7 ? 1 : (t < 9 ? 2 : 3)), b = t < 4 ? t : (t < 7 ? t - 3 : (t < 9 ? t - 5 : 3));
+          const int i = 8 * a + (l >> 2), j = 8 * b + 2 * (l & 3) + (e & 1);
+          if (i <= j) G[i + j * GLD] = v;
         }
         __syncthreads();
         // does any pair of this visit (all slot pairs in round 0, the cross pairs later) need a rotation?
         int need = 0;
-        for (int e = tid; e < 32 * 32; e += NT) {
-          const int i = e & 31, j = e >> 5;
-          if (i < j && (full || (i < 16 && j >= 16)) && valid(i) && valid(j)) {
-            const double al = G[i * (GLD + 1)] * q.sc, be = G[j * (GLD + 1)] * q.sc, ga = G[i + j * GLD] * q.sc;
-            if (al > q.zthr && be > q.zthr && ga * ga > q.tol2 * al * be) need = 1;
+#pragma unroll
+        for (int k4 = 0; k4 < 4; ++k4) {
+          const int e = tid + NT * k4, i = e & 31, j = e >> 5;
+          if (i < j && (full || (i < 16 && j >= 16))) {
+            const double al = G[i * (GLD + 1)], be = G[j * (GLD + 1)], ga = G[i + j * GLD];
+            need |= (al > q.zthr) && (be > q.zthr) && (ga * ga > q.tol2 * al * be);
           }
         }
         if (!__syncthreads_or(need)) continue;   // block pair unchanged
         if (tid < 16) {   // the rotations of inner round 0 (pair index = tid)
-          const int x = full ? rr_player(tid, 0, 32) : tid, y = full ? rr_player(31 - tid, 0, 32) : 16 + tid;
-          set_pair(s_ra[0][tid], s_rb[0][tid], x, y, G[x * (GLD + 1)], G[y * (GLD + 1)], G[x + y * GLD], q);
+          const int x = tid, y = full ? 31 - tid : 16 + tid;
+          const double al = G[x * (GLD + 1)], be = G[y * (GLD + 1)], ga = G[x + y * GLD];
+          const Rot R = make_rot_nb(al, be, ga, q);
+          s_csp[0][tid] = make_double2(R.c, -R.s);
+          s_dg[0][2 * tid] = fma(-R.t, ga, al);
+          s_dg[0][2 * tid + 1] = fma(R.t, ga, be);
+          s_off[0][tid] = R.apply ? 0.0 : ga;
+          const unsigned b = __ballot_sync(0xffffu, R.apply);
+          if (tid == 0) s_rot = b != 0;
         }
-        if (tid == 0) s_rot = 0;
         __syncthreads();
-        if (tid < 16 && s_ra[0][tid].on) s_rot = 1;
-        {
-          // V = I, its rows in the registers of warp 6 during the inner rounds
-          double vrow[32];
-#pragma unroll
-          for (int c = 0; c < 32; ++c) vrow[c] = (c == lane) ? 1.0 : 0.0;
-          unsigned long long pre = (warp == 3 && lane < 16) ? s_sched[16 + lane] : 0ull;
-          if (full) {
-            for (int r = 0; r < 31; ++r)
-              gram_round<true>(G, vrow, s_ra[r & 1], s_rb[r & 1], s_ra[(r + 1) & 1], s_rb[(r + 1) & 1], s_blk, s_sched,
-                               r, 31, q, &s_rot, pre);
-          } else {
-            for (int r = 0; r < 16; ++r)
-              gram_round<false>(G, vrow, s_ra[r & 1], s_rb[r & 1], s_ra[(r + 1) & 1], s_rb[(r + 1) & 1], s_blk,
-                                s_sched, r, 16, q, &s_rot, pre);
-          }
-          if (warp == 6) {
-#pragma unroll
-            for (int c = 0; c < 32; ++c) V[lane + c * GLD] = vrow[c];
-          }
-        }
-        any |= (s_rot != 0);
+        const bool rot = full ? inner_rounds<true>(G, V, s_csp, s_dg, s_off, q)
+                              : inner_rounds<false>(G, V, s_csp, s_dg, s_off, q);
+        if (rot) s_rot = 1;
         __syncthreads();   // V complete
-        // columns <- S V, written to the problem's columns: 8-row tiles dealt to the warps
-        for (int rt = warp; rt * 8 < m; rt += 2 * NW) {   // row tiles rt and rt + NW
-          const int r0 = rt * 8 + qr, r1 = (rt + NW) * 8 + qr;   // A rows (lane / 4) = C rows
-          double c[2][4][2] = {};
+        any |= (s_rot != 0);
+        // columns <- S V, written to the problem's columns: 8-row tiles dealt to the warps, V's fragments
+        // in registers
+        {
+          double vf[8][4];
 #pragma unroll
-          for (int k0 = 0; k0 < 32; k0 += 4) {
-            const int k = k0 + qc;
-            const bool vk = valid(k);
-            const double a0 = (vk && r0 < m) ? S[(size_t)k * ms + r0] : 0.0;
-            const double a1 = (vk && r1 < m) ? S[(size_t)k * ms + r1] : 0.0;
+          for (int k = 0; k < 8; ++k)
 #pragma unroll
-            for (int tn = 0; tn < 4; ++tn) {
-              const double b = V[k + (8 * tn + qr) * GLD];
-              dmma(c[0][tn][0], c[0][tn][1], a0, b);
-              dmma(c[1][tn][0], c[1][tn][1], a1, b);
-            }
+            for (int tn = 0; tn < 4; ++tn) vf[k][tn] = V[4 * k + qc + (8 * tn + qr) * GLD];
+          int off[8];                           // this lane's columns of X (slots 8 tn + 2 qc + e), -1: none
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const int slot = 8 * (u >> 1) + 2 * qc + (u & 1);
+            off[u] = valid(slot) ? (slot < 16 ? act[bi * 16 + slot] : act[bj * 16 + slot - 16]) * D.ldx : -1;
           }
+          double a[8];
+          const double* Sa = S + qc * ms;
+          if (warp * 8 < m) {
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int rw = u ? r1 : r0;
-            if (rw >= m) continue;
+            for (int k = 0; k < 8; ++k) a[k] = Sa[(size_t)(4 * k) * ms + warp * 8 + qr];
+          }
+          for (int r0 = warp * 8 + qr; r0 - qr < m; r0 += 8 * NW) {
+            double c[4][2] = {}, an[8];
+            // the next tile's rows (the last tile loads its own again) while this one is multiplied
+            const double* Sn = Sa + (r0 - qr + 8 * NW < m ? r0 + 8 * NW : r0);
 #pragma unroll
-            for (int tn = 0; tn < 4; ++tn)
+            for (int k = 0; k < 8; ++k) an[k] = Sn[4 * k * ms];
 #pragma unroll
-              for (int e = 0; e < 2; ++e) {
-                const int slot = 8 * tn + 2 * qc + e;
-                if (valid(slot)) {
-                  const int col = slot < 16 ? act[bi * 16 + slot] : act[bj * 16 + slot - 16];
-                  D.X[(long long)col * D.ldx + rw] = c[u][tn][e];
-                }
-              }
+            for (int k = 0; k < 8; ++k) {
+#pragma unroll
+              for (int tn = 0; tn < 4; ++tn) dmma(c[tn][0], c[tn][1], a[k], vf[k][tn]);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) a[k] = an[k];
+            if (r0 < m) {
+#pragma unroll
+              for (int u = 0; u < 8; ++u)
+                if (off[u] >= 0) D.X[off[u] + r0] = c[u >> 1][u & 1];
+            }
           }
         }
         __syncthreads();   // S and V are read before the next visit loads
@@ -1212,7 +1220,10 @@ static void launch_jacobi_block(const JacobiDesc* d_descs, int count, int max_m,
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(count * csize));
   cfg.blockDim = dim3(NT);
-  cfg.dynamicSmemBytes = smem;
+  // Launches that leave every CTA an SM of its own ask for more than half of an SM's shared memory:
+  // otherwise two CTAs of a cluster may land on one SM and share its tensor cores (one 248 x 248 problem
+  // 1.37 ms, 1.30 apart)
+  cfg.dynamicSmemBytes = (size_t)count * csize <= (size_t)current_sm_count() ? std::max(smem, kLoneCtaSmem) : smem;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
