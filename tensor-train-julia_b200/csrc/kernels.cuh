@@ -5,14 +5,20 @@
 namespace ttc {
 
 // ---- grouped FP64 GEMM (gemm_f64.cu)
-void launch_gemm_f64(const GemmDesc* d_descs, int nd, long long total_tiles, cudaStream_t s);
-// ---- the same problems with float data in A, B and C, FP32 accumulation (gemm_f32.cu)
-void launch_gemm_f32(const GemmDesc* d_descs, int nd, long long total_tiles, cudaStream_t s);
-long long gemm_tiles(const GemmDesc& d);
-// Split-K count for one FP64 problem of a launch of launch_tiles output tiles on nsm SMs (1: no
+// tile: one of the output tile shapes (gemm_pick_tile), for which the descriptors' tile_start is filled.
+constexpr int kGemmTiles = 3;
+void launch_gemm_f64(const GemmDesc* d_descs, int nd, long long total_tiles, int tile, cudaStream_t s);
+// The tile shape for one launch of nd problems (ksplit set) on nsm SMs.
+int gemm_pick_tile(const GemmDesc* d, int nd, int nsm);
+long long gemm_tiles(const GemmDesc& d, int tile);
+// Tile 0 (64 x 64), in which the K splits are counted.
+constexpr int kGemmRefTile = 0;
+// Split-K count for one FP64 problem of a launch of launch_tiles reference tiles on nsm SMs (1: no
 // split), and the partial-tile workspace (doubles) a split problem needs.
 int gemm_pick_ksplit(const GemmDesc& d, long long launch_tiles, int nsm);
-long long gemm_split_ws_doubles(const GemmDesc& d);
+long long gemm_split_ws_doubles(const GemmDesc& d, int tile);
+// ---- the same problems with float data in A, B and C, FP32 accumulation (gemm_f32.cu)
+void launch_gemm_f32(const GemmDesc* d_descs, int nd, long long total_tiles, cudaStream_t s);
 
 // Device-side size bound: min(cap, mult * *p) when p is given (a rank that an earlier kernel of
 // the same plan wrote), else cap.  Rows or columns beyond the bound are exactly zero in the

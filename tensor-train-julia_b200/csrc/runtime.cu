@@ -143,7 +143,7 @@ static void launch_op(ttc_context* c, const Plan& p, const Op& op) {
   {
     const unsigned char* d = p.d_blob + op.off;
     switch (op.kind) {
-      case OP_GEMM: launch_gemm_f64((const GemmDesc*)d, op.count, op.total, s); break;
+      case OP_GEMM: launch_gemm_f64((const GemmDesc*)d, op.count, op.total, op.a, s); break;
       case OP_QR:
         if (op.total) launch_qr_seq((const QRDesc*)d, op.count, op.a, s, c->d_flags);
         else launch_qr((const QRDesc*)d, op.count, op.a, s, c->d_flags);
@@ -411,37 +411,38 @@ const int* Builder::const_ints(const std::vector<int>& v) {
 }
 void Builder::gemm(std::vector<GemmDesc> v) {
   std::vector<GemmDesc> w;
-  long long out_tiles = 0;
+  long long ref_tiles = 0;
   for (auto& d : v) {
     d.ksplit = 1; d.ws = nullptr; d.cnt = nullptr;
-    out_tiles += gemm_tiles(d);
-  }
-  const int nsm = current_sm_count();
-  long long t = 0;
-  for (auto& d : v) {
-    if (gemm_tiles(d) == 0) continue;
+    if (gemm_tiles(d, kGemmRefTile) == 0) continue;
     if (d.m0 <= 0) d.m0 = std::max(d.m, 1);
     if (d.n0 <= 0) d.n0 = std::max(d.n, 1);
     if (d.k0e <= 0) d.k0e = std::max(d.k, 1);
     if (wsbase) check_gemm(d);
-    const long long tiles_out = gemm_tiles(d);
-    d.ksplit = gemm_pick_ksplit(d, out_tiles, nsm);
+    ref_tiles += gemm_tiles(d, kGemmRefTile);
+    w.push_back(d);
+  }
+  if (w.empty()) return;
+  const int nsm = current_sm_count();
+  for (auto& d : w) d.ksplit = gemm_pick_ksplit(d, ref_tiles, nsm);
+  const int tile = gemm_pick_tile(w.data(), (int)w.size(), nsm);
+  long long t = 0;
+  for (auto& d : w) {
     if (d.ksplit > 1) {
-      d.ws = wd((size_t)gemm_split_ws_doubles(d));
+      d.ws = wd((size_t)gemm_split_ws_doubles(d, tile));
       // one counter per output tile, zero in the plan blob; the kernel leaves them zero
+      const long long tiles_out = gemm_tiles(d, tile) / d.ksplit;
       const size_t o = plan->push(std::vector<unsigned>((size_t)tiles_out, 0u));
       d.cnt = reinterpret_cast<unsigned*>(blob_base + o);
       if (wsbase) {
-        region_check(d.ws, sizeof(double) * (size_t)gemm_split_ws_doubles(d), "gemm split-K partials");
+        region_check(d.ws, sizeof(double) * (size_t)gemm_split_ws_doubles(d, tile), "gemm split-K partials");
         region_check(d.cnt, sizeof(unsigned) * (size_t)tiles_out, "gemm split-K counters");
       }
     }
     d.tile_start = t;
-    t += gemm_tiles(d);
-    w.push_back(d);
+    t += gemm_tiles(d, tile);
   }
-  if (w.empty()) return;
-  Op op; op.kind = OP_GEMM; op.off = plan->push(w); op.count = (int)w.size(); op.total = t;
+  Op op; op.kind = OP_GEMM; op.off = plan->push(w); op.count = (int)w.size(); op.total = t; op.a = tile;
   for (auto& d : w) op.flops += 2.0 * d.m * d.n * d.k * std::max(1, d.batch);
   plan->ops.push_back(op);
 }
@@ -449,7 +450,7 @@ void Builder::gemm32(std::vector<GemmDesc> v) {
   std::vector<GemmDesc> w;
   long long t = 0;
   for (auto& d : v) {
-    const long long n = gemm_tiles(d);
+    const long long n = gemm_tiles(d, kGemmRefTile);
     if (n == 0) continue;
     if (d.m0 <= 0) d.m0 = std::max(d.m, 1);
     if (d.n0 <= 0) d.n0 = std::max(d.n, 1);

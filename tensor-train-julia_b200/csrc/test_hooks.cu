@@ -152,7 +152,7 @@ int ttc_test_gemm_runs(ttc_context* c, int m, int n, int k, int batch, int m0, i
       d.C = dC.as<double>(); d.c_i0 = cs[0]; d.c_i1 = cs[1]; d.c_j0 = cs[2]; d.c_j1 = cs[3]; d.c_b = cs[4];
       d.alpha = alpha; d.beta = beta;
       B.gemm({d});
-      ks = gemm_pick_ksplit(d, gemm_tiles(d), current_sm_count());
+      ks = gemm_pick_ksplit(d, gemm_tiles(d, kGemmRefTile), current_sm_count());
     });
     for (int r = 0; r < runs; ++r) run_plan(c, *p);
     TTC_CUDA(cudaStreamSynchronize(c->stream));
