@@ -9,6 +9,10 @@
 namespace ttc {
 
 void ensure_stage(ttc_context* c, size_t bytes);
+struct HostCopy { void* dst; const void* src; size_t bytes; };
+void parallel_memcpy(const std::vector<HostCopy>& cps);
+// The pieces lie one after another in the staging area (src: their place in the pinned half).
+void staged_download(ttc_context* c, const std::vector<HostCopy>& pieces);
 void validate_ttv(const ttc_ttv* x);
 // Upload m host TTs into batch slots [first, first+m).  With `reverse`, slot core k holds
 // core N-1-k of the host TT with its two rank indices swapped (the mirror-image TT).
@@ -65,6 +69,7 @@ struct DevTTO {
   std::vector<int> rks;
   std::vector<long long> off;
   double* d = nullptr;
+  ttc_context* ctx = nullptr;
   ~DevTTO();
   double* core(int k) const { return d + off[k]; }
 };

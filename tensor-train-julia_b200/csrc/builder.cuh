@@ -65,9 +65,16 @@ CopyDesc cd3(const double* src, double* dst, long long e0, long long e1, long lo
 Plan* get_plan(ttc_context* c, const std::string& key, const std::function<void(Builder&)>& fn);
 void run_plan(ttc_context* c, Plan& p);
 void ensure_workspace(ttc_context* c, size_t bytes);
+// cudaMalloc that gives the context's idle blocks back and tries once more when memory runs out.
+cudaError_t dev_malloc(ttc_context* c, void** p, size_t bytes);
+// A device block for the duration of one call, from the context's idle blocks where one fits, and its
+// return (waits for the context's stream).  block_trim frees every idle block.
+cudaError_t block_get(ttc_context* c, void** p, size_t bytes);
+void block_put(ttc_context* c, void* p) noexcept;
+void block_trim(ttc_context* c) noexcept;
 void check_device_flags(ttc_context* c);
 
-ttc_batch* batch_create(ttc_context* c, int count, int N, const long long* dims, const int* cap);
+ttc_batch* batch_create(ttc_context* c, int count, int N, const long long* dims, const int* cap, bool pooled = true);
 void batch_destroy(ttc_batch* b);
 void batch_sync_ranks(ttc_batch* b);
 std::string batch_key(const ttc_batch* b);

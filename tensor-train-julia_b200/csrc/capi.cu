@@ -44,7 +44,7 @@ void ensure_stage(ttc_context* c, size_t bytes) {
   if (c->h_stage) cudaFreeHost(c->h_stage);
   c->d_stage = nullptr; c->h_stage = nullptr; c->stage_bytes = 0;
   const size_t nb = bytes + bytes / 4 + (1 << 16);
-  if (cudaMalloc(&c->d_stage, nb) != cudaSuccess) { cudaGetLastError(); throw Error(TTC_ENOMEM, "staging allocation failed"); }
+  if (dev_malloc(c, &c->d_stage, nb) != cudaSuccess) { throw Error(TTC_ENOMEM, "staging allocation failed"); }
   if (cudaMallocHost(&c->h_stage, nb) != cudaSuccess) { cudaGetLastError(); throw Error(TTC_ENOMEM, "pinned staging allocation failed"); }
   c->stage_bytes = nb;
   region_add(c->d_stage, nb);
@@ -55,12 +55,11 @@ static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 // Host copies of a transfer (dst, src, bytes), split over host threads: packing hundreds of MB
 // into the pinned staging buffer is bound by host memory bandwidth, which one thread does not
 // reach.  Small transfers stay on the calling thread.
-struct HostCopy { void* dst; const void* src; size_t bytes; };
 // Host staging is done in chunks of about this many bytes, each chunk's transfer overlapping
 // the staging of the next.
 constexpr size_t kStageChunk = 48u << 20;
 
-static void parallel_memcpy(const std::vector<HostCopy>& cps) {
+void parallel_memcpy(const std::vector<HostCopy>& cps) {
   size_t total = 0;
   for (const auto& c : cps) total += c.bytes;
   const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
@@ -83,6 +82,38 @@ static void parallel_memcpy(const std::vector<HostCopy>& cps) {
   for (unsigned i = 1; i < nt; ++i) th.emplace_back(work, total * i / nt, total * (i + 1) / nt);
   work(0, total / nt);
   for (auto& t : th) t.join();
+}
+
+// Brings the start of the device staging area to the pinned one, and each piece of it to its place.
+void staged_download(ttc_context* c, const std::vector<HostCopy>& hcp) {
+  // transfer chunk by chunk, an event after each; unpack a chunk while the next ones arrive
+  std::vector<std::pair<size_t, size_t>> groups;   // [gi, gj) of hcp
+  std::vector<cudaEvent_t> evs;
+  size_t sent = 0;
+  try {
+    for (size_t gi = 0; gi < hcp.size();) {
+      size_t gj = gi, bytes = 0;
+      while (gj < hcp.size() && (gj == gi || bytes < kStageChunk)) bytes += hcp[gj++].bytes;
+      cudaEvent_t e;
+      TTC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      evs.push_back(e);
+      TTC_CUDA(cudaMemcpyAsync((char*)c->h_stage + sent, (char*)c->d_stage + sent, bytes, cudaMemcpyDeviceToHost, c->stream));
+      TTC_CUDA(cudaEventRecord(e, c->stream));
+      groups.push_back({gi, gj});
+      sent += bytes;
+      gi = gj;
+    }
+    for (size_t g = 0; g < groups.size(); ++g) {
+      TTC_CUDA(cudaEventSynchronize(evs[g]));
+      parallel_memcpy(std::vector<HostCopy>(hcp.begin() + (long)groups[g].first, hcp.begin() + (long)groups[g].second));
+    }
+  } catch (...) {
+    cudaStreamSynchronize(c->stream);
+    for (auto e : evs) cudaEventDestroy(e);
+    throw;
+  }
+  TTC_CUDA(cudaStreamSynchronize(c->stream));
+  for (auto e : evs) cudaEventDestroy(e);
 }
 
 void validate_ttv(const ttc_ttv* x) {
@@ -270,34 +301,7 @@ void batch_download_many(ttc_batch* b, int first, int m, ttc_ttv_out* ys, bool r
         hcp.push_back({ys[i].cores[ko], (double*)h + offs[q++], cnt * sizeof(double)});
       }
     }
-    // transfer chunk by chunk, an event after each; unpack a chunk while the next ones arrive
-    std::vector<std::pair<size_t, size_t>> groups;   // [gi, gj) of hcp
-    std::vector<cudaEvent_t> evs;
-    size_t sent = 0;
-    try {
-      for (size_t gi = 0; gi < hcp.size();) {
-        size_t gj = gi, bytes = 0;
-        while (gj < hcp.size() && (gj == gi || bytes < kStageChunk)) bytes += hcp[gj++].bytes;
-        cudaEvent_t e;
-        TTC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        evs.push_back(e);
-        TTC_CUDA(cudaMemcpyAsync(h + sent, d + sent, bytes, cudaMemcpyDeviceToHost, c->stream));
-        TTC_CUDA(cudaEventRecord(e, c->stream));
-        groups.push_back({gi, gj});
-        sent += bytes;
-        gi = gj;
-      }
-      for (size_t g = 0; g < groups.size(); ++g) {
-        TTC_CUDA(cudaEventSynchronize(evs[g]));
-        parallel_memcpy(std::vector<HostCopy>(hcp.begin() + (long)groups[g].first, hcp.begin() + (long)groups[g].second));
-      }
-    } catch (...) {
-      cudaStreamSynchronize(c->stream);
-      for (auto e : evs) cudaEventDestroy(e);
-      throw;
-    }
-    TTC_CUDA(cudaStreamSynchronize(c->stream));
-    for (auto e : evs) cudaEventDestroy(e);
+    staged_download(c, hcp);
   }
   for (int i = 0; i < m; ++i) {
     const int t = first + i;
@@ -401,7 +405,7 @@ std::vector<const double*> upload_host_blocks(ttc_context* c, const std::vector<
   if (total > c->sk_cap) {
     if (c->d_sk) { region_remove(c->d_sk); cudaFree(c->d_sk); }
     c->d_sk = nullptr;
-    TTC_CUDA(cudaMalloc(&c->d_sk, total * sizeof(double)));
+    TTC_CUDA(dev_malloc(c, (void**)&c->d_sk, total * sizeof(double)));
     region_add(c->d_sk, total * sizeof(double));
     c->sk_cap = total;
   }
@@ -469,6 +473,7 @@ int ttc_destroy(ttc_context* c) {
     oneshot_clear(c);
   } catch (...) {
   }
+  block_trim(c);
   for (void* p : {(void*)c->ws, c->d_stage, (void*)c->d_sk, (void*)c->d_flags, (void*)c->d_one}) region_remove(p);
   if (c->ws) cudaFree(c->ws);
   if (c->d_stage) cudaFree(c->d_stage);
@@ -527,7 +532,7 @@ int ttc_batch_create(ttc_context* c, int32_t count, int32_t N, const int64_t* di
     for (int t = 0; t < count; ++t)
       TTC_REQUIRE(cp[(size_t)t * (N + 1)] == 1 && cp[(size_t)t * (N + 1) + N] == 1, TTC_EDIM,
                   "batch: boundary capacities must be 1");
-    *out = batch_create(c, count, N, d.data(), cp.data());
+    *out = batch_create(c, count, N, d.data(), cp.data(), false);   // the caller's, freed with it
   });
 }
 

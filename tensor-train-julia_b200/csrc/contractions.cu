@@ -30,7 +30,7 @@ static void run_once(ttc_context* c, const std::function<void(Builder&)>& fn) {
 
 // ---------------------------------------------------------------- TToperator upload
 DevTTO::~DevTTO() {
-  if (d) { region_remove(d); cudaFree(d); }
+  block_put(ctx, d);
 }
 
 DevTTO* tto_upload(ttc_context* c, const ttc_tto* H) {
@@ -38,6 +38,7 @@ DevTTO* tto_upload(ttc_context* c, const ttc_tto* H) {
   std::unique_ptr<DevTTO> D(new DevTTO());
   const int N = H->N;
   D->N = N;
+  D->ctx = c;
   D->dims.assign(H->dims, H->dims + N);
   D->rks.assign(H->rks, H->rks + N + 1);
   TTC_REQUIRE(D->rks[0] == 1, TTC_EDIM, "TToperator: first rank must be 1");
@@ -48,8 +49,7 @@ DevTTO* tto_upload(ttc_context* c, const ttc_tto* H) {
     D->off[k] = o;
     o += (D->rks[k] * D->dims[k] * D->dims[k] * (long long)D->rks[k + 1] + 31) & ~31LL;
   }
-  TTC_CUDA(cudaMalloc(&D->d, sizeof(double) * std::max<long long>(o, 1)));
-  region_add(D->d, sizeof(double) * std::max<long long>(o, 1));
+  TTC_CUDA(block_get(c, (void**)&D->d, sizeof(double) * std::max<long long>(o, 1)));
   ensure_stage(c, sizeof(double) * o + 256 + sizeof(CopyDesc) * N);
   double* hs = (double*)c->h_stage;
   std::vector<CopyDesc> cp;
@@ -527,11 +527,17 @@ double dot_host(ttc_context* c, const ttc_ttv* a, const ttc_ttv* b, double* cons
       }
     }
   });
-  std::vector<double> h(tot);
-  TTC_CUDA(cudaMemcpy(h.data(), Wd, tot * sizeof(double), cudaMemcpyDeviceToHost));
-  if (W_out)
-    for (int k = 0; k <= N; ++k)
-      std::memcpy(W_out[k], h.data() + off[k], (size_t)A->rk(0, k) * Bt->rk(0, k) * sizeof(double));
+  const double* h = (const double*)c->h_stage;
+  if (!W_out) {
+    const size_t at = reverse ? off[0] : off[N];
+    TTC_CUDA(cudaMemcpyAsync(c->h_stage, Wd + at, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    TTC_CUDA(cudaStreamSynchronize(c->stream));
+    return h[0];
+  }
+  std::vector<HostCopy> out;
+  for (int k = 0; k <= N; ++k)
+    out.push_back({W_out[k], h + off[k], (size_t)A->rk(0, k) * Bt->rk(0, k) * sizeof(double)});
+  staged_download(c, out);
   return reverse ? h[off[0]] : h[off[N]];
 }
 
@@ -766,13 +772,12 @@ void rayleigh_grad_host(ttc_context* c, const ttc_tto* Hh, const ttc_ttv* x, int
   float* Xf = nullptr;
   float* Hf = nullptr;
   std::vector<double*> own;
-  struct FreeV { std::vector<double*>& v; ~FreeV() { for (auto* p : v) { region_remove(p); cudaFree(p); } } } fv{own};
+  struct FreeV { ttc_context* c; std::vector<double*>& v; ~FreeV() { for (auto* p : v) block_put(c, p); } } fv{c, own};
   auto dev_alloc = [&](size_t bytes) {
     double* p = nullptr;
-    TTC_CUDA(cudaMalloc(&p, std::max<size_t>(bytes, 16)));
-    own.push_back(p);
-    region_add(p, std::max<size_t>(bytes, 16));
-    return p;
+    own.push_back(nullptr);
+    TTC_CUDA(block_get(c, (void**)&p, bytes));
+    return own.back() = p;
   };
   if (f32) {
     size_t ht = 0;
@@ -897,6 +902,7 @@ void rayleigh_grad_host(ttc_context* c, const ttc_tto* Hh, const ttc_ttv* x, int
   TTC_REQUIRE(nn > 0.0, TTC_EARG, "rayleigh_grad: <x|x> is zero");
   const double Rq = e / nn;
   *value = Rq;
+  ensure_stage(c, sizeof(double) * gsz + 256);        // the gradient in the caller's layout
   // pass 2: right-to-left, recomputing each segment's left environments from its checkpoint
   run_once(c, [&](Builder& B) {
     double* Rh = B.wd(1); double* Rn = B.wd(1);
@@ -965,24 +971,26 @@ void rayleigh_grad_host(ttc_context* c, const ttc_tto* Hh, const ttc_ttv* x, int
       GEMM(B, {gd(r0, r0, n * r1, Tn, 1, r0, xcore(k), xc, 1, Rn_new, 1, r0)});
       Rh = Rh_new; Rn = Rn_new;
     }
+    // internal (a, i, d) -> Julia (i, a, d) in the staging area
+    const double* src = dG;
+    if (f32) {
+      double* wide = B.wd(gsz);
+      CvtDesc w{};
+      w.src = dG; w.dst = wide; w.rows = (long long)gsz; w.cols = 1; w.ss_i = 1; w.ds_i = 1; w.alpha = 1.0;
+      B.widen({w});
+      src = wide;
+    }
+    std::vector<CopyDesc> cp;
+    for (int k = 0; k < N; ++k) {
+      const long long r0 = rk(k), r1 = rk(k + 1), n = X->dims[k];
+      cp.push_back(cd3(src + goff[k], (double*)c->d_stage + goff[k], n, r0, r1, r0, 1, r0 * n, 1, n, n * r0));
+    }
+    B.copy(cp);
   });
-  std::vector<double> hg(gsz);
-  if (f32) {
-    std::vector<float> hf(gsz);
-    TTC_CUDA(cudaMemcpy(hf.data(), dG, gsz * sizeof(float), cudaMemcpyDeviceToHost));
-    for (size_t e = 0; e < gsz; ++e) hg[e] = hf[e];
-  } else {
-    TTC_CUDA(cudaMemcpy(hg.data(), dG, gsz * sizeof(double), cudaMemcpyDeviceToHost));
-  }
-  // internal (a, i, d) -> Julia (i, a, d)
-  for (int k = 0; k < N; ++k) {
-    const int r0 = rk(k), r1 = rk(k + 1), n = (int)X->dims[k];
-    const double* src = hg.data() + goff[k];
-    double* dst = grads[k];
-    for (int d = 0; d < r1; ++d)
-      for (int a = 0; a < r0; ++a)
-        for (int i = 0; i < n; ++i) dst[i + (size_t)n * (a + (size_t)r0 * d)] = src[a + (size_t)r0 * (i + (size_t)n * d)];
-  }
+  std::vector<HostCopy> out;
+  for (int k = 0; k < N; ++k)
+    out.push_back({grads[k], (const double*)c->h_stage + goff[k], (size_t)rk(k) * X->dims[k] * rk(k + 1) * sizeof(double)});
+  staged_download(c, out);
 }
 
 }  // namespace ttc

@@ -774,7 +774,7 @@ Plan* get_plan(ttc_context* c, const std::string& key, const std::function<void(
   ensure_workspace(c, meas->ws_needed);
   std::unique_ptr<Plan> p(new Plan());
   const size_t blob_cap = meas->blob.size() + 256;
-  TTC_CUDA(cudaMalloc(&p->d_blob, blob_cap));
+  TTC_CUDA(dev_malloc(c, (void**)&p->d_blob, blob_cap));
   region_add(p->d_blob, blob_cap);
   p->d_blob_cap = blob_cap;
   {
@@ -793,6 +793,90 @@ Plan* get_plan(ttc_context* c, const std::string& key, const std::function<void(
   return raw;
 }
 
+// ---------------------------------------------------------------- device blocks of one-shot calls
+// A one-shot call holds its operands on the device for the call's duration only.  cudaMalloc and cudaFree
+// of a block of a megabyte or more map and unmap memory, 100 to 300 us a pair and tens of milliseconds
+// where the driver gives back a large mapping: of a dot and a partial contraction at ranks 128 x 77
+// (6.2 ms) they took 2.7 ms, of a gradient at r 192 (20 ms at best, 60 at times) 5 to 50.  Blocks of that
+// size are kept by their context, up to kPoolBytes together, and freed with it or when memory runs out;
+// smaller ones come out of the driver's own 2 MB slabs at 2 us and stay with cudaMalloc.
+namespace {
+constexpr size_t kPoolMin = 1u << 20, kPoolBytes = 512u << 20;
+}
+
+void block_trim(ttc_context* c) noexcept {
+  std::lock_guard<std::mutex> lk(c->blocks.mu);
+  for (auto& b : c->blocks.idle) cudaFree(b.p);
+  c->blocks.idle.clear();
+  c->blocks.held = 0;
+}
+
+cudaError_t dev_malloc(ttc_context* c, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    block_trim(c);
+    e = cudaMalloc(p, bytes);
+  }
+  if (e != cudaSuccess) { cudaGetLastError(); *p = nullptr; }
+  return e;
+}
+
+cudaError_t block_get(ttc_context* c, void** p, size_t bytes) {
+  BlockPool& P = c->blocks;
+  *p = nullptr;
+  size_t cap = std::max<size_t>(bytes, 16);
+  if (cap >= kPoolMin) {
+    cap = (cap + (2u << 20) - 1) / (2u << 20) * (2u << 20);
+    std::lock_guard<std::mutex> lk(P.mu);
+    auto best = P.idle.end();                  // the smallest that fits and wastes at most a quarter
+    for (auto it = P.idle.begin(); it != P.idle.end(); ++it)
+      if (it->cap >= cap && it->cap <= cap + cap / 4 && (best == P.idle.end() || it->cap < best->cap)) best = it;
+    if (best != P.idle.end()) {
+      *p = best->p;
+      P.cap[best->p] = best->cap;
+      P.held -= best->cap;
+      P.idle.erase(best);
+    }
+  }
+  if (!*p) {
+    const cudaError_t e = dev_malloc(c, p, cap);
+    if (e != cudaSuccess) return e;
+    if (cap >= kPoolMin) {
+      std::lock_guard<std::mutex> lk(P.mu);
+      P.cap[*p] = cap;
+    }
+  }
+  region_add(*p, std::max<size_t>(bytes, 16));
+  return cudaSuccess;
+}
+
+void block_put(ttc_context* c, void* p) noexcept {
+  if (!p) return;
+  BlockPool& P = c->blocks;
+  region_remove(p);
+  const bool idle = cudaStreamSynchronize(c->stream) == cudaSuccess;   // nothing of the call still uses it
+  std::lock_guard<std::mutex> lk(P.mu);
+  auto it = P.cap.find(p);
+  const size_t cap = it == P.cap.end() ? 0 : it->second;
+  if (it != P.cap.end()) P.cap.erase(it);
+  if (!idle || cap == 0 || cap > kPoolBytes) {
+    cudaFree(p);
+    return;
+  }
+  while (P.held + cap > kPoolBytes) {
+    P.held -= P.idle.front().cap;
+    cudaFree(P.idle.front().p);
+    P.idle.pop_front();
+  }
+  try {
+    P.idle.push_back({p, cap});
+    P.held += cap;
+  } catch (...) {
+    cudaFree(p);
+  }
+}
+
 void ensure_workspace(ttc_context* c, size_t bytes) {
   if (bytes <= c->ws_bytes) return;
   TTC_CUDA(cudaStreamSynchronize(c->stream));
@@ -800,8 +884,7 @@ void ensure_workspace(ttc_context* c, size_t bytes) {
   c->ws = nullptr;
   c->ws_bytes = 0;
   const size_t nb = bytes + bytes / 4 + (1 << 20);
-  if (cudaMalloc(&c->ws, nb) != cudaSuccess) {
-    cudaGetLastError();
+  if (dev_malloc(c, (void**)&c->ws, nb) != cudaSuccess) {
     throw Error(TTC_ENOMEM, "workspace allocation of " + std::to_string(nb) + " bytes failed");
   }
   c->ws_bytes = nb;
@@ -834,10 +917,11 @@ void check_device_flags(ttc_context* c) {
 }
 
 // ---------------------------------------------------------------- batches
-ttc_batch* batch_create(ttc_context* c, int count, int N, const long long* dims, const int* cap) {
+ttc_batch* batch_create(ttc_context* c, int count, int N, const long long* dims, const int* cap, bool pooled) {
   TTC_REQUIRE(count > 0 && N > 0, TTC_EARG, "batch: count and N must be positive");
   std::unique_ptr<ttc_batch> b(new ttc_batch());
   b->ctx = c; b->count = count; b->N = N;
+  b->pooled = pooled;
   b->dims.assign(dims, dims + N);
   for (int k = 0; k < N; ++k) TTC_REQUIRE(dims[k] > 0, TTC_EARG, "batch: dims must be positive");
   b->cap.assign(cap, cap + (size_t)count * (N + 1));
@@ -856,13 +940,12 @@ ttc_batch* batch_create(ttc_context* c, int count, int N, const long long* dims,
   }
   b->tt_off[count] = o;
   b->total = o;
-  if (cudaMalloc(&b->d_cores, sizeof(double) * std::max<long long>(o, 1)) != cudaSuccess) {
-    cudaGetLastError();
+  const size_t core_bytes = sizeof(double) * std::max<long long>(o, 1);
+  if ((pooled ? block_get(c, (void**)&b->d_cores, core_bytes) : dev_malloc(c, (void**)&b->d_cores, core_bytes)) != cudaSuccess)
     throw Error(TTC_ENOMEM, "batch allocation failed");
-  }
-  TTC_CUDA(cudaMalloc(&b->d_rks, sizeof(int) * (size_t)count * (N + 1)));
-  TTC_CUDA(cudaMalloc(&b->d_zero, sizeof(int) * count));
-  region_add(b->d_cores, sizeof(double) * std::max<long long>(o, 1));
+  if (!pooled) region_add(b->d_cores, core_bytes);
+  TTC_CUDA(dev_malloc(c, (void**)&b->d_rks, sizeof(int) * (size_t)count * (N + 1)));
+  TTC_CUDA(dev_malloc(c, (void**)&b->d_zero, sizeof(int) * count));
   region_add(b->d_rks, sizeof(int) * (size_t)count * (N + 1));
   region_add(b->d_zero, sizeof(int) * count);
   TTC_CUDA(cudaMemsetAsync(b->d_cores, 0, sizeof(double) * std::max<long long>(o, 1), c->stream));
@@ -891,7 +974,8 @@ void batch_sync_ranks(ttc_batch* b) {
 void batch_destroy(ttc_batch* b) {
   if (!b) return;
   region_remove(b->d_cores); region_remove(b->d_rks); region_remove(b->d_zero);
-  if (b->d_cores) cudaFree(b->d_cores);
+  if (b->pooled) block_put(b->ctx, b->d_cores);
+  else if (b->d_cores) cudaFree(b->d_cores);
   if (b->d_rks) cudaFree(b->d_rks);
   if (b->d_zero) cudaFree(b->d_zero);
   // plans keyed on this batch stay valid only while it lives

@@ -9,7 +9,9 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <cstring>
+#include <list>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -90,6 +92,17 @@ struct Plan {
 
 }  // namespace ttc
 
+namespace ttc {
+// Idle device blocks of one context (block_get, block_put).
+struct BlockPool {
+  struct Block { void* p; size_t cap; };
+  std::mutex mu;
+  std::list<Block> idle;                       // the one given back last at the end
+  size_t held = 0;                             // bytes of idle
+  std::unordered_map<void*, size_t> cap;       // blocks in use, by address
+};
+}  // namespace ttc
+
 struct ttc_context {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -115,10 +128,12 @@ struct ttc_context {
   // the same shape, most recently used last; reuse also lets the plan cache, which is keyed on
   // batch identity, replay the captured plan
   std::vector<std::pair<std::string, ttc_batch*>> oneshot;
+  ttc::BlockPool blocks;
 };
 
 struct ttc_batch {
   ttc_context* ctx = nullptr;
+  bool pooled = false;               // d_cores comes from the context's block pool
   int count = 0, N = 0;
   std::vector<long long> dims;       // N
   std::vector<int> cap;              // count*(N+1)
