@@ -90,39 +90,32 @@ struct OpEnvStep {
   int batch; long long v_b, s_b, w_b;  // block batching (sketch blocks)
 };
 
-// The three products of a step, each added to the problems of its launch.  T1: r n R1 g doubles, T2: r R n g.
-static void op_env_descs(const OpEnvStep& st, double* T1, double* T2, std::vector<GemmDesc>& g1, std::vector<GemmDesc>& g2,
-                         std::vector<GemmDesc>* g3) {
-  const int r = st.r, r1 = st.r1, R = st.R, R1 = st.R1, n = st.n, g = st.g;
-  // 1. T1[(a,z), (be,ga)] = sum_al A[a,z,al] V[al,(be,ga)]
-  GemmDesc d1 = gd(r * n, R1 * g, r1, st.A, 1, (long long)st.xc * n, st.V, 1, r1, T1, 1, (long long)r * n);
-  d1.m0 = r; d1.a_i0 = 1; d1.a_i1 = st.xc; d1.c_i0 = 1; d1.c_i1 = r;
-  d1.batch = st.batch; d1.b_b = st.v_b; d1.c_b = (long long)r * n * R1 * g;
-  g1.push_back(d1);
-  // 2. T2[a, b, ze, ga] = sum_{z,be} T1[a,z,be,ga] H[b,ze,z,be]
-  GemmDesc d2{};
-  d2.m = r * g; d2.n = R * n; d2.k = n * R1; d2.batch = st.batch;
-  d2.m0 = r; d2.n0 = R; d2.k0e = n;
-  d2.A = T1; d2.a_i0 = 1; d2.a_i1 = (long long)r * n * R1; d2.a_k0 = r; d2.a_k1 = (long long)r * n;
-  d2.a_b = (long long)r * n * R1 * g;
-  d2.B = st.H; d2.b_k0 = (long long)R * n; d2.b_k1 = (long long)R * n * n; d2.b_j0 = 1; d2.b_j1 = R;
-  d2.C = T2; d2.c_i0 = 1; d2.c_i1 = (long long)r * R * n; d2.c_j0 = r; d2.c_j1 = (long long)r * R;
-  d2.c_b = (long long)r * R * n * g;
-  d2.alpha = 1.0; d2.beta = 0.0;
-  g2.push_back(d2);
-  // 3. W[(a,b), c] = sum_{(ze,ga)} T2[(a,b),(ze,ga)] S[(ze,ga), c]
-  if (!g3) return;
-  GemmDesc d3 = gd(r * R, st.cdim, n * g, T2, 1, (long long)r * R, st.S, st.s_k, st.s_c, st.W, 1, (long long)r * R);
-  d3.batch = st.batch; d3.a_b = (long long)r * R * n * g; d3.b_b = st.s_b; d3.c_b = st.w_b;
-  g3->push_back(d3);
-}
-
 static void emit_op_env(Builder& B, const std::vector<OpEnvStep>& steps) {
   std::vector<GemmDesc> g1, g2, g3;
   for (const auto& st : steps) {
-    double* T1 = B.wd((size_t)st.r * st.n * st.R1 * st.g * st.batch);
-    double* T2 = B.wd((size_t)st.r * st.R * st.n * st.g * st.batch);
-    op_env_descs(st, T1, T2, g1, g2, &g3);
+    const int r = st.r, r1 = st.r1, R = st.R, R1 = st.R1, n = st.n, g = st.g;
+    double* T1 = B.wd((size_t)r * n * R1 * g * st.batch);
+    double* T2 = B.wd((size_t)r * R * n * g * st.batch);
+    // 1. T1[(a,z), (be,ga)] = sum_al A[a,z,al] V[al,(be,ga)]
+    GemmDesc d1 = gd(r * n, R1 * g, r1, st.A, 1, (long long)st.xc * n, st.V, 1, r1, T1, 1, (long long)r * n);
+    d1.m0 = r; d1.a_i0 = 1; d1.a_i1 = st.xc; d1.c_i0 = 1; d1.c_i1 = r;
+    d1.batch = st.batch; d1.b_b = st.v_b; d1.c_b = (long long)r * n * R1 * g;
+    g1.push_back(d1);
+    // 2. T2[a, b, ze, ga] = sum_{z,be} T1[a,z,be,ga] H[b,ze,z,be]
+    GemmDesc d2{};
+    d2.m = r * g; d2.n = R * n; d2.k = n * R1; d2.batch = st.batch;
+    d2.m0 = r; d2.n0 = R; d2.k0e = n;
+    d2.A = T1; d2.a_i0 = 1; d2.a_i1 = (long long)r * n * R1; d2.a_k0 = r; d2.a_k1 = (long long)r * n;
+    d2.a_b = (long long)r * n * R1 * g;
+    d2.B = st.H; d2.b_k0 = (long long)R * n; d2.b_k1 = (long long)R * n * n; d2.b_j0 = 1; d2.b_j1 = R;
+    d2.C = T2; d2.c_i0 = 1; d2.c_i1 = (long long)r * R * n; d2.c_j0 = r; d2.c_j1 = (long long)r * R;
+    d2.c_b = (long long)r * R * n * g;
+    d2.alpha = 1.0; d2.beta = 0.0;
+    g2.push_back(d2);
+    // 3. W[(a,b), c] = sum_{(ze,ga)} T2[(a,b),(ze,ga)] S[(ze,ga), c]
+    GemmDesc d3 = gd(r * R, st.cdim, n * g, T2, 1, (long long)r * R, st.S, st.s_k, st.s_c, st.W, 1, (long long)r * R);
+    d3.batch = st.batch; d3.a_b = (long long)r * R * n * g; d3.b_b = st.s_b; d3.c_b = st.w_b;
+    g3.push_back(d3);
   }
   B.gemm(g1);
   B.gemm(g2);
@@ -763,7 +756,7 @@ double norm_host(ttc_context* c, const ttc_ttv* x) {
 // site; the contractions with L_k then go in one launch for all sites.
 // One launch per product, the products with R_{k+1} formed twice and the left chain run again from
 // checkpoints every four sites took 600 launches and 11.6 ms at d 32, r 192, R 18 where this takes 100
-// launches and 4.6 ms; in FP32 19.2 and 6.2 ms.  What is kept per site (r n r R + r r R numbers) is less
+// launches and 4.0 ms; in FP32 19.2 and 3.5 ms (6.2 before the smaller tiles of the FP32 GEMM).  What is kept per site (r n r R + r r R numbers) is less
 // than the scratch of that recomputation (five such blocks a site), so `ckpt` no longer changes the layout.
 void rayleigh_grad_host(ttc_context* c, const ttc_tto* Hh, const ttc_ttv* x, int ckpt, double* value,
                         double* const* grads, bool f32) {
@@ -887,24 +880,36 @@ void rayleigh_grad_host(ttc_context* c, const ttc_tto* Hh, const ttc_ttv* x, int
     q.alpha = 1.0; q.beta = 0.0;
     g3.push_back(q);
   };
-  // right env step k+1 -> k, R_k[f0, e0, d0] = sum x[d0,i,d] H[e0,i,j,e] x[f0,j,f] R[f,e,d], stored (ket, H,
-  // bra); the product before the last, T2[f0, e0, i, d], and xRn[f0, j, d] = sum_f x[f0,j,f] Rn[d,f] are
-  // kept for the gradient.  Site 0 has no environment to its left to hand on.
+  // right env step k+1 -> k, R_k[f0, e0, d0] = sum x[d0,i,d] H[e0,i,j,e] x[f0,j,f] R[f,e,d], stored (H, ket,
+  // bra); the product before the last, HxR[f0, e0, i, d], stored (H, ket, i, bra), and xRn[f0, j, d] =
+  // sum_f x[f0,j,f] Rn[d,f] are kept for the gradient.  With the H index first every operand of every
+  // product is read along a unit stride.  Site 0 has no environment to its left to hand on.
   auto right_step = [&](Builder& B, int k, const double* Rh, const double* Rn, double* Rh_new, double* Rn_new, Descs& g1,
                         Descs& g2, Descs& g3) {
-    const int r0 = rk(k), r1 = rk(k + 1), R1 = Rk(k + 1), n = (int)X->dims[k];
+    const int r0 = rk(k), r1 = rk(k + 1), R0 = Rk(k), R1 = Rk(k + 1), n = (int)X->dims[k];
     const int xc = X->capr(0, k);
-    OpEnvStep st{};
-    st.A = xcore(k); st.r = r0; st.xc = xc; st.r1 = r1;
-    st.H = hcore(k); st.R = Rk(k); st.R1 = R1; st.n = n;
-    st.g = r1; st.cdim = r0;
-    st.S = xcore(k); st.s_k = xc; st.s_c = 1;
-    st.V = Rh; st.W = Rh_new; st.batch = 1; st.v_b = st.s_b = st.w_b = 0;
-    op_env_descs(st, B.wd((size_t)r0 * n * R1 * r1), HxR[k], g1, g2, k > 0 ? &g3 : nullptr);
+    // U[(c, j), (e, d)] = sum_f x[c,j,f] R[f,e,d]
+    double* U = B.wd((size_t)r0 * n * R1 * r1);
+    GemmDesc u = gd(r0 * n, R1 * r1, r1, xcore(k), 1, (long long)xc * n, Rh, R1, 1, U, 1, (long long)r0 * n);
+    u.m0 = r0; u.a_i0 = 1; u.a_i1 = xc; u.c_i0 = 1; u.c_i1 = r0;
+    u.n0 = R1; u.b_j0 = 1; u.b_j1 = (long long)R1 * r1;
+    u.c_j0 = (long long)r0 * n; u.c_j1 = (long long)r0 * n * R1;
+    g1.push_back(u);
+    // HxR[(b, c), (i, d)] = sum_{(j, e)} U[c,j,e,d] H[b,i,j,e]
+    GemmDesc w{};
+    w.m = r0 * r1; w.n = R0 * n; w.k = n * R1; w.batch = 1;
+    w.m0 = r0; w.n0 = R0; w.k0e = n;
+    w.A = U; w.a_i0 = 1; w.a_i1 = (long long)r0 * n * R1; w.a_k0 = r0; w.a_k1 = (long long)r0 * n;
+    w.B = hcore(k); w.b_k0 = (long long)R0 * n; w.b_k1 = (long long)R0 * n * n; w.b_j0 = 1; w.b_j1 = R0;
+    w.C = HxR[k]; w.c_i0 = R0; w.c_i1 = (long long)R0 * r0 * n; w.c_j0 = 1; w.c_j1 = (long long)R0 * r0;
+    w.alpha = 1.0; w.beta = 0.0;
+    g2.push_back(w);
     GemmDesc t = gd(r0 * n, r1, r1, xcore(k), 1, (long long)xc * n, Rn, r1, 1, xRn[k], 1, (long long)r0 * n);
     t.m0 = r0; t.a_i0 = 1; t.a_i1 = xc; t.c_i0 = 1; t.c_i1 = r0;
     g1.push_back(t);
     if (k == 0) return;
+    // R_k[(b, c), a] = sum_{(i, d)} HxR[(b, c), (i, d)] x[a, i, d]
+    g3.push_back(gd(R0 * r0, r0, n * r1, HxR[k], 1, (long long)R0 * r0, xcore(k), xc, 1, Rh_new, 1, (long long)R0 * r0));
     double* Tn = B.wd((size_t)r0 * n * r1);
     GemmDesc a1 = gd(r0 * n, r1, r1, xcore(k), 1, (long long)xc * n, Rn, 1, r1, Tn, 1, (long long)r0 * n);
     a1.m0 = r0; a1.a_i0 = 1; a1.a_i1 = xc; a1.c_i0 = 1; a1.c_i1 = r0;
@@ -954,10 +959,8 @@ void rayleigh_grad_host(ttc_context* c, const ttc_tto* Hh, const ttc_ttv* x, int
     Descs gh, gn;
     for (int k = 0; k < N; ++k) {
       const int r0 = rk(k), R0 = Rk(k), nr = (int)X->dims[k] * rk(k + 1);
-      // G[a, (i, d)] = (2/nn) sum_{(b, c)} L[a, b, c] HxR[c, b, (i, d)], b first
-      GemmDesc g = gd(r0, nr, R0 * r0, Lh[k], 1, r0, HxR[k], 1, (long long)R0 * r0, gcore(k), 1, r0, 2.0 / nn);
-      g.k0e = R0; g.a_k0 = r0; g.a_k1 = (long long)r0 * R0; g.b_k0 = r0; g.b_k1 = 1;
-      gh.push_back(g);
+      // G[a, (i, d)] = (2/nn) sum_{(b, c)} L[a, b, c] HxR[(b, c), (i, d)]
+      gh.push_back(gd(r0, nr, R0 * r0, Lh[k], 1, r0, HxR[k], 1, (long long)R0 * r0, gcore(k), 1, r0, 2.0 / nn));
       // G -= (2R/nn) Ln[a,c] xRn[c,(i,d)]
       gn.push_back(gd(r0, nr, r0, Ln[k], 1, r0, xRn[k], 1, r0, gcore(k), 1, r0, -2.0 * Rq / nn, 1.0));
     }

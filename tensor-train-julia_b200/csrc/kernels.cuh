@@ -18,7 +18,10 @@ constexpr int kGemmRefTile = 0;
 int gemm_pick_ksplit(const GemmDesc& d, long long launch_tiles, int nsm);
 long long gemm_split_ws_doubles(const GemmDesc& d, int tile);
 // ---- the same problems with float data in A, B and C, FP32 accumulation (gemm_f32.cu)
-void launch_gemm_f32(const GemmDesc* d_descs, int nd, long long total_tiles, cudaStream_t s);
+constexpr int kGemm32Tiles = 3;
+void launch_gemm_f32(const GemmDesc* d_descs, int nd, long long total_tiles, int tile, cudaStream_t s);
+int gemm32_pick_tile(const GemmDesc* d, int nd, int nsm);
+long long gemm32_tiles(const GemmDesc& d, int tile);
 
 // Device-side size bound: min(cap, mult * *p) when p is given (a rank that an earlier kernel of
 // the same plan wrote), else cap.  Rows or columns beyond the bound are exactly zero in the

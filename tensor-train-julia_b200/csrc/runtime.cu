@@ -158,7 +158,7 @@ static void launch_op(ttc_context* c, const Plan& p, const Op& op) {
       case OP_ZERO: launch_zero((const ZeroDesc*)d, op.count, op.total, s); break;
       case OP_SUMSQ: launch_sumsq((const NormDesc*)d, op.count, s); break;
       case OP_APPLY: launch_apply((const ApplyDesc*)d, op.count, op.a, op.b, s); break;
-      case OP_GEMM32: launch_gemm_f32((const GemmDesc*)d, op.count, op.total, s); break;
+      case OP_GEMM32: launch_gemm_f32((const GemmDesc*)d, op.count, op.total, op.a, s); break;
       case OP_CVT32: launch_cvt_f32((const CvtDesc*)d, op.count, op.total, s); break;
       case OP_WIDEN: launch_widen((const CvtDesc*)d, op.count, op.total, s); break;
       case OP_PHILOX: launch_philox((const PhiloxDesc*)d, op.count, op.total, s); break;
@@ -448,20 +448,22 @@ void Builder::gemm(std::vector<GemmDesc> v) {
 }
 void Builder::gemm32(std::vector<GemmDesc> v) {
   std::vector<GemmDesc> w;
-  long long t = 0;
   for (auto& d : v) {
-    const long long n = gemm_tiles(d, kGemmRefTile);
-    if (n == 0) continue;
+    if (gemm32_tiles(d, 0) == 0) continue;
     if (d.m0 <= 0) d.m0 = std::max(d.m, 1);
     if (d.n0 <= 0) d.n0 = std::max(d.n, 1);
     if (d.k0e <= 0) d.k0e = std::max(d.k, 1);
     if (wsbase) check_gemm(d, 4);
-    d.tile_start = t;
-    t += n;
     w.push_back(d);
   }
   if (w.empty()) return;
-  Op op; op.kind = OP_GEMM32; op.off = plan->push(w); op.count = (int)w.size(); op.total = t;
+  const int tile = gemm32_pick_tile(w.data(), (int)w.size(), current_sm_count());
+  long long t = 0;
+  for (auto& d : w) {
+    d.tile_start = t;
+    t += gemm32_tiles(d, tile);
+  }
+  Op op; op.kind = OP_GEMM32; op.off = plan->push(w); op.count = (int)w.size(); op.total = t; op.a = tile;
   for (auto& d : w) op.flops += 2.0 * d.m * d.n * d.k * std::max(1, d.batch);
   plan->ops.push_back(op);
 }

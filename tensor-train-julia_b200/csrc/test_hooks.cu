@@ -169,6 +169,28 @@ int ttc_test_gemm(ttc_context* c, int m, int n, int k, int batch, int m0, int n0
                             1, nullptr);
 }
 
+// ttc_test_gemm with float A, B and C.
+int ttc_test_gemm32(ttc_context* c, int m, int n, int k, int batch, int m0, int n0, int k0e, const float* A,
+                    long long a_len, const long long* as, const float* Bh, long long b_len, const long long* bs,
+                    float* Ch, long long c_len, const long long* cs, double alpha, double beta) {
+  return hook(c, [&] {
+    DevBuf dA(a_len * 4), dB(b_len * 4), dC(c_len * 4);
+    TTC_CUDA(cudaMemcpy(dA.p, A, a_len * 4, cudaMemcpyHostToDevice));
+    TTC_CUDA(cudaMemcpy(dB.p, Bh, b_len * 4, cudaMemcpyHostToDevice));
+    TTC_CUDA(cudaMemcpy(dC.p, Ch, c_len * 4, cudaMemcpyHostToDevice));
+    run_plan_once(c, [&](Builder& B) {
+      GemmDesc d{};
+      d.m = m; d.n = n; d.k = k; d.batch = batch; d.m0 = m0; d.n0 = n0; d.k0e = k0e;
+      d.A = dA.as<double>(); d.a_i0 = as[0]; d.a_i1 = as[1]; d.a_k0 = as[2]; d.a_k1 = as[3]; d.a_b = as[4];
+      d.B = dB.as<double>(); d.b_k0 = bs[0]; d.b_k1 = bs[1]; d.b_j0 = bs[2]; d.b_j1 = bs[3]; d.b_b = bs[4];
+      d.C = dC.as<double>(); d.c_i0 = cs[0]; d.c_i1 = cs[1]; d.c_j0 = cs[2]; d.c_j1 = cs[3]; d.c_b = cs[4];
+      d.alpha = alpha; d.beta = beta;
+      B.gemm32({d});
+    });
+    TTC_CUDA(cudaMemcpy(Ch, dC.p, c_len * 4, cudaMemcpyDeviceToHost));
+  });
+}
+
 // Householder QR of A (m x n, col-major): Q (m x K), R (K x n).
 int ttc_test_qr(ttc_context* c, int m, int n, const double* A, double* Q, double* R) {
   return hook(c, [&] {
