@@ -191,18 +191,25 @@ int ttc_test_gemm32(ttc_context* c, int m, int n, int k, int batch, int m0, int 
   });
 }
 
-// Householder QR of A (m x n, col-major): Q (m x K), R (K x n).
-int ttc_test_qr(ttc_context* c, int m, int n, const double* A, double* Q, double* R) {
+// Householder QR of A (m x n, col-major): Q (m x K), R (K x n); total: by the kernel that adds every sum over
+// all rows in one order.
+static int test_qr(ttc_context* c, int m, int n, const double* A, double* Q, double* R, bool total) {
   return hook(c, [&] {
     const int K = std::min(m, n);
     DevBuf dA((size_t)m * n * 8), dQ((size_t)m * K * 8), dR((size_t)K * n * 8), dT((size_t)((K + 15) / 16 + 1) * 256 * 8);
     TTC_CUDA(cudaMemcpy(dA.p, A, (size_t)m * n * 8, cudaMemcpyHostToDevice));
     run_plan_once(c, [&](Builder& B) {
-      B.qr({{m, n, dA.as<double>(), m, dQ.as<double>(), m, dR.as<double>(), K, dT.as<double>()}});
+      B.qr({{m, n, dA.as<double>(), m, dQ.as<double>(), m, dR.as<double>(), K, dT.as<double>()}}, total);
     });
     TTC_CUDA(cudaMemcpy(Q, dQ.p, (size_t)m * K * 8, cudaMemcpyDeviceToHost));
     TTC_CUDA(cudaMemcpy(R, dR.p, (size_t)K * n * 8, cudaMemcpyDeviceToHost));
   });
+}
+int ttc_test_qr(ttc_context* c, int m, int n, const double* A, double* Q, double* R) {
+  return test_qr(c, m, n, A, Q, R, false);
+}
+int ttc_test_qr_seq(ttc_context* c, int m, int n, const double* A, double* Q, double* R) {
+  return test_qr(c, m, n, A, Q, R, true);
 }
 
 // One-sided Jacobi of X (m x n): X <- X W (orthogonal columns), sigma, perm; W if accw.
