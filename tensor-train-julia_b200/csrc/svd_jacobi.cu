@@ -1011,27 +1011,43 @@ __global__ void __launch_bounds__(NT, 2)
   }
 }
 
-// Small problems (m, n <= 32, no W): one warp per problem, lane j holding column j in
-// registers.  A round of the circle method pairs the columns; the two lanes of a pair exchange
-// their columns by shuffles and both compute alpha, beta, gamma with the same operations in the
-// same order (so both find the same rotation bit for bit), each updating its own column.  No
-// barrier is needed, which is what bounds the cluster kernel on these sizes.  Same rotation, zero
-// threshold and convergence rule (a sweep without rotations) as the cluster kernel.
+// Small problems (m, n <= 32, no W): one warp per problem, L = 32 / PAIRS lanes per pair of columns, lane h of a
+// pair with the rows h, h + L, ... of both (RPL of them).  Pair p holds the columns at positions p and
+// ne - 1 - p of the circle method; between rounds the positions 1 .. ne - 1 move on by one, a shuffle from the
+// pair above or below.  A round is then a chain of RPL products, log2 L exchanges, the rotation and the move.
+// Same rotation, zero threshold and convergence rule as the cluster kernel.
+// What bounds it is that chain, 600 to 800 cycles: one warp runs alone on its scheduler.  One problem of
+// 8, 16, 20, 32 columns: 20, 37, 81, 149 us, where a column per lane, exchanged whole in every round with its 32
+// products in a row, took 65, 145, 206, 393; 600 problems of 32 columns 221 (499).  The block kernel, a CTA
+// per problem: 174 for one of 32 columns, 574 for 600.
+template <int PAIRS, int RPL>
 __global__ void __launch_bounds__(128) jacobi_small_kernel(const JacobiDesc* __restrict__ descs, int count, int* flags,
                                                           int max_sweeps) {
-  const int lane = threadIdx.x & 31;
+  constexpr int L = 32 / PAIRS;
+  const int lane = threadIdx.x & 31, p = lane / L, h = lane % L;
   const int prob = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (prob >= count) return;                        // uniform within the warp
   const JacobiDesc D = descs[prob];
   if (D.m <= 0 || D.n <= 0) return;
   const int m = max(1, dev_bound(D.m, D.m_dev, D.m_mult)), n = D.n;
-  double x[32];
+  const int ne = n + (n & 1), cx = p, cy = ne - 1 - p;   // the pair's columns before and after every sweep
+  const bool live = p < ne / 2, last = p == ne / 2 - 1;
+  double x[RPL], y[RPL];
+  double nx = 0.0, ny = 0.0;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) x[i] = (lane < n && i < m) ? D.X[(long long)lane * D.ldx + i] : 0.0;
-  double nrm = 0.0;
+  for (int i = 0; i < RPL; ++i) {
+    const int r = L * i + h;
+    x[i] = (live && r < m) ? D.X[(long long)cx * D.ldx + r] : 0.0;
+    y[i] = (live && r < m && cy < n) ? D.X[(long long)cy * D.ldx + r] : 0.0;
+    nx = fma(x[i], x[i], nx);
+    ny = fma(y[i], y[i], ny);
+  }
+  auto pair_sum = [](double v) {
 #pragma unroll
-  for (int i = 0; i < 32; ++i) nrm = fma(x[i], x[i], nrm);
-  const double fro2 = warp_sum(nrm);
+    for (int o = 1; o < L; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  };
+  const double fro2 = warp_sum(nx + ny);
   RotCfg q;
   {
     const double tol = jac_tol(D.m);
@@ -1041,59 +1057,66 @@ __global__ void __launch_bounds__(128) jacobi_small_kernel(const JacobiDesc* __r
     q.tol2 = tol * tol;
     q.zthr = q.tol2 * fro2 * q.sc;
   }
-  const int ne = n + (n & 1);
   bool converged = false;
   int sweep = 0;
   for (; sweep < max_sweeps && !converged; ++sweep) {
     bool any = false;
+#pragma unroll 1
     for (int rd = 0; rd < ne - 1; ++rd) {
-      // this lane's position in the round, and its partner column
-      int pos = 0;
-      if (lane != 0) pos = ((lane - 1 - rd) % (ne - 1) + (ne - 1)) % (ne - 1) + 1;
-      const int partner = rr_player(ne - 1 - pos, rd, ne);
-      const bool act = lane < n && partner < n;
-      const int src = act ? partner : lane;
-      const bool low = lane < partner;
-      double a = 0.0, b = 0.0, g = 0.0;            // alpha (low column), beta (high), gamma
-      double y[32];
+      double a = x[0] * x[0], b = y[0] * y[0], g = x[0] * y[0];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        y[i] = __shfl_sync(0xffffffffu, x[i], src);
-        const double lo = low ? x[i] : y[i], hi = low ? y[i] : x[i];
-        a = fma(lo, lo, a);
-        b = fma(hi, hi, b);
-        g = fma(lo, hi, g);
+      for (int i = 1; i < RPL; ++i) {
+        a = fma(x[i], x[i], a);
+        b = fma(y[i], y[i], b);
+        g = fma(x[i], y[i], g);
       }
-      const Rot R = act ? make_rot(a, b, g, q) : Rot{1.0, 0.0, false};
-      if (R.apply) {
-        any = true;
+      a = pair_sum(a); b = pair_sum(b); g = pair_sum(g);
+      const Rot R = make_rot_nb(a * q.sc, b * q.sc, g * q.sc, q);
+      any |= R.apply;
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
-          x[i] = low ? (R.c * x[i] - R.s * y[i]) : fma(R.s, y[i], R.c * x[i]);
+      for (int i = 0; i < RPL; ++i) {
+        const double u = R.c * x[i] - R.s * y[i], v = fma(R.s, x[i], R.c * y[i]);
+        const double up = __shfl_down_sync(0xffffffffu, u, L), dn = __shfl_up_sync(0xffffffffu, v, L);
+        x[i] = p == 0 ? u : last ? v : up;
+        y[i] = p == 0 ? (last ? v : up) : dn;
       }
     }
     converged = !__any_sync(0xffffffffu, any);
   }
   if (!converged && lane == 0) atomicOr(flags, DFLAG_JACOBI_NOCONV);
   if (D.info && lane == 0) *D.info = converged ? sweep : -sweep;
-  double c2 = 0.0;
+  nx = ny = 0.0;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) c2 = fma(x[i], x[i], c2);
-  const double sg = sqrt(c2);
-  if (lane < n) {
+  for (int i = 0; i < RPL; ++i) {
+    nx = fma(x[i], x[i], nx);
+    ny = fma(y[i], y[i], ny);
+  }
+  nx = sqrt(pair_sum(nx));
+  ny = sqrt(pair_sum(ny));
 #pragma unroll
-    for (int i = 0; i < 32; ++i)
-      if (i < m) D.X[(long long)lane * D.ldx + i] = x[i];
-    D.sigma[lane] = sg;
+  for (int i = 0; i < RPL; ++i) {
+    const int r = L * i + h;
+    if (live && r < m) {
+      D.X[(long long)cx * D.ldx + r] = x[i];
+      if (cy < n) D.X[(long long)cy * D.ldx + r] = y[i];
+    }
   }
   // ranking by decreasing value (NaN last, ties by index), as in the cluster kernel
-  const double key = (lane < n) ? ((sg == sg) ? sg : -1.0) : -2.0;
-  int rank = 0;
+  const double kx = nx == nx ? nx : -1.0, ky = ny == ny ? ny : -1.0;
+  int rx = 0, ry = 0;
   for (int j = 0; j < n; ++j) {
-    const double w = __shfl_sync(0xffffffffu, key, j);
-    rank += (w > key) || (w == key && j < lane);
+    const double w = j < ne / 2 ? __shfl_sync(0xffffffffu, kx, L * j) : __shfl_sync(0xffffffffu, ky, L * (ne - 1 - j));
+    rx += (w > kx) || (w == kx && j < cx);
+    ry += (w > ky) || (w == ky && j < cy);
   }
-  if (lane < n) D.perm[rank] = lane;
+  if (live && h == 0) {
+    D.sigma[cx] = nx;
+    D.perm[rx] = cx;
+    if (cy < n) {
+      D.sigma[cy] = ny;
+      D.perm[ry] = cy;
+    }
+  }
 }
 
 // Problem order of a launch: by decreasing size m x n^2, m the rows left by the device bound and
@@ -1245,7 +1268,9 @@ void launch_jacobi(const JacobiDesc* d_descs, int count, int max_m, int max_n, b
   TTC_REQUIRE(smem <= 200 * 1024, TTC_EDIM, "jacobi: matrix too large for the shared-memory blocks");
   if (count > kJacobiOrderMax) order = nullptr;
   if (!accw && max_m <= 32 && max_n <= 32) {       // every problem fits one warp's registers
-    jacobi_small_kernel<<<(unsigned)((count + 3) / 4), 128, 0, s>>>(d_descs, count, d_flags, max_sweeps);
+    const unsigned grid = (unsigned)((count + 3) / 4);
+    if (max_m <= 16 && max_n <= 16) jacobi_small_kernel<8, 4><<<grid, 128, 0, s>>>(d_descs, count, d_flags, max_sweeps);
+    else jacobi_small_kernel<16, 16><<<grid, 128, 0, s>>>(d_descs, count, d_flags, max_sweeps);
     TTC_CHECK_LAUNCH();
     return;
   }
