@@ -56,8 +56,7 @@ __global__ void final_kernel(const FinalDesc* descs) {
 }
 void launch_final(const FinalDesc* d, int count, long long max_n, cudaStream_t s) {
   if (count <= 0) return;
-  const long long blocks = std::max<long long>(1, std::min<long long>((max_n + 255) / 256, 148LL * 4));
-  final_kernel<<<dim3((unsigned)blocks, (unsigned)count), 256, 0, s>>>(d);
+  final_kernel<<<dim3(elem_blocks(max_n, 256, count), (unsigned)count), 256, 0, s>>>(d);
   TTC_CHECK_LAUNCH();
 }
 
@@ -71,55 +70,81 @@ void launch_setrank(const SetRankDesc* d, int count, cudaStream_t s) {
   TTC_CHECK_LAUNCH();
 }
 
+// f(source offset, destination offset) for every element of a conversion, with 32-bit divisions where the
+// element count allows it.
+template <class F>
+__device__ __forceinline__ void each_elem(const CvtDesc& D, F&& f) {
+  const long long total = D.rows * D.cols;
+  if (total < (1LL << 31)) {
+    const unsigned rows = (unsigned)D.rows, step = gridDim.x * blockDim.x;
+    for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < (unsigned)total; e += step) {
+      const unsigned j = e / rows, i = e - j * rows;
+      f(i * D.ss_i + j * D.ss_j, i * D.ds_i + j * D.ds_j);
+    }
+    return;
+  }
+  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
+    const long long j = e / D.rows, i = e - j * D.rows;
+    f(i * D.ss_i + j * D.ss_j, i * D.ds_i + j * D.ds_j);
+  }
+}
+
 __global__ void cvt_f32_kernel(const CvtDesc* descs) {
   const CvtDesc D = descs[blockIdx.y];
-  const long long total = D.rows * D.cols;
   float* dst = reinterpret_cast<float*>(D.dst);
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    const long long i = e % D.rows, j = e / D.rows;
-    dst[i * D.ds_i + j * D.ds_j] = (float)(D.alpha * D.src[i * D.ss_i + j * D.ss_j]);
-  }
+  each_elem(D, [&](long long from, long long to) { dst[to] = (float)(D.alpha * D.src[from]); });
 }
 void launch_cvt_f32(const CvtDesc* d, int count, long long max_elems, cudaStream_t s) {
   if (count <= 0 || max_elems <= 0) return;
-  const long long blocks = std::min<long long>((max_elems + 255) / 256, 148LL * 8);
-  cvt_f32_kernel<<<dim3((unsigned)blocks, (unsigned)count), 256, 0, s>>>(d);
+  cvt_f32_kernel<<<dim3(elem_blocks(max_elems, 256, count), (unsigned)count), 256, 0, s>>>(d);
   TTC_CHECK_LAUNCH();
 }
 __global__ void widen_kernel(const CvtDesc* descs) {
   const CvtDesc D = descs[blockIdx.y];
-  const long long total = D.rows * D.cols;
   const float* src = reinterpret_cast<const float*>(D.src);
   double* dst = reinterpret_cast<double*>(D.dst);
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    const long long i = e % D.rows, j = e / D.rows;
-    dst[i * D.ds_i + j * D.ds_j] = D.alpha * (double)src[i * D.ss_i + j * D.ss_j];
-  }
+  each_elem(D, [&](long long from, long long to) { dst[to] = D.alpha * (double)src[from]; });
 }
 void launch_widen(const CvtDesc* d, int count, long long max_elems, cudaStream_t s) {
   if (count <= 0 || max_elems <= 0) return;
-  const long long blocks = std::min<long long>((max_elems + 255) / 256, 148LL * 8);
-  widen_kernel<<<dim3((unsigned)blocks, (unsigned)count), 256, 0, s>>>(d);
+  widen_kernel<<<dim3(elem_blocks(max_elems, 256, count), (unsigned)count), 256, 0, s>>>(d);
   TTC_CHECK_LAUNCH();
 }
 
+// A conversion that reads along one index and writes along the other (most operands of the sketches' GEMMs
+// are transposed) goes through 32 x 32 shared-memory tiles, so that both sides are coalesced.
 template <typename T>
-__global__ void cvt_bf16_kernel(const CvtDesc* descs) {
+__global__ void __launch_bounds__(256) cvt_bf16_kernel(const CvtDesc* descs) {
+  __shared__ T tile[32][34];
   const CvtDesc D = descs[blockIdx.y];
-  const long long total = D.rows * D.cols;
   T* dst = reinterpret_cast<T*>(D.dst);
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    const long long i = e % D.rows, j = e / D.rows;
-    const double v = D.alpha * D.src[i * D.ss_i + j * D.ss_j];
-    if constexpr (sizeof(T) == 4) dst[i * D.ds_i + j * D.ds_j] = round_tf32((float)v);   // TF32 operand
-    else dst[i * D.ds_i + j * D.ds_j] = __double2bfloat16(v);
+  auto cvt = [&](double x) -> T {
+    const double v = D.alpha * x;
+    if constexpr (sizeof(T) == 4) return round_tf32((float)v);      // TF32 operand
+    else return __double2bfloat16(v);
+  };
+  if (D.ss_i == 1 && D.ds_j == 1 && D.ds_i != 1 && D.rows >= 16 && D.cols >= 16) {
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;         // 32 x 8 threads
+    const long long ti = (D.rows + 31) / 32, tiles = ti * ((D.cols + 31) / 32);
+    for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
+      const long long i0 = t % ti * 32, j0 = t / ti * 32;
+#pragma unroll
+      for (int k = ty; k < 32; k += 8)
+        if (i0 + tx < D.rows && j0 + k < D.cols) tile[k][tx] = cvt(D.src[i0 + tx + (j0 + k) * D.ss_j]);
+      __syncthreads();
+#pragma unroll
+      for (int k = ty; k < 32; k += 8)
+        if (i0 + k < D.rows && j0 + tx < D.cols) dst[(i0 + k) * D.ds_i + j0 + tx] = tile[tx][k];
+      __syncthreads();
+    }
+    return;
   }
+  each_elem(D, [&](long long from, long long to) { dst[to] = cvt(D.src[from]); });
 }
 void launch_cvt_bf16(const CvtDesc* d, int count, long long max_elems, cudaStream_t s, bool f32) {
   if (count <= 0 || max_elems <= 0) return;
-  const long long blocks = std::min<long long>((max_elems + 255) / 256, 148LL * 8);
-  if (f32) cvt_bf16_kernel<float><<<dim3((unsigned)blocks, (unsigned)count), 256, 0, s>>>(d);
-  else cvt_bf16_kernel<__nv_bfloat16><<<dim3((unsigned)blocks, (unsigned)count), 256, 0, s>>>(d);
+  if (f32) cvt_bf16_kernel<float><<<dim3(elem_blocks(max_elems, 1024, count), (unsigned)count), 256, 0, s>>>(d);
+  else cvt_bf16_kernel<__nv_bfloat16><<<dim3(elem_blocks(max_elems, 1024, count), (unsigned)count), 256, 0, s>>>(d);
   TTC_CHECK_LAUNCH();
 }
 

@@ -191,6 +191,29 @@ int ttc_test_gemm32(ttc_context* c, int m, int n, int k, int batch, int m0, int 
   });
 }
 
+// dst[i ds_i + j ds_j] = src[i ss_i + j ss_j] as BF16 (dst: 16-bit words), or TF32 (dst: floats), `count` times side by
+// side; other entries of dst stay.
+int ttc_test_cvt(ttc_context* c, int rows, int cols, long long ss_i, long long ss_j, long long ds_i, long long ds_j, int count,
+                 int tf32, const double* src, long long src_len, void* dst, long long dst_bytes) {
+  return hook(c, [&] {
+    DevBuf s(src_len * 8 * count), d(dst_bytes * count);
+    for (int t = 0; t < count; ++t)
+      TTC_CUDA(cudaMemcpy(s.as<double>() + t * src_len, src, src_len * 8, cudaMemcpyHostToDevice));
+    TTC_CUDA(cudaMemcpy(d.p, dst, dst_bytes * count, cudaMemcpyHostToDevice));
+    run_plan_once(c, [&](Builder& B) {
+      std::vector<CvtDesc> v;
+      for (int t = 0; t < count; ++t) {
+        CvtDesc e{};
+        e.src = s.as<double>() + t * src_len; e.dst = d.as<char>() + t * dst_bytes;
+        e.rows = rows; e.cols = cols; e.ss_i = ss_i; e.ss_j = ss_j; e.ds_i = ds_i; e.ds_j = ds_j; e.alpha = 1.0;
+        v.push_back(e);
+      }
+      B.cvt_bf16(v, tf32 != 0);
+    });
+    TTC_CUDA(cudaMemcpy(dst, d.p, dst_bytes * count, cudaMemcpyDeviceToHost));
+  });
+}
+
 // Householder QR of A (m x n, col-major): Q (m x K), R (K x n); total: by the kernel that adds every sum over
 // all rows in one order.
 static int test_qr(ttc_context* c, int m, int n, const double* A, double* Q, double* R, bool total) {

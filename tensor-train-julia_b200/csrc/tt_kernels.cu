@@ -77,22 +77,24 @@ __global__ void __launch_bounds__(NT) copy4_kernel(const CopyDesc* __restrict__ 
 void launch_copy(const CopyDesc* d, int count, long long max_elems, cudaStream_t s) {
   if (count <= 0 || max_elems <= 0) return;
   // about four elements per thread; with `count` copies in the grid's y dimension
-  const long long blocks = std::min<long long>((max_elems + 4 * NT - 1) / (4 * NT), 148LL * 8);
-  dim3 grid((unsigned)blocks, (unsigned)count);
+  dim3 grid(elem_blocks(max_elems, 4 * NT, count), (unsigned)count);
   copy4_kernel<<<grid, NT, 0, s>>>(d);
   TTC_CHECK_LAUNCH();
 }
 
 __global__ void zero_kernel(const ZeroDesc* __restrict__ descs) {
   const ZeroDesc D = descs[blockIdx.y];
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < D.n; e += (long long)gridDim.x * blockDim.x)
-    D.p[e] = 0.0;
+  const long long step = (long long)gridDim.x * NT;
+  for (long long e = (long long)blockIdx.x * NT + threadIdx.x; e < D.n; e += 4 * step) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (e + u * step < D.n) D.p[e + u * step] = 0.0;
+  }
 }
 
 void launch_zero(const ZeroDesc* d, int count, long long max_n, cudaStream_t s) {
   if (count <= 0 || max_n <= 0) return;
-  const long long blocks = std::min<long long>((max_n + NT - 1) / NT, 148LL * 8);
-  zero_kernel<<<dim3((unsigned)blocks, (unsigned)count), NT, 0, s>>>(d);
+  zero_kernel<<<dim3(elem_blocks(max_n, 4 * NT, count), (unsigned)count), NT, 0, s>>>(d);
   TTC_CHECK_LAUNCH();
 }
 
@@ -181,9 +183,9 @@ __global__ void select_kernel(const SelectDesc* __restrict__ descs) {
   const SelectDesc D = descs[blockIdx.y];
   const int k = *D.rank;
   const int rows = max(D.rows, D.zrows);
-  const long long total = (long long)rows * D.cols;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(e / rows), r = (int)(e - (long long)c * rows);
+  const unsigned total = (unsigned)rows * (unsigned)D.cols;    // a factor of at most a few thousand squared
+  for (unsigned e = blockIdx.x * NT + threadIdx.x; e < total; e += gridDim.x * NT) {
+    const int c = (int)(e / (unsigned)rows), r = (int)(e - (unsigned)c * (unsigned)rows);
     double v = 0.0;
     if (c < k && r < D.rows) {
       const int src = D.perm[c];
@@ -198,8 +200,7 @@ __global__ void select_kernel(const SelectDesc* __restrict__ descs) {
 void launch_select(const SelectDesc* d, int count, int max_rows, int max_cols, cudaStream_t s) {
   if (count <= 0) return;
   const long long total = (long long)max_rows * max_cols;
-  const long long blocks = std::max<long long>(1, std::min<long long>((total + NT - 1) / NT, 148LL * 4));
-  select_kernel<<<dim3((unsigned)blocks, (unsigned)count), NT, 0, s>>>(d);
+  select_kernel<<<dim3(elem_blocks(total, NT, count), (unsigned)count), NT, 0, s>>>(d);
   TTC_CHECK_LAUNCH();
 }
 
