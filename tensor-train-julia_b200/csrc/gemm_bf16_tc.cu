@@ -132,6 +132,7 @@ __device__ __forceinline__ int find_desc(const Bf16GemmDesc* __restrict__ d, int
 
 template <bool TF32>
 __global__ void __launch_bounds__(NT, 1) gemm_bf16_tc_kernel(const Bf16GemmDesc* __restrict__ descs, int nd, int* flags) {
+  dep_wait();
   constexpr int EB = TF32 ? 4 : 2;         // operand element bytes
   constexpr int BK = 128 / EB;             // K elements per 128-byte tile row
   constexpr int CH = 16 / EB;              // K elements per 16-byte chunk
@@ -296,7 +297,7 @@ void launch_tc(const Bf16GemmDesc* d, int nd, long long total_tiles, cudaStream_
   attr_once.run(dev, [smem] {
     TTC_CUDA(cudaFuncSetAttribute(gemm_bf16_tc_kernel<TF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   });
-  gemm_bf16_tc_kernel<TF32><<<(unsigned)total_tiles, NT, smem, s>>>(d, nd, d_flags);
+  launch_dep(gemm_bf16_tc_kernel<TF32>, (unsigned)total_tiles, NT, smem, s, d, nd, d_flags);
   TTC_CHECK_LAUNCH();
 }
 }  // namespace

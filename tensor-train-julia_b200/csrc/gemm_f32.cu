@@ -49,6 +49,7 @@ constexpr size_t kSmem32 = sizeof(float) * (STAGES * kStageFloats<BM, BN> > BN *
 // 4 x 8 threads.
 template <int BM, int BN, int TM, int TN, int STAGES, int MINB>
 __global__ void __launch_bounds__(BM / TM * (BN / TN), MINB) gemm_f32_grouped_kernel(const GemmDesc* __restrict__ descs, int nd) {
+  dep_wait();
   constexpr int NT = BM / TM * (BN / TN), PA = BM + 4, PB = BN + 4;
   constexpr int LA = BM * BK / NT, LB = BN * BK / NT, KQ = NT / BK;
   constexpr int GM = BM / TM, GN = BN / TN;                  // threads along rows and columns
@@ -199,8 +200,8 @@ void launch_t(const GemmDesc* d_descs, int nd, long long total_tiles, cudaStream
     TTC_CUDA(cudaFuncSetAttribute(gemm_f32_grouped_kernel<BM, BN, TM, TN, STAGES, MINB>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem32<BM, BN, STAGES>));
   });
-  gemm_f32_grouped_kernel<BM, BN, TM, TN, STAGES, MINB>
-      <<<(unsigned)total_tiles, BM / TM * (BN / TN), kSmem32<BM, BN, STAGES>, s>>>(d_descs, nd);
+  launch_dep(gemm_f32_grouped_kernel<BM, BN, TM, TN, STAGES, MINB>, (unsigned)total_tiles, BM / TM * (BN / TN),
+             kSmem32<BM, BN, STAGES>, s, d_descs, nd);
   TTC_CHECK_LAUNCH();
 }
 }  // namespace

@@ -60,6 +60,7 @@ constexpr size_t kGemmSmem = sizeof(double) * STAGES * kStageDoubles<BM, BN>;
 // WM x WN warps, each a (BM / WM) x (BN / WN) part of the tile in 8 x 8 fragments.
 template <int BM, int BN, int WM, int WN, int STAGES, int MINB>
 __global__ void __launch_bounds__(WM * WN * 32, MINB) gemm_f64_grouped_kernel(const GemmDesc* __restrict__ descs, int nd) {
+  dep_wait();
   constexpr int NT = WM * WN * 32, PA = BM + 4, PB = BN + 4;
   constexpr int FM = BM / WM / 8, FN = BN / WN / 8;
   constexpr int LA = BM * BK / NT, LB = BN * BK / NT;      // elements of A and B a thread loads per stage
@@ -272,7 +273,8 @@ void launch_t(const GemmDesc* d_descs, int nd, long long total_tiles, cudaStream
     TTC_CUDA(cudaFuncSetAttribute(gemm_f64_grouped_kernel<BM, BN, WM, WN, STAGES, MINB>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem<BM, BN, STAGES>));
   });
-  gemm_f64_grouped_kernel<BM, BN, WM, WN, STAGES, MINB><<<(unsigned)total_tiles, WM * WN * 32, kGemmSmem<BM, BN, STAGES>, s>>>(d_descs, nd);
+  launch_dep(gemm_f64_grouped_kernel<BM, BN, WM, WN, STAGES, MINB>, (unsigned)total_tiles, WM * WN * 32,
+             kGemmSmem<BM, BN, STAGES>, s, d_descs, nd);
   TTC_CHECK_LAUNCH();
 }
 }  // namespace

@@ -539,6 +539,7 @@ __device__ __noinline__ bool factor_panel(double* A, int lda, int mp, int jb, in
 template <int NW>
 __global__ void __launch_bounds__(NW * 32, NW <= 8 ? 2 : 1)
     householder_qr_kernel(const QRDesc* __restrict__ descs, int csize, int* flags) {
+  dep_wait();
   extern __shared__ __align__(16) double sm[];
   cg::cluster_group cluster = cg::this_cluster();
   const int crank = (int)cluster.block_rank();
@@ -616,6 +617,7 @@ __global__ void __launch_bounds__(NW * 32, NW <= 8 ? 2 : 1)
 template <int NW>
 __global__ void __launch_bounds__(NW * 32, NW <= 8 ? 2 : 1)
     householder_apply_q_kernel(const QApplyDesc* __restrict__ descs, int csize) {
+  dep_wait();
   extern __shared__ __align__(16) double sm[];
   const int crank = (int)(blockIdx.x % csize);
   const QApplyDesc D = descs[blockIdx.x / csize];
@@ -665,7 +667,7 @@ void launch_qr_apply_t(const QApplyDesc* d_descs, int count, int max_m, cudaStre
   TTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, householder_apply_q_kernel<NW>, NW * 32, smem));
   const int csize = std::min(8, std::max(1, current_sm_count() * std::max(1, per_sm) / count));
   const size_t smem_l = count * csize <= current_sm_count() ? std::max(smem, kLoneCtaSmem) : smem;
-  householder_apply_q_kernel<NW><<<(unsigned)(count * csize), NW * 32, smem_l, s>>>(d_descs, csize);
+  launch_dep(householder_apply_q_kernel<NW>, (unsigned)(count * csize), NW * 32, smem_l, s, d_descs, csize);
   TTC_CHECK_LAUNCH();
 }
 
@@ -695,13 +697,15 @@ void launch_qr_t(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, in
   // one CTA per SM while there are SMs for all
   cfg.dynamicSmemBytes = count * csize <= current_sm_count() ? std::max(smem, kLoneCtaSmem) : smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = (unsigned)csize;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   TTC_CUDA(cudaLaunchKernelEx(&cfg, householder_qr_kernel<NW>, d_descs, csize, d_flags));
   TTC_CHECK_LAUNCH();
 }

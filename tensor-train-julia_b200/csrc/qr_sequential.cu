@@ -362,6 +362,7 @@ __device__ __noinline__ bool panel_steps_regs(int mp, int jb) {
 }  // namespace
 
 __global__ void __launch_bounds__(NT, 1) householder_qr_seq_kernel(const QRDesc* __restrict__ descs, int csize, int* flags) {
+  dep_wait();
   cg::cluster_group cluster = cg::this_cluster();
   const int crank = (int)cluster.block_rank();
   const QRDesc D = descs[blockIdx.x / csize];
@@ -568,13 +569,15 @@ void launch_qr_cfg(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, 
   cfg.blockDim = dim3(NT);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = (unsigned)csize;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   TTC_CUDA(cudaLaunchKernelEx(&cfg, householder_qr_seq_kernel, d_descs, csize, d_flags));
   TTC_CHECK_LAUNCH();
 }

@@ -12,17 +12,19 @@ namespace ttc {
 
 // ---------------------------------------------------------------- control kernels
 __global__ void zerochk_kernel(const ZeroChkDesc* d, int count) {
+  dep_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < count) *d[i].flag = (sqrt(*d[i].sumsq) < d[i].tol) ? 1 : 0;
 }
 void launch_zerochk(const ZeroChkDesc* d, int count, cudaStream_t s) {
   if (count <= 0) return;
-  zerochk_kernel<<<(count + 127) / 128, 128, 0, s>>>(d, count);
+  launch_dep(zerochk_kernel, (count + 127) / 128, 128, 0, s, d, count);
   TTC_CHECK_LAUNCH();
 }
 
 // One CTA per problem: the largest sigma (block reduction), then the column scaling.
 __global__ void pinv_scale_kernel(const PinvScaleDesc* descs) {
+  dep_wait();
   const PinvScaleDesc D = descs[blockIdx.x];
   __shared__ double s_max[32];
   double mx = 0.0;
@@ -42,11 +44,12 @@ __global__ void pinv_scale_kernel(const PinvScaleDesc* descs) {
 }
 void launch_pinv_scale(const PinvScaleDesc* d, int count, cudaStream_t s) {
   if (count <= 0) return;
-  pinv_scale_kernel<<<count, 256, 0, s>>>(d);
+  launch_dep(pinv_scale_kernel, count, 256, 0, s, d);
   TTC_CHECK_LAUNCH();
 }
 
 __global__ void final_kernel(const FinalDesc* descs) {
+  dep_wait();
   const FinalDesc D = descs[blockIdx.y];
   if (*D.flag == 0) return;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < D.n; e += (long long)gridDim.x * blockDim.x)
@@ -56,17 +59,18 @@ __global__ void final_kernel(const FinalDesc* descs) {
 }
 void launch_final(const FinalDesc* d, int count, long long max_n, cudaStream_t s) {
   if (count <= 0) return;
-  final_kernel<<<dim3(elem_blocks(max_n, 256, count), (unsigned)count), 256, 0, s>>>(d);
+  launch_dep(final_kernel, dim3(elem_blocks(max_n, 256, count), (unsigned)count), 256, 0, s, d);
   TTC_CHECK_LAUNCH();
 }
 
 __global__ void setrank_kernel(const SetRankDesc* d) {
+  dep_wait();
   const SetRankDesc D = d[blockIdx.x];
   for (int i = threadIdx.x; i < D.n; i += blockDim.x) D.dst[i] = D.src[i];
 }
 void launch_setrank(const SetRankDesc* d, int count, cudaStream_t s) {
   if (count <= 0) return;
-  setrank_kernel<<<count, 64, 0, s>>>(d);
+  launch_dep(setrank_kernel, count, 64, 0, s, d);
   TTC_CHECK_LAUNCH();
 }
 
@@ -90,16 +94,18 @@ __device__ __forceinline__ void each_elem(const CvtDesc& D, F&& f) {
 }
 
 __global__ void cvt_f32_kernel(const CvtDesc* descs) {
+  dep_wait();
   const CvtDesc D = descs[blockIdx.y];
   float* dst = reinterpret_cast<float*>(D.dst);
   each_elem(D, [&](long long from, long long to) { dst[to] = (float)(D.alpha * D.src[from]); });
 }
 void launch_cvt_f32(const CvtDesc* d, int count, long long max_elems, cudaStream_t s) {
   if (count <= 0 || max_elems <= 0) return;
-  cvt_f32_kernel<<<dim3(elem_blocks(max_elems, 256, count), (unsigned)count), 256, 0, s>>>(d);
+  launch_dep(cvt_f32_kernel, dim3(elem_blocks(max_elems, 256, count), (unsigned)count), 256, 0, s, d);
   TTC_CHECK_LAUNCH();
 }
 __global__ void widen_kernel(const CvtDesc* descs) {
+  dep_wait();
   const CvtDesc D = descs[blockIdx.y];
   const float* src = reinterpret_cast<const float*>(D.src);
   double* dst = reinterpret_cast<double*>(D.dst);
@@ -107,7 +113,7 @@ __global__ void widen_kernel(const CvtDesc* descs) {
 }
 void launch_widen(const CvtDesc* d, int count, long long max_elems, cudaStream_t s) {
   if (count <= 0 || max_elems <= 0) return;
-  widen_kernel<<<dim3(elem_blocks(max_elems, 256, count), (unsigned)count), 256, 0, s>>>(d);
+  launch_dep(widen_kernel, dim3(elem_blocks(max_elems, 256, count), (unsigned)count), 256, 0, s, d);
   TTC_CHECK_LAUNCH();
 }
 
@@ -115,6 +121,7 @@ void launch_widen(const CvtDesc* d, int count, long long max_elems, cudaStream_t
 // are transposed) goes through 32 x 32 shared-memory tiles, so that both sides are coalesced.
 template <typename T>
 __global__ void __launch_bounds__(256) cvt_bf16_kernel(const CvtDesc* descs) {
+  dep_wait();
   __shared__ T tile[32][34];
   const CvtDesc D = descs[blockIdx.y];
   T* dst = reinterpret_cast<T*>(D.dst);
@@ -143,8 +150,8 @@ __global__ void __launch_bounds__(256) cvt_bf16_kernel(const CvtDesc* descs) {
 }
 void launch_cvt_bf16(const CvtDesc* d, int count, long long max_elems, cudaStream_t s, bool f32) {
   if (count <= 0 || max_elems <= 0) return;
-  if (f32) cvt_bf16_kernel<float><<<dim3(elem_blocks(max_elems, 1024, count), (unsigned)count), 256, 0, s>>>(d);
-  else cvt_bf16_kernel<__nv_bfloat16><<<dim3(elem_blocks(max_elems, 1024, count), (unsigned)count), 256, 0, s>>>(d);
+  if (f32) launch_dep(cvt_bf16_kernel<float>, dim3(elem_blocks(max_elems, 1024, count), (unsigned)count), 256, 0, s, d);
+  else launch_dep(cvt_bf16_kernel<__nv_bfloat16>, dim3(elem_blocks(max_elems, 1024, count), (unsigned)count), 256, 0, s, d);
   TTC_CHECK_LAUNCH();
 }
 

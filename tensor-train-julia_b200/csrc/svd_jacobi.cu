@@ -349,6 +349,7 @@ template <int RMAX>
 __global__ void __launch_bounds__(NT, RMAX <= 8 ? 2 : 1)
     jacobi_svd_kernel(const JacobiDesc* __restrict__ descs, const int* __restrict__ order, int bw, int csize,
                       int* flags, int max_sweeps) {
+  dep_wait();
   extern __shared__ double sm[];
   __shared__ int s_any, s_nact;
   __shared__ double s_red[NW];
@@ -753,6 +754,7 @@ __device__ __forceinline__ bool inner_rounds(double* G, double* V, double2 (*CSP
 __global__ void __launch_bounds__(NT, 2)
     jacobi_block_kernel(const JacobiDesc* __restrict__ descs, const int* __restrict__ order, int csize, int* flags,
                         int max_sweeps) {
+  dep_wait();
   extern __shared__ __align__(16) double sm[];
   __shared__ int s_any, s_nact;
   __shared__ double s_red[NW];
@@ -1023,6 +1025,7 @@ __global__ void __launch_bounds__(NT, 2)
 template <int PAIRS, int RPL>
 __global__ void __launch_bounds__(128) jacobi_small_kernel(const JacobiDesc* __restrict__ descs, int count, int* flags,
                                                           int max_sweeps) {
+  dep_wait();
   constexpr int L = 32 / PAIRS;
   const int lane = threadIdx.x & 31, p = lane / L, h = lane % L;
   const int prob = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -1122,6 +1125,7 @@ __global__ void __launch_bounds__(128) jacobi_small_kernel(const JacobiDesc* __r
 // Problem order of a launch: by decreasing size m x n^2, m the rows left by the device bound and
 // n the columns (at most m when bounded: the bounded factor is square), ties by index.
 __global__ void jacobi_order_kernel(const JacobiDesc* __restrict__ descs, int count, int* __restrict__ order) {
+  dep_wait();
   for (int i = threadIdx.x; i < count; i += blockDim.x) {
     auto key = [&](int j) {
       const JacobiDesc& d = descs[j];
@@ -1185,7 +1189,7 @@ static void launch_jacobi_t(const JacobiDesc* d_descs, int count, int max_n, int
     TTC_CUDA(cudaFuncSetAttribute(jacobi_svd_kernel<RMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
   });
   if (order) {
-    jacobi_order_kernel<<<1, 512, 0, s>>>(d_descs, count, order);
+    launch_dep(jacobi_order_kernel, 1, 512, 0, s, d_descs, count, order);
     TTC_CHECK_LAUNCH();
   }
   const int csize = jacobi_cluster_size<RMAX>(count, max_n, bw, smem, order != nullptr);
@@ -1194,13 +1198,15 @@ static void launch_jacobi_t(const JacobiDesc* d_descs, int count, int max_n, int
   cfg.blockDim = dim3(NT);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = (unsigned)csize;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   TTC_CUDA(cudaLaunchKernelEx(&cfg, jacobi_svd_kernel<RMAX>, d_descs, (const int*)order, bw, csize, d_flags,
                               max_sweeps));
   TTC_CHECK_LAUNCH();
@@ -1236,7 +1242,7 @@ static void launch_jacobi_block(const JacobiDesc* d_descs, int count, int max_m,
   const size_t smem = sizeof(double) * block_dyn_doubles(smem_stride(max_m), max_n) + sizeof(int) * (size_t)max_n;
   TTC_REQUIRE(smem <= 200 * 1024, TTC_EDIM, "jacobi: matrix too large for the shared-memory blocks");
   if (order) {
-    jacobi_order_kernel<<<1, 512, 0, s>>>(d_descs, count, order);
+    launch_dep(jacobi_order_kernel, 1, 512, 0, s, d_descs, count, order);
     TTC_CHECK_LAUNCH();
   }
   const int csize = jacobi_block_csize(count, max_n, smem, order != nullptr);
@@ -1248,13 +1254,15 @@ static void launch_jacobi_block(const JacobiDesc* d_descs, int count, int max_m,
   // 1.37 ms, 1.30 apart)
   cfg.dynamicSmemBytes = (size_t)count * csize <= (size_t)current_sm_count() ? std::max(smem, kLoneCtaSmem) : smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = (unsigned)csize;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   TTC_CUDA(cudaLaunchKernelEx(&cfg, jacobi_block_kernel, d_descs, (const int*)order, csize, d_flags, max_sweeps));
   TTC_CHECK_LAUNCH();
 }
@@ -1269,8 +1277,8 @@ void launch_jacobi(const JacobiDesc* d_descs, int count, int max_m, int max_n, b
   if (count > kJacobiOrderMax) order = nullptr;
   if (!accw && max_m <= 32 && max_n <= 32) {       // every problem fits one warp's registers
     const unsigned grid = (unsigned)((count + 3) / 4);
-    if (max_m <= 16 && max_n <= 16) jacobi_small_kernel<8, 4><<<grid, 128, 0, s>>>(d_descs, count, d_flags, max_sweeps);
-    else jacobi_small_kernel<16, 16><<<grid, 128, 0, s>>>(d_descs, count, d_flags, max_sweeps);
+    if (max_m <= 16 && max_n <= 16) launch_dep(jacobi_small_kernel<8, 4>, grid, 128, 0, s, d_descs, count, d_flags, max_sweeps);
+    else launch_dep(jacobi_small_kernel<16, 16>, grid, 128, 0, s, d_descs, count, d_flags, max_sweeps);
     TTC_CHECK_LAUNCH();
     return;
   }

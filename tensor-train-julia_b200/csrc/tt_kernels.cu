@@ -21,6 +21,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 // coalesced; every other copy maps consecutive threads to consecutive dim-0 elements, with
 // 32-bit index arithmetic when the copy has fewer than 2^31 elements.
 __global__ void __launch_bounds__(NT) copy4_kernel(const CopyDesc* __restrict__ descs) {
+  dep_wait();
   __shared__ double tile[32][33];
   const CopyDesc D = descs[blockIdx.y];
   long long e0 = D.ext[0], e1 = D.ext[1];
@@ -78,11 +79,12 @@ void launch_copy(const CopyDesc* d, int count, long long max_elems, cudaStream_t
   if (count <= 0 || max_elems <= 0) return;
   // about four elements per thread; with `count` copies in the grid's y dimension
   dim3 grid(elem_blocks(max_elems, 4 * NT, count), (unsigned)count);
-  copy4_kernel<<<grid, NT, 0, s>>>(d);
+  launch_dep(copy4_kernel, grid, NT, 0, s, d);
   TTC_CHECK_LAUNCH();
 }
 
 __global__ void zero_kernel(const ZeroDesc* __restrict__ descs) {
+  dep_wait();
   const ZeroDesc D = descs[blockIdx.y];
   const long long step = (long long)gridDim.x * NT;
   for (long long e = (long long)blockIdx.x * NT + threadIdx.x; e < D.n; e += 4 * step) {
@@ -94,12 +96,13 @@ __global__ void zero_kernel(const ZeroDesc* __restrict__ descs) {
 
 void launch_zero(const ZeroDesc* d, int count, long long max_n, cudaStream_t s) {
   if (count <= 0 || max_n <= 0) return;
-  zero_kernel<<<dim3(elem_blocks(max_n, 4 * NT, count), (unsigned)count), NT, 0, s>>>(d);
+  launch_dep(zero_kernel, dim3(elem_blocks(max_n, 4 * NT, count), (unsigned)count), NT, 0, s, d);
   TTC_CHECK_LAUNCH();
 }
 
 // ---------------------------------------------------------------- sum of squares
 __global__ void sumsq_kernel(const NormDesc* __restrict__ descs) {
+  dep_wait();
   __shared__ double red[NT / 32];
   const NormDesc D = descs[blockIdx.x];
   double a = 0.0;
@@ -116,7 +119,7 @@ __global__ void sumsq_kernel(const NormDesc* __restrict__ descs) {
 
 void launch_sumsq(const NormDesc* d, int count, cudaStream_t s) {
   if (count <= 0) return;
-  sumsq_kernel<<<count, NT, 0, s>>>(d);
+  launch_dep(sumsq_kernel, count, NT, 0, s, d);
   TTC_CHECK_LAUNCH();
 }
 
@@ -129,6 +132,7 @@ void launch_sumsq(const NormDesc* d, int count, cudaStream_t s) {
 constexpr int kTruncStage = 2048;
 __global__ void __launch_bounds__(32) truncate_kernel(const TruncDesc* __restrict__ descs, int count, double tol,
                                                       long long rmax) {
+  dep_wait();
   __shared__ double sv[kTruncStage];
   const int p = blockIdx.x, lane = threadIdx.x;
   if (p >= count) return;
@@ -174,12 +178,13 @@ __global__ void __launch_bounds__(32) truncate_kernel(const TruncDesc* __restric
 
 void launch_truncate(const TruncDesc* d, int count, double tol, long long rmax, cudaStream_t s) {
   if (count <= 0) return;
-  truncate_kernel<<<count, 32, 0, s>>>(d, count, tol, rmax);
+  launch_dep(truncate_kernel, count, 32, 0, s, d, count, tol, rmax);
   TTC_CHECK_LAUNCH();
 }
 
 // ---------------------------------------------------------------- column selection
 __global__ void select_kernel(const SelectDesc* __restrict__ descs) {
+  dep_wait();
   const SelectDesc D = descs[blockIdx.y];
   const int k = *D.rank;
   const int rows = max(D.rows, D.zrows);
@@ -200,7 +205,7 @@ __global__ void select_kernel(const SelectDesc* __restrict__ descs) {
 void launch_select(const SelectDesc* d, int count, int max_rows, int max_cols, cudaStream_t s) {
   if (count <= 0) return;
   const long long total = (long long)max_rows * max_cols;
-  select_kernel<<<dim3(elem_blocks(total, NT, count), (unsigned)count), NT, 0, s>>>(d);
+  launch_dep(select_kernel, dim3(elem_blocks(total, NT, count), (unsigned)count), NT, 0, s, d);
   TTC_CHECK_LAUNCH();
 }
 
@@ -215,6 +220,7 @@ void launch_select(const SelectDesc* d, int count, int max_rows, int max_cols, c
 // through the column by constant increments (the block size divided by R), with no division per
 // element; an element costs 2n shared-memory loads, n FMAs and one store.
 __global__ void apply_kernel(const ApplyDesc* __restrict__ descs) {
+  dep_wait();
   extern __shared__ double asm_[];
   const ApplyDesc D = descs[blockIdx.y];
   const int nun = blockIdx.x;
@@ -266,7 +272,7 @@ void launch_apply(const ApplyDesc* d, int count, int max_rn, int max_smem_double
   attr_once.run(dev, [] {
     TTC_CUDA(cudaFuncSetAttribute(apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
   });
-  apply_kernel<<<dim3((unsigned)max_rn, (unsigned)count), NT, smem, s>>>(d);
+  launch_dep(apply_kernel, dim3((unsigned)max_rn, (unsigned)count), NT, smem, s, d);
   TTC_CHECK_LAUNCH();
 }
 
@@ -288,6 +294,7 @@ __device__ __forceinline__ void philox10(unsigned c[4], unsigned k0, unsigned k1
 }
 
 __global__ void philox_kernel(const PhiloxDesc* __restrict__ descs) {
+  dep_wait();
   const PhiloxDesc D = descs[blockIdx.y];
   const long long nctr = (D.count + 3) / 4;
   const double inv = 1.0 / 4294967296.0;
@@ -313,7 +320,7 @@ __global__ void philox_kernel(const PhiloxDesc* __restrict__ descs) {
 void launch_philox(const PhiloxDesc* d, int count, long long max_count, cudaStream_t s) {
   if (count <= 0 || max_count <= 0) return;
   const long long blocks = std::min<long long>(((max_count + 3) / 4 + NT - 1) / NT, 148LL * 8);
-  philox_kernel<<<dim3((unsigned)blocks, (unsigned)count), NT, 0, s>>>(d);
+  launch_dep(philox_kernel, dim3((unsigned)blocks, (unsigned)count), NT, 0, s, d);
   TTC_CHECK_LAUNCH();
 }
 
