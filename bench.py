@@ -357,8 +357,7 @@ def other_configs(ttcuda, ctx, hbm_peak, stream):
     gd = math.sqrt(sum(float(np.sum((a - b) ** 2)) for a, b in zip(G32, G64)))
     gn = math.sqrt(sum(float(np.sum(b ** 2)) for b in G64))
     out["config4"] = {"workload": "gradient of <x|H|x>/<x|x> w.r.t. every core, 4x4 open Hubbard MPO (t=1, U=8, "
-                                  f"snake ordering, MPO ranks up to {max(H4.tto_rks)}), x rank 256, environments "
-                                  "checkpointed every 4 sites, FP64",
+                                  f"snake ordering, MPO ranks up to {max(H4.tto_rks)}), x rank 256, FP64",
                       "value": 1e3 / ms_g, "unit": "gradients/s", "ms": ms_g,
                       "path": "ttc_rayleigh_grad on host tensors",
                       "gemm_f64": {"ms": prof4[0], "launches": prof4[1], "gflop": prof4[2] / 1e9,

@@ -109,7 +109,7 @@ __device__ __forceinline__ float round_tf32(float x) {
 // blocks may be set up while the one before drains, and waits at its first statement until that one has
 // completed and its writes are visible.  Every thread of every kernel launched so makes dep_wait its first
 // statement (before any return): a kernel ends only after all those before it.
-// Rounding of 20 sites at rank 15 (173 launches) 1.457 -> 1.378 ms, operator rounding at r 128, R 6 (288) 8.88 ->
+// Rounding a sum of three rank-5 trains of 12 sites (173 launches) 1.457 -> 1.378 ms, operator rounding at r 128, R 6 (288) 8.88 ->
 // 8.41, a dot and a partial contraction (130) 2.75 -> 2.56, batches and large ranks the same.  No kernel lets the
 // next one start early (griddepcontrol.launch_dependents): blocks that wait beside running ones cost 1.43, 9.30,
 // 2.56 in these and 19.4 -> 20.8 in a randomized batch; only below 64 or 8 blocks 1.42 and 1.43 in the first.

@@ -756,8 +756,9 @@ double norm_host(ttc_context* c, const ttc_ttv* x) {
 // site; the contractions with L_k then go in one launch for all sites.
 // One launch per product, the products with R_{k+1} formed twice and the left chain run again from
 // checkpoints every four sites took 600 launches and 11.6 ms at d 32, r 192, R 18 where this takes 100
-// launches and 4.0 ms; in FP32 19.2 and 3.5 ms (6.2 before the smaller tiles of the FP32 GEMM).  What is kept per site (r n r R + r r R numbers) is less
-// than the scratch of that recomputation (five such blocks a site), so `ckpt` no longer changes the layout.
+// launches and 4.0 ms; in FP32 19.2 and 3.5 ms.  What is kept per site (r n r R + r r R numbers) is less than
+// the scratch of that recomputation (five such blocks a site): a context holds 0.76 GB after this gradient,
+// where it held 2.0 GB with every environment stored and 2.8 with every fourth.  So `ckpt` has no effect.
 void rayleigh_grad_host(ttc_context* c, const ttc_tto* Hh, const ttc_ttv* x, int ckpt, double* value,
                         double* const* grads, bool f32) {
   BatchHolder BH;
