@@ -10,7 +10,8 @@
 //
 // What bounds it: the tensor cores' 64 FMA per cycle and SM, that is 1024 cycles for 16 K steps of a
 // 64 x 64 tile, so that a launch of a few such tiles leaves most SMs idle for K / 16 of these.  The tile
-// is therefore chosen for a whole launch (gemm_pick_tile) among 64 x 64, 64 x 32 and 32 x 32.
+// is therefore chosen for a whole launch (gemm_pick_tile) among 64 x 64, 64 x 32, 32 x 32 and
+// 16 x 16.
 // Every output element adds its K steps in the same order whatever the tile, and the K splits are a
 // function of the shapes alone, so the choice does not change a bit of the result.
 //
@@ -35,7 +36,7 @@ constexpr int BK = 16;
 constexpr int REF_BM = 64, REF_BN = 64;
 
 struct TileShape { int bm, bn; };
-constexpr TileShape kTiles[kGemmTiles] = {{64, 64}, {64, 32}, {32, 32}};
+constexpr TileShape kTiles[kGemmTiles] = {{64, 64}, {64, 32}, {32, 32}, {16, 16}};
 
 __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -286,7 +287,8 @@ void launch_gemm_f64(const GemmDesc* d_descs, int nd, long long total_tiles, int
   switch (tile) {
     case 0: launch_t<64, 64, 2, 2, 4, 3>(d_descs, nd, total_tiles, s); break;
     case 1: launch_t<64, 32, 2, 2, 5, 3>(d_descs, nd, total_tiles, s); break;
-    default: launch_t<32, 32, 2, 2, 4, 6>(d_descs, nd, total_tiles, s); break;
+    case 2: launch_t<32, 32, 2, 2, 4, 6>(d_descs, nd, total_tiles, s); break;
+    default: launch_t<16, 16, 2, 2, 4, 8>(d_descs, nd, total_tiles, s); break;
   }
 }
 
@@ -318,15 +320,21 @@ int gemm_pick_tile(const GemmDesc* d, int nd, int nsm) {
   // shape against this rule (ms): operator rounding r 320 x R 64 16.8 / 18.1 / 20.5 against 15.9, r 128 x R 6
   // 4.3 / 3.1 / 3.0 against 3.0, gradient 14.6 / 11.9 / 11.7 against 11.6, 60 ragged trains 6.2 / 5.6 / 5.7
   // against 5.6.
-  constexpr double cost[kGemmTiles] = {1.0, 1.05, 1.3};
+  constexpr double cost[3] = {1.0, 1.05, 1.3};
   int best = 0;
   double best_t = 0.0;
-  for (int t = 0; t < kGemmTiles; ++t) {
-    long long tiles = 0;
+  long long tiles = 0;
+  for (int t = 0; t < 3; ++t) {
+    tiles = 0;
     for (int i = 0; i < nd; ++i) tiles += gemm_tiles(d[i], t);
     const double turns = (double)((tiles + nsm - 1) / nsm) * kTiles[t].bm * kTiles[t].bn * cost[t];
     if (t == 0 || turns < best_t) { best = t; best_t = turns; }
   }
+  // Launches of at most one 32 x 32 tile per SM wait for the instructions of the one warp on each scheduler
+  // (170 per K step, 6 cycles each), of which a 16 x 16 tile has half: operator rounding at r 128, R 6 8.40 ->
+  // 8.12 ms, a dot and a partial contraction 2.57 -> 2.39, three rank-5 trains rounded 1.370 -> 1.338.  Eight
+  // warps per tile 8.23, 2.51, 1.355; 16 x 32 tiles 8.25, 2.44, 1.362; up to two tiles per SM the same.
+  if (best == 2 && tiles <= nsm) best = 3;
   return best;
 }
 

@@ -16,7 +16,7 @@ inline unsigned elem_blocks(long long max_elems, int per_block, int count) {
 
 // ---- grouped FP64 GEMM (gemm_f64.cu)
 // tile: one of the output tile shapes (gemm_pick_tile), for which the descriptors' tile_start is filled.
-constexpr int kGemmTiles = 3;
+constexpr int kGemmTiles = 4;
 void launch_gemm_f64(const GemmDesc* d_descs, int nd, long long total_tiles, int tile, cudaStream_t s);
 // The tile shape for one launch of nd problems (ksplit set) on nsm SMs.
 int gemm_pick_tile(const GemmDesc* d, int nd, int nsm);

@@ -1,5 +1,5 @@
-"""The grouped FP64 GEMM at the edges of its three output tiles (64 x 64, 64 x 32, 32 x 32, chosen by the
-launch's size), over strides, split dimensions and K splits, and with more problems than one round of the
+"""The grouped FP64 GEMM at the edges of its four output tiles (64 x 64, 64 x 32, 32 x 32, 16 x 16, chosen by
+the launch's size), over strides, split dimensions and K splits, and with more problems than one round of the
 descriptor search covers."""
 import ctypes as C
 
@@ -29,7 +29,7 @@ def check(got, a, b, c0):
     assert (np.abs(got - want) <= (a.shape[-1] + 2) * EPS * mag).all()
 
 
-@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (31, 33, 15), (32, 32, 16), (33, 31, 17), (63, 65, 48), (64, 64, 64),
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (15, 17, 16), (16, 16, 33), (17, 15, 8), (31, 33, 15), (32, 32, 16), (33, 31, 17), (63, 65, 48), (64, 64, 64),
                                    (65, 63, 4), (97, 40, 80), (129, 95, 31)])
 @pytest.mark.parametrize("trans", [False, True])
 def test_tiles_agree(m, n, k, trans):
