@@ -63,6 +63,8 @@ CopyDesc cd3(const double* src, double* dst, long long e0, long long e1, long lo
              long long s2, long long d0, long long d1, long long d2, double alpha = 1.0);
 
 Plan* get_plan(ttc_context* c, const std::string& key, const std::function<void(Builder&)>& fn);
+// Bytes of workspace that get_plan would ask for.
+size_t plan_workspace(ttc_context* c, const std::function<void(Builder&)>& fn);
 void run_plan(ttc_context* c, Plan& p);
 void ensure_workspace(ttc_context* c, size_t bytes);
 // cudaMalloc that gives the context's idle blocks back and tries once more when memory runs out.

@@ -917,7 +917,8 @@ void rayleigh_grad_host(ttc_context* c, const ttc_tto* Hh, const ttc_ttv* x, int
     g1.push_back(a1);
     g2.push_back(gd(r0, r0, n * r1, Tn, 1, r0, xcore(k), xc, 1, Rn_new, 1, r0));
   };
-  run_once(c, [&](Builder& B) {
+  double nn = 1.0, Rq = 0.0;                          // of the first plan, for the second's scalings
+  const std::function<void(Builder&)> chains = [&](Builder& B) {
     reserve(B);
     size_t mh = 1, mn = 1;
     for (int k = 0; k < N; ++k) {
@@ -945,18 +946,9 @@ void rayleigh_grad_host(ttc_context* c, const ttc_tto* Hh, const ttc_ttv* x, int
     } else {
       B.copy({cd2(Lh[N], dval, 1, 1, 0, 0, 0, 0), cd2(Ln[N], dval + 1, 1, 1, 0, 0, 0, 0)});
     }
-  });
-  double hv[2];
-  TTC_CUDA(cudaMemcpy(hv, dval, sizeof(hv), cudaMemcpyDeviceToHost));
-  const double e = hv[0], nn = hv[1];
-  TTC_REQUIRE(nn > 0.0, TTC_EARG, "rayleigh_grad: <x|x> is zero");
-  const double Rq = e / nn;
-  *value = Rq;
-  ensure_stage(c, sizeof(double) * gsz + 256);        // the gradient in the caller's layout
-  const char* ws = c->ws;                             // the second plan needs no more of it than the first
-  run_once(c, [&](Builder& B) {
+  };
+  const std::function<void(Builder&)> products = [&](Builder& B) {
     reserve(B);
-    TTC_REQUIRE(c->ws == ws, TTC_EINTERNAL, "rayleigh_grad: the workspace moved between its plans");
     Descs gh, gn;
     for (int k = 0; k < N; ++k) {
       const int r0 = rk(k), R0 = Rk(k), nr = (int)X->dims[k] * rk(k + 1);
@@ -979,6 +971,22 @@ void rayleigh_grad_host(ttc_context* c, const ttc_tto* Hh, const ttc_ttv* x, int
       cp.push_back(cd3(wide + goff[k], (double*)c->d_stage + goff[k], n, r0, r1, r0, 1, r0 * n, 1, n, n * r0));
     }
     B.copy(cp);
+  };
+  // What the first plan leaves lies in the workspace, which therefore has to be large enough for both before
+  // the first one runs: the second one's K splits can need more of it (d 32, r 132, R 8: 94 MB against 88).
+  ensure_workspace(c, std::max(plan_workspace(c, chains), plan_workspace(c, products)));
+  ensure_stage(c, sizeof(double) * gsz + 256);        // the gradient in the caller's layout
+  const size_t ws_bytes = c->ws_bytes;
+  run_once(c, chains);
+  double hv[2];
+  TTC_CUDA(cudaMemcpy(hv, dval, 2 * sizeof(double), cudaMemcpyDeviceToHost));
+  nn = hv[1];
+  TTC_REQUIRE(nn > 0.0, TTC_EARG, "rayleigh_grad: <x|x> is zero");
+  Rq = hv[0] / nn;
+  *value = Rq;
+  run_once(c, [&](Builder& B) {
+    TTC_REQUIRE(c->ws_bytes == ws_bytes, TTC_EINTERNAL, "rayleigh_grad: the workspace grew between its plans");
+    products(B);
   });
   std::vector<HostCopy> out;
   for (int k = 0; k < N; ++k)

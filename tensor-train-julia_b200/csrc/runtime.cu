@@ -794,17 +794,26 @@ CopyDesc cd3(const double* src, double* dst, long long e0, long long e1, long lo
   return c;
 }
 
+// The measuring pass of a plan: its workspace and blob sizes, no addresses.
+static void measure_plan(ttc_context* c, const std::function<void(Builder&)>& fn, Plan& meas) {
+  Builder b;
+  b.ctx = c; b.plan = &meas; b.wsbase = nullptr; b.blob_base = nullptr;
+  fn(b);
+  meas.ws_needed = b.wshw;
+}
+
+size_t plan_workspace(ttc_context* c, const std::function<void(Builder&)>& fn) {
+  Plan meas;
+  measure_plan(c, fn, meas);
+  return meas.ws_needed;
+}
+
 // Two passes: measure (workspace and blob sizes), allocate, then build for real.
 Plan* get_plan(ttc_context* c, const std::string& key, const std::function<void(Builder&)>& fn) {
   auto it = c->plans.find(key);
   if (it != c->plans.end() && it->second->ws_base == (void*)c->ws) return it->second.get();
   std::unique_ptr<Plan> meas(new Plan());
-  {
-    Builder b;
-    b.ctx = c; b.plan = meas.get(); b.wsbase = nullptr; b.blob_base = nullptr;
-    fn(b);
-    meas->ws_needed = b.wshw;
-  }
+  measure_plan(c, fn, *meas);
   ensure_workspace(c, meas->ws_needed);
   std::unique_ptr<Plan> p(new Plan());
   const size_t blob_cap = meas->blob.size() + 256;
