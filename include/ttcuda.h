@@ -272,8 +272,10 @@ int ttc_tt_scale(ttc_context* ctx, double a, const ttc_ttv* x, ttc_ttv_out* out)
 /* Gradient of R(x) = <x|H|x>/<x|x> with respect to every core (H symmetric).
  * No reference method: it is assembled from the environment contractions of
  * src/als.jl:9-25 and dot_operator.  grads[k] has the layout of core k.
- * ckpt_every is accepted for its callers and has no effect: the environments and the
- * products kept for every site take less memory than recomputing them did. */
+ * ckpt_every > 1: when the environments and products of all sites take more than an eighth of
+ * the device's memory, only every ckpt_every-th left environment is stored and the others are
+ * recomputed, a segment of ckpt_every sites at a time (memory O(d / ckpt_every + ckpt_every)
+ * sites instead of O(d)).  ckpt_every <= 1, or less memory: everything is stored. */
 int ttc_rayleigh_grad(ttc_context* ctx, const ttc_tto* H, const ttc_ttv* x, int32_t ckpt_every,
                       double* value, double* const* grads);
 /* The same gradient with every contraction in a chosen precision: TTC_PREC_FP64, or TTC_PREC_FP32

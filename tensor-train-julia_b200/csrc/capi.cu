@@ -454,6 +454,9 @@ int ttc_create(ttc_context** out, int device) {
     const double one[8] = {1.0, 0, 0, 0, 0, 0, 0, 0};
     TTC_CUDA(cudaMemcpy(c->d_one, one, sizeof(one), cudaMemcpyHostToDevice));
     for (auto& e : c->ev) TTC_CUDA(cudaEventCreate(&e));
+    size_t free_bytes = 0, total_bytes = 0;
+    TTC_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+    c->grad_keep = total_bytes / 8;
   });
   if (st != TTC_OK) {
     g_err_noctx = c->err;

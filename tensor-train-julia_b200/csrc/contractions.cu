@@ -756,9 +756,12 @@ double norm_host(ttc_context* c, const ttc_ttv* x) {
 // site; the contractions with L_k then go in one launch for all sites.
 // One launch per product, the products with R_{k+1} formed twice and the left chain run again from
 // checkpoints every four sites took 600 launches and 11.6 ms at d 32, r 192, R 18 where this takes 100
-// launches and 4.0 ms; in FP32 19.2 and 3.5 ms.  What is kept per site (r n r R + r r R numbers) is less than
-// the scratch of that recomputation (five such blocks a site): a context holds 0.76 GB after this gradient,
-// where it held 2.0 GB with every environment stored and 2.8 with every fourth.  So `ckpt` has no effect.
+// launches and 4.0 ms; in FP32 19.2 and 3.5 ms.
+// What is kept per site, r n r R + r r R numbers, is more than a device has for the longest trains and largest
+// ranks.  Above the context's grad_keep bytes (an eighth of the device's memory) the left chain goes alone and
+// leaves every ckpt-th L_k; the right chain then goes from the last segment of ckpt sites to the first, a
+// segment's left environments formed again beside it: at the same case with every fourth, 10.9 ms in place of
+// 8.7 a call and 205 MB of workspace in place of 716, in FP32 9.9 in place of 7.3.
 void rayleigh_grad_host(ttc_context* c, const ttc_tto* Hh, const ttc_ttv* x, int ckpt, double* value,
                         double* const* grads, bool f32) {
   BatchHolder BH;
@@ -767,7 +770,6 @@ void rayleigh_grad_host(ttc_context* c, const ttc_tto* Hh, const ttc_ttv* x, int
   const int N = x->N;
   TTC_REQUIRE(H->N == N && H->dims == X->dims, TTC_EDIM, "rayleigh_grad: dimensions differ");
   TTC_REQUIRE(H->rks[N] == 1, TTC_EDIM, "rayleigh_grad: last operator rank must be 1");
-  (void)ckpt;
   // FP32 variant: float copies of the TT and MPO cores (same element offsets), every contraction
   // on the FP32 grouped GEMM, environments and gradient in float, widened for the host
   const size_t esz = f32 ? sizeof(float) : sizeof(double);
@@ -816,26 +818,37 @@ void rayleigh_grad_host(ttc_context* c, const ttc_tto* Hh, const ttc_ttv* x, int
   };
   auto rk = [&](int k) { return X->rk(0, k); };
   auto Rk = [&](int k) { return H->rks[k]; };
-  // What the first plan leaves for the second, at the start of the workspace of both: left environments,
-  // kept products, the quotient's two values in FP64, the gradient and its FP64 copy.
+  // What the first plan leaves for the second, at the start of the workspace of both: left environments
+  // (those with held(k)), the products kept with them, the quotient's two values in FP64 and the gradient.
   std::vector<double*> Lh(N + 1), Ln(N + 1), HxR(N), xRn(N);
   std::vector<size_t> goff(N);
-  size_t gsz = 0;
-  for (int k = 0; k < N; ++k) { goff[k] = gsz; gsz += (size_t)rk(k) * X->dims[k] * rk(k + 1); }
-  double *dG = nullptr, *dval = nullptr, *wide = nullptr;
+  size_t gsz = 0, keep = 0;
+  for (int k = 0; k < N; ++k) {
+    const size_t core = (size_t)rk(k) * X->dims[k] * rk(k + 1);
+    goff[k] = gsz;
+    gsz += core;
+    keep += esz * ((size_t)rk(k) * rk(k) * (Rk(k) + 1) + core * (Rk(k) + 1));
+  }
+  const bool all = ckpt <= 1 || keep <= c->grad_keep;
+  auto held = [&](int k) { return all || k % ckpt == 0 || k == N; };
+  double *dG = nullptr, *dval = nullptr;
+  auto elems = [&](Builder& B, size_t n) { return B.wd((n * esz + 7) / 8); };
+  auto env = [&](Builder& B, int k) {
+    Lh[k] = elems(B, (size_t)rk(k) * Rk(k) * rk(k));
+    Ln[k] = elems(B, (size_t)rk(k) * rk(k));
+  };
+  auto kept_products = [&](Builder& B, int k) {
+    const size_t core = (size_t)rk(k) * X->dims[k] * rk(k + 1);
+    HxR[k] = elems(B, core * Rk(k));
+    xRn[k] = elems(B, core);
+  };
   auto reserve = [&](Builder& B) {
-    auto kept = [&](size_t elems) { return B.wd((elems * esz + 7) / 8); };
     for (int k = 0; k <= N; ++k) {
-      Lh[k] = kept((size_t)rk(k) * Rk(k) * rk(k));
-      Ln[k] = kept((size_t)rk(k) * rk(k));
-      if (k == N) break;
-      const size_t core = (size_t)rk(k) * X->dims[k] * rk(k + 1);
-      HxR[k] = kept(core * Rk(k));
-      xRn[k] = kept(core);
+      if (held(k)) env(B, k);
+      if (all && k < N) kept_products(B, k);
     }
     dval = B.wd(4);
-    dG = kept(gsz);                                   // this precision, offsets goff
-    wide = f32 ? B.wd(gsz) : dG;
+    dG = elems(B, gsz);                               // this precision, offsets goff
   };
   auto gcore = [&](int k) -> double* {
     return f32 ? reinterpret_cast<double*>(reinterpret_cast<float*>(dG) + goff[k]) : dG + goff[k];
@@ -847,9 +860,9 @@ void rayleigh_grad_host(ttc_context* c, const ttc_tto* Hh, const ttc_ttv* x, int
     const int r0 = rk(k), r1 = rk(k + 1), R0 = Rk(k), R1 = Rk(k + 1), n = (int)X->dims[k];
     const int xc = X->capr(0, k);
     // T1[(a, b), (j, c')] = sum_c L[a,b,c] x[c, j, c']   (L as ((a,b) x c))
-    double* T1 = B.wd((size_t)r0 * R0 * n * r1);
+    double* T1 = elems(B, (size_t)r0 * R0 * n * r1);
     g1.push_back(gd(r0 * R0, n * r1, r0, Lh[k], 1, (long long)r0 * R0, xcore(k), 1, xc, T1, 1, (long long)r0 * R0));
-    double* T2 = B.wd((size_t)r0 * n * r1 * R1);
+    double* T2 = elems(B, (size_t)r0 * n * r1 * R1);
     // T2[(a, c'), (i, b')] = sum_{(b,j)} T1[a, b, j, c'] H[b, i, j, b']   (stored (a, i, c', b'))
     GemmDesc f{};
     f.m = r0 * r1; f.n = n * R1; f.k = R0 * n; f.batch = 1;
@@ -870,7 +883,7 @@ void rayleigh_grad_host(ttc_context* c, const ttc_tto* Hh, const ttc_ttv* x, int
     h.alpha = 1.0; h.beta = 0.0;
     g3.push_back(h);
     // norm env: Ln'[a', c'] = sum x[a,i,a'] (sum_c Ln[a,c] x[c,i,c'])
-    double* U = B.wd((size_t)r0 * n * r1);
+    double* U = elems(B, (size_t)r0 * n * r1);
     g1.push_back(gd(r0, n * r1, r0, Ln[k], 1, r0, xcore(k), 1, xc, U, 1, r0));
     GemmDesc q{};
     q.m = r1; q.n = r1; q.k = r0 * n; q.batch = 1;
@@ -890,7 +903,7 @@ void rayleigh_grad_host(ttc_context* c, const ttc_tto* Hh, const ttc_ttv* x, int
     const int r0 = rk(k), r1 = rk(k + 1), R0 = Rk(k), R1 = Rk(k + 1), n = (int)X->dims[k];
     const int xc = X->capr(0, k);
     // U[(c, j), (e, d)] = sum_f x[c,j,f] R[f,e,d]
-    double* U = B.wd((size_t)r0 * n * R1 * r1);
+    double* U = elems(B, (size_t)r0 * n * R1 * r1);
     GemmDesc u = gd(r0 * n, R1 * r1, r1, xcore(k), 1, (long long)xc * n, Rh, R1, 1, U, 1, (long long)r0 * n);
     u.m0 = r0; u.a_i0 = 1; u.a_i1 = xc; u.c_i0 = 1; u.c_i1 = r0;
     u.n0 = R1; u.b_j0 = 1; u.b_j1 = (long long)R1 * r1;
@@ -911,32 +924,62 @@ void rayleigh_grad_host(ttc_context* c, const ttc_tto* Hh, const ttc_ttv* x, int
     if (k == 0) return;
     // R_k[(b, c), a] = sum_{(i, d)} HxR[(b, c), (i, d)] x[a, i, d]
     g3.push_back(gd(R0 * r0, r0, n * r1, HxR[k], 1, (long long)R0 * r0, xcore(k), xc, 1, Rh_new, 1, (long long)R0 * r0));
-    double* Tn = B.wd((size_t)r0 * n * r1);
+    double* Tn = elems(B, (size_t)r0 * n * r1);
     GemmDesc a1 = gd(r0 * n, r1, r1, xcore(k), 1, (long long)xc * n, Rn, 1, r1, Tn, 1, (long long)r0 * n);
     a1.m0 = r0; a1.a_i0 = 1; a1.a_i1 = xc; a1.c_i0 = 1; a1.c_i1 = r0;
     g1.push_back(a1);
     g2.push_back(gd(r0, r0, n * r1, Tn, 1, r0, xcore(k), xc, 1, Rn_new, 1, r0));
   };
   double nn = 1.0, Rq = 0.0;                          // of the first plan, for the second's scalings
-  const std::function<void(Builder&)> chains = [&](Builder& B) {
-    reserve(B);
+  // two buffers for each environment of a chain, used in turn
+  auto in_turn = [&](Builder& B, double* (&h)[2], double* (&m)[2]) {
     size_t mh = 1, mn = 1;
     for (int k = 0; k < N; ++k) {
       mh = std::max(mh, (size_t)rk(k) * Rk(k) * rk(k));
       mn = std::max(mn, (size_t)rk(k) * rk(k));
     }
-    double* Rh[2] = {B.wd(mh), B.wd(mh)};
-    double* Rn[2] = {B.wd(mn), B.wd(mn)};
-    for (double* one : {Lh[0], Ln[0], Rh[0], Rn[0]}) set_one(B, one);
-    for (int t = 0; t < N; ++t) {
-      const size_t mk = B.mark();
-      Descs g1, g2, g3;
-      left_step(B, t, g1, g2, g3);
-      right_step(B, N - 1 - t, Rh[t & 1], Rn[t & 1], Rh[(t + 1) & 1], Rn[(t + 1) & 1], g1, g2, g3);
-      GEMM(B, g1);
-      GEMM(B, g2);
-      GEMM(B, g3);
-      B.release(mk);
+    for (double** p : {&h[0], &h[1]}) *p = elems(B, mh);
+    for (double** p : {&m[0], &m[1]}) *p = elems(B, mn);
+  };
+  double *Rh[2], *Rn[2];
+  // One turn: the left step from site l and the right step from site r (-1: none).
+  auto turn = [&](Builder& B, int l, int r) {
+    const size_t mk = B.mark();
+    Descs g1, g2, g3;
+    if (l >= 0) left_step(B, l, g1, g2, g3);
+    const int t = (N - 1 - r) & 1;
+    if (r >= 0) right_step(B, r, Rh[t], Rn[t], Rh[t ^ 1], Rn[t ^ 1], g1, g2, g3);
+    GEMM(B, g1);
+    GEMM(B, g2);
+    GEMM(B, g3);
+    B.release(mk);
+  };
+  // The gradient of sites lo .. hi - 1 from their left environments and kept products.
+  auto gradient = [&](Builder& B, int lo, int hi) {
+    Descs gh, gn;
+    for (int k = lo; k < hi; ++k) {
+      const int r0 = rk(k), R0 = Rk(k), nr = (int)X->dims[k] * rk(k + 1);
+      // G[a, (i, d)] = (2/nn) sum_{(b, c)} L[a, b, c] HxR[(b, c), (i, d)]
+      gh.push_back(gd(r0, nr, R0 * r0, Lh[k], 1, r0, HxR[k], 1, (long long)R0 * r0, gcore(k), 1, r0, 2.0 / nn));
+      // G -= (2R/nn) Ln[a,c] xRn[c,(i,d)]
+      gn.push_back(gd(r0, nr, r0, Ln[k], 1, r0, xRn[k], 1, r0, gcore(k), 1, r0, -2.0 * Rq / nn, 1.0));
+    }
+    GEMM(B, gh);
+    GEMM(B, gn);
+  };
+  const std::function<void(Builder&)> chains = [&](Builder& B) {
+    reserve(B);
+    if (all) {
+      in_turn(B, Rh, Rn);
+      for (double* one : {Lh[0], Ln[0], Rh[0], Rn[0]}) set_one(B, one);
+      for (int t = 0; t < N; ++t) turn(B, t, N - 1 - t);
+    } else {
+      double *h[2], *m[2];
+      in_turn(B, h, m);
+      for (int k = 0; k < N; ++k)
+        if (!held(k)) { Lh[k] = h[k & 1]; Ln[k] = m[k & 1]; }
+      for (double* one : {Lh[0], Ln[0]}) set_one(B, one);
+      for (int t = 0; t < N; ++t) turn(B, t, -1);
     }
     if (f32) {
       CvtDesc w1{}, w2{};
@@ -949,17 +992,26 @@ void rayleigh_grad_host(ttc_context* c, const ttc_tto* Hh, const ttc_ttv* x, int
   };
   const std::function<void(Builder&)> products = [&](Builder& B) {
     reserve(B);
-    Descs gh, gn;
-    for (int k = 0; k < N; ++k) {
-      const int r0 = rk(k), R0 = Rk(k), nr = (int)X->dims[k] * rk(k + 1);
-      // G[a, (i, d)] = (2/nn) sum_{(b, c)} L[a, b, c] HxR[(b, c), (i, d)]
-      gh.push_back(gd(r0, nr, R0 * r0, Lh[k], 1, r0, HxR[k], 1, (long long)R0 * r0, gcore(k), 1, r0, 2.0 / nn));
-      // G -= (2R/nn) Ln[a,c] xRn[c,(i,d)]
-      gn.push_back(gd(r0, nr, r0, Ln[k], 1, r0, xRn[k], 1, r0, gcore(k), 1, r0, -2.0 * Rq / nn, 1.0));
+    if (all) {
+      gradient(B, 0, N);
+    } else {
+      in_turn(B, Rh, Rn);
+      for (double* one : {Rh[0], Rn[0]}) set_one(B, one);
+      for (int hi = N; hi > 0;) {
+        const int lo = (hi - 1) / ckpt * ckpt;
+        const size_t mk = B.mark();
+        for (int k = lo; k < hi; ++k) {
+          if (k > lo) env(B, k);
+          kept_products(B, k);
+        }
+        for (int t = 0; t < hi - lo; ++t) turn(B, t < hi - lo - 1 ? lo + t : -1, hi - 1 - t);
+        gradient(B, lo, hi);
+        B.release(mk);
+        hi = lo;
+      }
     }
-    GEMM(B, gh);
-    GEMM(B, gn);
     // internal (a, i, d) -> Julia (i, a, d) in the staging area
+    double* wide = f32 ? B.wd(gsz) : dG;
     if (f32) {
       CvtDesc w{};
       w.src = dG; w.dst = wide; w.rows = (long long)gsz; w.cols = 1; w.ss_i = 1; w.ds_i = 1; w.alpha = 1.0;

@@ -129,6 +129,7 @@ struct ttc_context {
   // batch identity, replay the captured plan
   std::vector<std::pair<std::string, ttc_batch*>> oneshot;
   ttc::BlockPool blocks;
+  size_t grad_keep = 0;              // bytes up to which a gradient keeps every site's environments
 };
 
 struct ttc_batch {

@@ -63,6 +63,15 @@ int ttc_test_set_jacobi_max_sweeps(ttc_context* c, int sweeps) {
   }
 }
 
+// Sets the bytes up to which the context's gradients keep every site's environments (default: an eighth of
+// the device's memory); *ws_bytes: the context's workspace as it stands.
+int ttc_test_grad_keep(ttc_context* c, long long bytes, long long* ws_bytes) {
+  return hook(c, [&] {
+    c->grad_keep = (size_t)bytes;
+    *ws_bytes = (long long)c->ws_bytes;
+  });
+}
+
 // Sets the poll limit of the tensor-core GEMM's bounded mbarrier waits on the context's device
 // (default 2^24), so that a test can make the waits run out on purpose.
 int ttc_test_set_tc_wait_limit(ttc_context* c, long long polls) {

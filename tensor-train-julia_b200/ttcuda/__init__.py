@@ -614,8 +614,9 @@ def tt_scale(a: float, x: TTvector) -> TTvector:
 
 def rayleigh_grad(H: TToperator, x: TTvector, ckpt_every: int = 4, precision: str = "fp64"):
     """Value and gradient of <x|H|x>/<x|x> with respect to every core of x (H symmetric), with
-    the contractions in FP64 or in FP32 with FP32 accumulation (precision="fp32").  ckpt_every has
-    no effect: the environments of every site are held."""
+    the contractions in FP64 or in FP32 with FP32 accumulation (precision="fp32").
+    When the environments and products of all sites take more than an eighth of the device's memory, only
+    every ckpt_every-th left environment is held and the others are recomputed (ckpt_every=1: never)."""
     prec = {"fp64": 0, "fp32": 3}.get(precision)
     if prec is None:
         raise ArgumentError(f"precision must be 'fp64' or 'fp32', not {precision!r}")

@@ -1,5 +1,8 @@
-"""The Rayleigh gradient's device memory: its two plans share what the first one leaves for the second, so
-a context whose workspace an earlier call has grown to any size in between must give the same bits."""
+"""The Rayleigh gradient's device memory.  Its two plans share what the first one leaves for the second, so
+a context whose workspace an earlier call has grown to any size in between must give the same bits; and above
+a bound it keeps only every ckpt_every-th left environment."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -28,3 +31,43 @@ def test_after_a_smaller_gradient(d, n, r, R, before, monkeypatch):
         ttcuda.rayleigh_grad(H, train(g, d, n, r0))
         v, G = ttcuda.rayleigh_grad(H, x)
         assert v == want and all(np.array_equal(a, b) for a, b in zip(G, Gw))
+
+
+def grad_keep(ctx, nbytes):
+    ws = C.c_longlong()
+    ctx.check(ttcuda.lib.ttc_test_grad_keep(ctx.h, C.c_longlong(nbytes), C.byref(ws)))
+    return ws.value
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("d", [1, 2, 9, 12])
+def test_checkpointed_gradient(d, precision, monkeypatch):
+    """Below 512 terms no sum is split, and a recomputed environment is the same bits: so is the gradient,
+    for segments of one site, that end short, and of more sites than there are."""
+    g = np.random.default_rng(d)
+    H, x = train(g, d, 3, 5, True), train(g, d, 3, 21)
+    want, Gw = ttcuda.rayleigh_grad(H, x, precision=precision)
+    ctx = ttcuda.Context(0)
+    monkeypatch.setattr(ttcuda, "_CTX", ctx)
+    grad_keep(ctx, 0)
+    for ckpt in (2, 3, 4, 5, 8, 20, 1, 0):
+        v, G = ttcuda.rayleigh_grad(H, x, ckpt_every=ckpt, precision=precision)
+        assert v == want and all(np.array_equal(a, b) for a, b in zip(G, Gw))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_checkpoints_bound_the_memory(precision, monkeypatch):
+    """Of 48 sites, each with an environment of r r R numbers and products of n r r R (n = 2): with all kept
+    48 x 3 such blocks; with every sixth environment kept 8 + 5 environments and the products of six sites, 25
+    blocks, and in both the scratch of a turn, at most 8."""
+    g = np.random.default_rng(1)
+    H, x = train(g, 48, 2, 6, True), train(g, 48, 2, 64)
+    used = {}
+    for keep, ckpt in ((1 << 40, 6), (0, 1), (0, 6)):
+        ctx = ttcuda.Context(0)
+        monkeypatch.setattr(ttcuda, "_CTX", ctx)
+        grad_keep(ctx, keep)
+        ttcuda.rayleigh_grad(H, x, ckpt_every=ckpt, precision=precision)
+        used[keep, ckpt] = grad_keep(ctx, keep)
+    assert used[0, 1] == used[1 << 40, 6]
+    assert used[0, 6] <= 0.4 * used[0, 1]
