@@ -448,11 +448,12 @@ int ttc_create(ttc_context** out, int device) {
     c->own_stream = true;
     TTC_CUDA(cudaMalloc(&c->d_flags, 64));
     region_add(c->d_flags, 64);
-    TTC_CUDA(cudaMemset(c->d_flags, 0, 64));
+    TTC_CUDA(cudaMemsetAsync(c->d_flags, 0, 64, c->stream));
     TTC_CUDA(cudaMalloc(&c->d_one, 64));
     region_add(c->d_one, 64);
     const double one[8] = {1.0, 0, 0, 0, 0, 0, 0, 0};
-    TTC_CUDA(cudaMemcpy(c->d_one, one, sizeof(one), cudaMemcpyHostToDevice));
+    TTC_CUDA(cudaMemcpyAsync(c->d_one, one, sizeof(one), cudaMemcpyHostToDevice, c->stream));
+    TTC_CUDA(cudaStreamSynchronize(c->stream));
     for (auto& e : c->ev) TTC_CUDA(cudaEventCreate(&e));
     size_t free_bytes = 0, total_bytes = 0;
     TTC_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));

@@ -827,7 +827,9 @@ Plan* get_plan(ttc_context* c, const std::string& key, const std::function<void(
     p->ws_needed = b.wshw;
   }
   TTC_REQUIRE(p->blob.size() <= blob_cap, TTC_EINTERNAL, "plan blob grew between passes");
-  TTC_CUDA(cudaMemcpy(p->d_blob, p->blob.data(), p->blob.size(), cudaMemcpyHostToDevice));
+  // On the stream that the plan runs on: a copy on another one may return with its last part still on the way
+  // (pageable memory goes through a staging buffer), and a kernel would read descriptors that are not there yet.
+  TTC_CUDA(cudaMemcpyAsync(p->d_blob, p->blob.data(), p->blob.size(), cudaMemcpyHostToDevice, c->stream));
   p->ws_base = c->ws;
   Plan* raw = p.get();
   c->stats.plans_built += 1;

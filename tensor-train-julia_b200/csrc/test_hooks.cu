@@ -39,10 +39,16 @@ int hook(ttc_context* c, F&& f) {
   }
 }
 
+// The plan of a hook, once the hook's own copies and fills (on the legacy stream) have arrived.
+Plan* hook_plan(ttc_context* c, const std::string& key, const std::function<void(Builder&)>& fn) {
+  TTC_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+  return get_plan(c, key, fn);
+}
+
 void run_plan_once(ttc_context* c, const std::function<void(Builder&)>& fn) {
   static unsigned long long serial = 0;
   const std::string key = "hook:" + std::to_string(++serial);
-  Plan* p = get_plan(c, key, fn);
+  Plan* p = hook_plan(c, key, fn);
   run_plan(c, *p);
   TTC_CUDA(cudaStreamSynchronize(c->stream));
   c->plans.erase(key);
@@ -97,7 +103,7 @@ int ttc_test_tc_gemm_bench(ttc_context* c, int m, int n, int k, int tf32, int re
       B.cvt_bf16({a, b}, tf32 != 0);
     });
     std::string key = "tcbench:" + std::to_string(m) + ":" + std::to_string(n) + ":" + std::to_string(k);
-    Plan* p = get_plan(c, key, [&](Builder& B) {
+    Plan* p = hook_plan(c, key, [&](Builder& B) {
       Bf16GemmDesc d{};
       d.m = m; d.n = n; d.k = k; d.m0 = m;
       d.A = dA.p; d.lda = ld; d.B = dB.p; d.ldb = ld;
@@ -153,7 +159,7 @@ int ttc_test_gemm_runs(ttc_context* c, int m, int n, int k, int batch, int m0, i
     static unsigned long long serial = 0;
     const std::string key = "hook-gemm:" + std::to_string(++serial);
     int ks = 1;
-    Plan* p = get_plan(c, key, [&](Builder& B) {
+    Plan* p = hook_plan(c, key, [&](Builder& B) {
       GemmDesc d{};
       d.m = m; d.n = n; d.k = k; d.batch = batch; d.m0 = m0; d.n0 = n0; d.k0e = k0e;
       d.A = dA.as<double>(); d.a_i0 = as[0]; d.a_i1 = as[1]; d.a_k0 = as[2]; d.a_k1 = as[3]; d.a_b = as[4];
@@ -278,7 +284,7 @@ int ttc_test_jacobi_bench(ttc_context* c, int count, int m, int n, const double*
     TTC_CUDA(cudaMemcpy(d0.p, X, per * count * 8, cudaMemcpyHostToDevice));
     static unsigned long long serial = 0;
     const std::string key = "hook-jacobi:" + std::to_string(++serial);
-    Plan* p = get_plan(c, key, [&](Builder& B) {
+    Plan* p = hook_plan(c, key, [&](Builder& B) {
       for (int r = 0; r < reps; ++r) {
         if (r == 0) B.stage(0);
         B.copy({cd2(d0.as<double>(), dX.as<double>(), (long long)(per * count), 1, 1, 0, 1, 0)});
