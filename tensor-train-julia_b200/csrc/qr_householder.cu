@@ -373,6 +373,10 @@ __device__ __forceinline__ void form_t(const PanelSm& S, int jb, double* Tg) {
 // c > jj then take the reflector (x unscaled), for c < jj the product is an entry of V^T V.  The warp of
 // column jj + 1 publishes that column and its squared norm.  The reflectors are scaled, and T formed,
 // after the last step.
+// The panel is factored times a power of two that brings its largest entry to 2^480, so that no square
+// leaves the normal range (columns of norms from 1e-290 to 1e300; without it from 1.5e-154 to 1e154): the
+// reflectors and T do not depend on the scale, and R takes it back.  Every operation commutes with it, so it
+// does not change a bit of what is in range without it.
 template <int NW, int LPC, int RI>
 __device__ __noinline__ bool factor_panel(double* A, int lda, int mp, int jb, int crank, int csize, double* Tws) {
   extern __shared__ __align__(16) double sm[];
@@ -403,8 +407,20 @@ __device__ __noinline__ bool factor_panel(double* A, int lda, int mp, int jb, in
 #pragma unroll
     for (int i = 0; i < RI; ++i)
       hi = max(hi, max(__double2hiint(cr[q][i][0]) & 0x7fffffff, __double2hiint(cr[q][i][1]) & 0x7fffffff));
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  int* his = reinterpret_cast<int*>(S.sv);    // free until the scales are written
+  if (lane == 0) his[warp] = hi;
   __syncwarp();
   cluster_arrive();                           // this CTA has read the panel (waited for before it is overwritten)
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < NW; ++w) hi = max(hi, his[w]);
+  const int sh = min(1000, 480 - ((hi >> 20) - 1023));
+  const double up = __hiloint2double((1023 + sh) << 20, 0), down = __hiloint2double((1023 - sh) << 20, 0);
+#pragma unroll
+  for (int q = 0; q < CPW; ++q)
+#pragma unroll
+    for (int i = 0; i < RI; ++i) { cr[q][i][0] *= up; cr[q][i][1] *= up; }
 
   // column j = c0 + q of some lanes of this warp
   auto publish = [&](const double (&v)[RI][2], int j, bool me) {
@@ -502,7 +518,7 @@ __device__ __noinline__ bool factor_panel(double* A, int lda, int mp, int jb, in
     const int c = c0 + q;
     const Reflector H(*reinterpret_cast<const double2*>(S.pub + 2 * min(c, jb - 1)));
     sc[q] = (c < jb) ? H.scale() : 0.0;
-    bc[q] = H.beta();
+    bc[q] = H.beta() * down;
     if (hl == 0) { S.sv[c] = sc[q]; S.tau[c] = (c < jb) ? H.tau() : 0.0; }
   }
   __syncthreads();
@@ -520,7 +536,7 @@ __device__ __noinline__ bool factor_panel(double* A, int lda, int mp, int jb, in
         v[e] = cr[q][i][e] * sc[q];
         g[e] = v[e];
         if (i == 0 && r + e <= c) {           // on and above the diagonal: R in global memory, V in the panel
-          g[e] = (r + e == c) ? bc[q] : cr[q][i][e];
+          g[e] = (r + e == c) ? bc[q] : cr[q][i][e] * down;
           v[e] = (r + e == c && own) ? 1.0 : 0.0;
         }
       }
