@@ -105,6 +105,39 @@ __device__ __forceinline__ float round_tf32(float x) {
   return __uint_as_float(r);
 }
 
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// D += A B on the FP64 tensor-core path (mma.sync m8n8k4): per lane a = A[lane>>2][lane&3],
+// b = B[lane&3][lane>>2], d = D[lane>>2][2(lane&3) + {0,1}].
+__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(d0), "+d"(d1)
+               : "d"(a), "d"(b));
+}
+
+// 1 / sqrt(x) for normal positive x below 2^1000: the hardware's approximation (relative error below
+// 2^-19) and one step of Chebyshev's third-order method for y^-2 = x, y (1 + e/2 + 3 e^2 / 8) with
+// e = 1 - x y^2: four dependent operations.  Its remainder 5 e^3 / 16 is below 2^-55, the rounding of x y
+// adds 2^-54 and the last one 2^-53: within 1.7 2^-53 in all.
+__device__ __forceinline__ double rsqrt_normal(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+// 1 / x for |x| from 2^-1000 to 2^1000: the hardware's approximation (2^-19 again) and one step of Chebyshev's method
+// for 1 / y = x, y (1 + e + e^2) with e = 1 - x y.  Its remainder e^3 is below 2^-57: within 1.1 2^-53.
+__device__ __forceinline__ double rcp_normal(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
 // Programmatic dependent launch.  A plan is a chain of up to 800 short kernels; each is launched so that its
 // blocks may be set up while the one before drains, and waits at its first statement until that one has
 // completed and its writes are visible.  Every thread of every kernel launched so makes dep_wait its first

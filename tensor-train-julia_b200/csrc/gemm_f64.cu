@@ -38,12 +38,6 @@ constexpr int REF_BM = 64, REF_BN = 64;
 struct TileShape { int bm, bn; };
 constexpr TileShape kTiles[kGemmTiles] = {{64, 64}, {64, 32}, {32, 32}, {16, 16}};
 
-__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
-}
-
 // 8 bytes global -> shared; zero when !on (the address is not read)
 __device__ __forceinline__ void cp8(unsigned dst, const double* src, bool on) {
   const int sz = on ? 8 : 0;

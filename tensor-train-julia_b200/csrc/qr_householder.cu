@@ -44,20 +44,6 @@ namespace ttc {
 namespace {
 constexpr int NB = 16;
 
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// D += A B on the FP64 tensor-core path (mma.sync m8n8k4): per lane a = A[lane>>2][lane&3],
-// b = B[lane&3][lane>>2], d = D[lane>>2][2(lane&3) + {0,1}].
-__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
-}
-
 __device__ __forceinline__ void cluster_arrive() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
 }
@@ -87,24 +73,6 @@ __device__ __forceinline__ void store2(const double (&v)[2], double* col, int r,
 }
 __device__ __forceinline__ bool vec_ok(const double* p, int ld, int mp) {
   return ((reinterpret_cast<uintptr_t>(p) & 15) == 0) && (((ld | mp) & 1) == 0);
-}
-
-// 1 / sqrt(x) for normal positive x below 2^1000: the hardware's approximation (relative error below
-// 2^-19) and one step of the third-order iteration y (1 + e/2 + 3 e^2 / 8), e = 1 - x y^2 (Householder's
-// method), whose remainder 5 e^3 / 16 is below 2^-55: four dependent operations.
-__device__ __forceinline__ double rsqrt_normal(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-(x * y), y, 1.0);
-  return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-// 1 / x for normal x away from the ends of the range: the hardware's approximation and y (1 + e + e^2),
-// e = 1 - x y (remainder e^3).
-__device__ __forceinline__ double rcp_normal(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
 }
 
 // The reflectors V of a panel in shared memory: column l at l * panel_ld(mp), its rows in groups of

@@ -57,12 +57,6 @@ constexpr int kU = kW + NW / 2 * 256;    // NW/2*128  and their -U
 constexpr int kP = kU + NW / 2 * 128;    // panel, panel_ld x NB
 extern __shared__ double sm[];
 
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
 // Block-wide sum; `red` holds NW doubles.  All threads get the result.
 __device__ double block_sum(double v, double* red) {
   v = warp_sum(v);
@@ -99,14 +93,6 @@ __device__ __forceinline__ void panel_load(double* P, const double* __restrict__
   asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
 __device__ __forceinline__ void panel_wait() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-// D += A B on the FP64 tensor-core path (mma.sync m8n8k4): per lane a = A[lane>>2][lane&3],
-// b = B[lane&3][lane>>2], d = D[lane>>2][2(lane&3) + {0,1}].
-__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
-}
 
 // T of a panel from T^{-1} + T^{-T} = V^T V (compact WY): T^{-1} = striu(G) + diag(1/tau), so
 // T[r][j] = -tau_r sum_{r < l <= j} G[r][l] T[l][j], T[j][j] = tau_j; lane j of the

@@ -53,12 +53,6 @@ constexpr int NW = NT / 32;
 // a few hundred, and the iteration would never stop.
 __device__ __forceinline__ double jac_tol(int m) { return (double)(m > 16 ? m : 16) * 2.220446049250313e-16; }
 
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
 struct Rot { double c, s, t; bool apply; };   // t = s / c (= s rsqrt(c^2): no division)
 
 // Parameters shared by all rotations of one problem.
@@ -253,12 +247,6 @@ __device__ __forceinline__ void gather_cols(double* __restrict__ dst, int dld, c
 __device__ __forceinline__ void scatter_cols(double* __restrict__ dst, long long ld, const double* __restrict__ src,
                                              int sld, const int* idx, int rows, int cols) {
   for (int c = threadIdx.x >> 5; c < cols; c += NW) copy_col_warp(dst + (long long)idx[c] * ld, src + (long long)c * sld, rows);
-}
-
-__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
 }
 
 // Screening of a block pair in the later sweeps: whether any column pair (a of block I, b of
@@ -561,15 +549,6 @@ __device__ __forceinline__ void cp_async8(double* dst, const double* src) {
 __device__ __forceinline__ void cp_async16(double* dst, const double* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
-}
-
-// 1 / sqrt(x) for normal positive x: the hardware's approximation (relative error below 2^-19) and one
-// third-order step y (1 + e/2 + 3 e^2 / 8), e = 1 - x y^2 (Householder's method; remainder 5 e^3 / 16).
-__device__ __forceinline__ double rsqrt_normal(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-(x * y), y, 1.0);
-  return fma(y * e, fma(e, 0.375, 0.5), y);
 }
 
 // make_rot without branches on scaled values, for the inner rounds' critical path: a pair that does not

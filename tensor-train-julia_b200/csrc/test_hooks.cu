@@ -22,6 +22,11 @@ struct DevBuf {
   template <class T> T* as() const { return (T*)p; }
 };
 
+__global__ void reciprocals_kernel(int n, const double* x, double* rs, double* rc) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) { rs[i] = rsqrt_normal(x[i]); rc[i] = rcp_normal(x[i]); }
+}
+
 template <class F>
 int hook(ttc_context* c, F&& f) {
   try {
@@ -82,6 +87,20 @@ int ttc_test_grad_keep(ttc_context* c, long long bytes, long long* ws_bytes) {
 // (default 2^24), so that a test can make the waits run out on purpose.
 int ttc_test_set_tc_wait_limit(ttc_context* c, long long polls) {
   return hook(c, [&] { set_tc_wait_limit(polls); });
+}
+
+// rs[i] = rsqrt_normal(x[i]), rc[i] = rcp_normal(x[i]).
+int ttc_test_reciprocals(ttc_context* c, int n, const double* x, double* rs, double* rc) {
+  return hook(c, [&] {
+    DevBuf d((size_t)n * 24);
+    TTC_CUDA(cudaMemcpy(d.p, x, (size_t)n * 8, cudaMemcpyHostToDevice));
+    TTC_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+    reciprocals_kernel<<<(n + 255) / 256, 256, 0, c->stream>>>(n, d.as<double>(), d.as<double>() + n, d.as<double>() + 2 * n);
+    TTC_CHECK_LAUNCH();
+    TTC_CUDA(cudaStreamSynchronize(c->stream));
+    TTC_CUDA(cudaMemcpy(rs, d.as<double>() + n, (size_t)n * 8, cudaMemcpyDeviceToHost));
+    TTC_CUDA(cudaMemcpy(rc, d.as<double>() + 2 * n, (size_t)n * 8, cudaMemcpyDeviceToHost));
+  });
 }
 
 // Device-resident timing of the tcgen05 GEMM C = A B^T (M x N, K; BF16 operands, or FP32 read as

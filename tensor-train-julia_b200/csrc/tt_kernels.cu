@@ -8,11 +8,6 @@ namespace ttc {
 namespace {
 constexpr int NT = 256;
 
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
 }  // namespace
 
 // ---------------------------------------------------------------- strided copy
