@@ -176,7 +176,7 @@ void batch_upload_many(ttc_batch* b, int first, int m, const ttc_ttv* xs, bool r
   CopyDesc* hc = (CopyDesc*)(h + off_desc);
   int* hr = (int*)(h + off_rk);
   size_t o = 0, ci = 0;
-  long long maxe = 0;
+  ElemCount elems;
   std::vector<HostCopy> hcp;
   for (int i = 0; i < m; ++i) {
     const ttc_ttv& x = xs[i];
@@ -192,7 +192,7 @@ void batch_upload_many(ttc_batch* b, int first, int m, const ttc_ttv* xs, bool r
         hc[ci++] = cd3((const double*)(d) + o, b->core(t, k), n, r0, r1, 1, n, n * r0, cap0, 1, cap0 * n);
       else
         hc[ci++] = cd3((const double*)(d) + o, b->core(t, k), n, r0, r1, 1, n, n * r0, cap0, cap0 * n, 1);
-      maxe = std::max<long long>(maxe, (long long)cnt);
+      elems.add((long long)cnt);
       o += cnt;
     }
     for (int k = 0; k <= N; ++k) hr[(size_t)i * (N + 1) + k] = (int)x.rks[reverse ? N - k : k];
@@ -220,7 +220,7 @@ void batch_upload_many(ttc_batch* b, int first, int m, const ttc_ttv* xs, bool r
     }
   }
   TTC_CUDA(cudaMemcpyAsync(d + off_desc, h + off_desc, total - off_desc, cudaMemcpyHostToDevice, c->stream));
-  launch_copy((const CopyDesc*)(d + off_desc), (int)ci, maxe, c->stream);
+  launch_copy((const CopyDesc*)(d + off_desc), (int)ci, elems, c->stream);
   TTC_CUDA(cudaMemcpyAsync(b->drk(first, 0), d + off_rk, (size_t)m * (N + 1) * sizeof(int), cudaMemcpyDeviceToDevice,
                            c->stream));
   TTC_CUDA(cudaMemsetAsync(b->d_zero + first, 0, sizeof(int) * m, c->stream));
@@ -269,7 +269,7 @@ void batch_download_many(ttc_batch* b, int first, int m, ttc_ttv_out* ys, bool r
   unsigned char* d = (unsigned char*)c->d_stage;
   CopyDesc* hc = (CopyDesc*)(h + off_desc);
   size_t o = 0, ci = 0;
-  long long maxe = 0;
+  ElemCount elems;
   std::vector<size_t> offs;
   for (int i = 0; i < m; ++i) {
     const int t = first + i;
@@ -281,13 +281,13 @@ void batch_download_many(ttc_batch* b, int first, int m, ttc_ttv_out* ys, bool r
         hc[ci++] = cd3(b->core(t, k), dst, n, r0, r1, cap0, 1, cap0 * n, 1, n, n * r0);
       else  // output (i, a, b) with a < r1, b < r0 from internal (b, i, a)
         hc[ci++] = cd3(b->core(t, k), dst, n, r1, r0, cap0, cap0 * n, 1, 1, n, n * r1);
-      maxe = std::max<long long>(maxe, n * r0 * r1);
+      elems.add(n * r0 * r1);
       offs.push_back(o);
       if (!direct) o += (size_t)n * r0 * r1;
     }
   }
   TTC_CUDA(cudaMemcpyAsync(d + off_desc, h + off_desc, nd * sizeof(CopyDesc), cudaMemcpyHostToDevice, c->stream));
-  launch_copy((const CopyDesc*)(d + off_desc), (int)ci, maxe, c->stream);
+  launch_copy((const CopyDesc*)(d + off_desc), (int)ci, elems, c->stream);
   if (direct) {
     TTC_CUDA(cudaStreamSynchronize(c->stream));
   } else {

@@ -53,7 +53,7 @@ DevTTO* tto_upload(ttc_context* c, const ttc_tto* H) {
   ensure_stage(c, sizeof(double) * o + 256 + sizeof(CopyDesc) * N);
   double* hs = (double*)c->h_stage;
   std::vector<CopyDesc> cp;
-  long long maxe = 0;
+  ElemCount elems;
   for (int k = 0; k < N; ++k) {
     const long long n = D->dims[k], R0 = D->rks[k], R1 = D->rks[k + 1];
     const long long cnt = n * n * R0 * R1;
@@ -66,12 +66,12 @@ DevTTO* tto_upload(ttc_context* c, const ttc_tto* H) {
     d.ds[0] = R0; d.ds[1] = R0 * n; d.ds[2] = 1; d.ds[3] = R0 * n * n;
     d.alpha = 1.0;
     cp.push_back(d);
-    maxe = std::max(maxe, cnt);
+    elems.add(cnt);
   }
   const size_t doff = ((size_t)o * sizeof(double) + 255) & ~size_t(255);
   std::memcpy((unsigned char*)c->h_stage + doff, cp.data(), cp.size() * sizeof(CopyDesc));
   TTC_CUDA(cudaMemcpyAsync(c->d_stage, c->h_stage, doff + cp.size() * sizeof(CopyDesc), cudaMemcpyHostToDevice, c->stream));
-  launch_copy((const CopyDesc*)((unsigned char*)c->d_stage + doff), N, maxe, c->stream);
+  launch_copy((const CopyDesc*)((unsigned char*)c->d_stage + doff), N, elems, c->stream);
   TTC_CUDA(cudaStreamSynchronize(c->stream));
   return D.release();
 }

@@ -4,14 +4,30 @@
 
 namespace ttc {
 
-// Blocks per problem of an element-wise launch over `count` problems (the grid's y dimension) of at most
-// max_elems elements, per_block a block: two waves of the chip's resident blocks over the whole launch, each
-// thread striding over its problem.  One block per per_block elements of the largest problem, whatever the
-// count, started up to 4 million blocks, most of them with nothing to do: the operand conversion of 60
-// sketches (3689 problems) 830 us, 262 so with its transposes in tiles.
-inline unsigned elem_blocks(long long max_elems, int per_block, int count) {
-  const long long fit = (max_elems + per_block - 1) / per_block, share = 148LL * 16 / (count > 0 ? count : 1);
-  return (unsigned)(fit < 1 || share < 1 ? 1 : fit < share ? fit : share);
+// Elements of an element-wise launch's problems: the largest, and all together.
+struct ElemCount {
+  long long max = 0, total = 0;
+  void add(long long n) {
+    max = n > max ? n : max;
+    total += n;
+  }
+};
+// Blocks per problem of an element-wise launch over `count` problems (the grid's y dimension) on nsm SMs; a
+// block takes per_block elements at least, its threads striding over the problem.  Sixteen blocks per SM (two
+// waves of the resident ones) are shared among the problems: of problems alike each gets as many.  A problem
+// much larger than the others gets up to sixteen, as far as its part of the elements goes, also where a share
+// by number is less; every other one starts as many, most of them with nothing to do.  The element-wise launches
+// of a rounding of one train of rank 700 and 1400 of rank 2 (d 22): one block per problem 14.7 ms, sixteen 2.1,
+// 32 2.2, 64 3.3; of one of rank 300 and 1400 of rank 2 (d 20) 3.6, 1.3, 1.7, 2.5; with 90 or 200 small ones the
+// same.  One block per per_block elements of the largest problem, whatever the count, started up to 4 million:
+// 16.9 and 6.8 ms, and the operand conversion of 60 sketches (3689 problems) 830 us, 262 so with its transposes
+// in tiles.
+inline unsigned elem_blocks(const ElemCount& e, int per_block, int count, int nsm) {
+  const double part = 16.0 * nsm * (double)e.max / (double)(e.total > 0 ? e.total : 1);
+  const long long fit = (e.max + per_block - 1) / per_block, like = 16LL * nsm / (count > 0 ? count : 1);
+  const long long share = (long long)part, most = like > 16 ? like : 16;
+  const long long b = fit < share ? fit : share;
+  return (unsigned)(b < 1 ? 1 : b < most ? b : most);
 }
 
 // ---- grouped FP64 GEMM (gemm_f64.cu)
@@ -120,7 +136,7 @@ struct SelectDesc {
   int scale;                 // 1: divide by sigma; 0: copy; 2: multiply by sigma
   int zrows;                 // when above rows: rows [rows, zrows) of every output column are zeroed
 };
-void launch_select(const SelectDesc* d, int count, int max_rows, int max_cols, cudaStream_t s);
+void launch_select(const SelectDesc* d, int count, const ElemCount& e, cudaStream_t s);
 
 // ---- general strided copy / permute of up to 4-D tensors (tt_kernels.cu)
 // dst[i0*ds0 + i1*ds1 + i2*ds2 + i3*ds3] = alpha * src[i0*ss0 + ...] for i < ext.
@@ -131,11 +147,11 @@ struct CopyDesc {
   long long ds[4];
   double alpha;
 };
-void launch_copy(const CopyDesc* d, int count, long long max_elems, cudaStream_t s);
+void launch_copy(const CopyDesc* d, int count, const ElemCount& e, cudaStream_t s);
 
 // Zero a set of flat ranges.
 struct ZeroDesc { double* p; long long n; };
-void launch_zero(const ZeroDesc* d, int count, long long max_n, cudaStream_t s);
+void launch_zero(const ZeroDesc* d, int count, const ElemCount& e, cudaStream_t s);
 
 // Sum of squares of `n` doubles per problem, written to out[i] (FP64, deterministic order).
 struct NormDesc { const double* p; long long n; double* out; };

@@ -57,9 +57,9 @@ __global__ void final_kernel(const FinalDesc* descs) {
   if (blockIdx.x == 0)
     for (int i = threadIdx.x; i < D.nrks; i += blockDim.x) D.rks[i] = D.rks_restore[i];
 }
-void launch_final(const FinalDesc* d, int count, long long max_n, cudaStream_t s) {
+void launch_final(const FinalDesc* d, int count, const ElemCount& e, cudaStream_t s) {
   if (count <= 0) return;
-  launch_dep(final_kernel, dim3(elem_blocks(max_n, 256, count), (unsigned)count), 256, 0, s, d);
+  launch_dep(final_kernel, dim3(elem_blocks(e, 256, count, current_sm_count()), (unsigned)count), 256, 0, s, d);
   TTC_CHECK_LAUNCH();
 }
 
@@ -99,9 +99,9 @@ __global__ void cvt_f32_kernel(const CvtDesc* descs) {
   float* dst = reinterpret_cast<float*>(D.dst);
   each_elem(D, [&](long long from, long long to) { dst[to] = (float)(D.alpha * D.src[from]); });
 }
-void launch_cvt_f32(const CvtDesc* d, int count, long long max_elems, cudaStream_t s) {
-  if (count <= 0 || max_elems <= 0) return;
-  launch_dep(cvt_f32_kernel, dim3(elem_blocks(max_elems, 256, count), (unsigned)count), 256, 0, s, d);
+void launch_cvt_f32(const CvtDesc* d, int count, const ElemCount& e, cudaStream_t s) {
+  if (count <= 0 || e.max <= 0) return;
+  launch_dep(cvt_f32_kernel, dim3(elem_blocks(e, 256, count, current_sm_count()), (unsigned)count), 256, 0, s, d);
   TTC_CHECK_LAUNCH();
 }
 __global__ void widen_kernel(const CvtDesc* descs) {
@@ -111,9 +111,9 @@ __global__ void widen_kernel(const CvtDesc* descs) {
   double* dst = reinterpret_cast<double*>(D.dst);
   each_elem(D, [&](long long from, long long to) { dst[to] = D.alpha * (double)src[from]; });
 }
-void launch_widen(const CvtDesc* d, int count, long long max_elems, cudaStream_t s) {
-  if (count <= 0 || max_elems <= 0) return;
-  launch_dep(widen_kernel, dim3(elem_blocks(max_elems, 256, count), (unsigned)count), 256, 0, s, d);
+void launch_widen(const CvtDesc* d, int count, const ElemCount& e, cudaStream_t s) {
+  if (count <= 0 || e.max <= 0) return;
+  launch_dep(widen_kernel, dim3(elem_blocks(e, 256, count, current_sm_count()), (unsigned)count), 256, 0, s, d);
   TTC_CHECK_LAUNCH();
 }
 
@@ -148,10 +148,11 @@ __global__ void __launch_bounds__(256) cvt_bf16_kernel(const CvtDesc* descs) {
   }
   each_elem(D, [&](long long from, long long to) { dst[to] = cvt(D.src[from]); });
 }
-void launch_cvt_bf16(const CvtDesc* d, int count, long long max_elems, cudaStream_t s, bool f32) {
-  if (count <= 0 || max_elems <= 0) return;
-  if (f32) launch_dep(cvt_bf16_kernel<float>, dim3(elem_blocks(max_elems, 1024, count), (unsigned)count), 256, 0, s, d);
-  else launch_dep(cvt_bf16_kernel<__nv_bfloat16>, dim3(elem_blocks(max_elems, 1024, count), (unsigned)count), 256, 0, s, d);
+void launch_cvt_bf16(const CvtDesc* d, int count, const ElemCount& e, cudaStream_t s, bool f32) {
+  if (count <= 0 || e.max <= 0) return;
+  const dim3 grid(elem_blocks(e, 1024, count, current_sm_count()), (unsigned)count);
+  if (f32) launch_dep(cvt_bf16_kernel<float>, grid, 256, 0, s, d);
+  else launch_dep(cvt_bf16_kernel<__nv_bfloat16>, grid, 256, 0, s, d);
   TTC_CHECK_LAUNCH();
 }
 
@@ -185,21 +186,21 @@ static void launch_op(ttc_context* c, const Plan& p, const Op& op) {
         launch_jacobi((const JacobiDesc*)d, op.count, op.a, op.b, op.total != 0, s, c->d_flags, op.iw, (int)op.rmax);
         break;
       case OP_TRUNC: launch_truncate((const TruncDesc*)d, op.count, op.tol, op.rmax, s); break;
-      case OP_SELECT: launch_select((const SelectDesc*)d, op.count, op.a, op.b, s); break;
-      case OP_COPY: launch_copy((const CopyDesc*)d, op.count, op.total, s); break;
-      case OP_ZERO: launch_zero((const ZeroDesc*)d, op.count, op.total, s); break;
+      case OP_SELECT: launch_select((const SelectDesc*)d, op.count, op.elems, s); break;
+      case OP_COPY: launch_copy((const CopyDesc*)d, op.count, op.elems, s); break;
+      case OP_ZERO: launch_zero((const ZeroDesc*)d, op.count, op.elems, s); break;
       case OP_SUMSQ: launch_sumsq((const NormDesc*)d, op.count, s); break;
       case OP_APPLY: launch_apply((const ApplyDesc*)d, op.count, op.a, op.b, s); break;
       case OP_GEMM32: launch_gemm_f32((const GemmDesc*)d, op.count, op.total, op.a, s); break;
-      case OP_CVT32: launch_cvt_f32((const CvtDesc*)d, op.count, op.total, s); break;
-      case OP_WIDEN: launch_widen((const CvtDesc*)d, op.count, op.total, s); break;
+      case OP_CVT32: launch_cvt_f32((const CvtDesc*)d, op.count, op.elems, s); break;
+      case OP_WIDEN: launch_widen((const CvtDesc*)d, op.count, op.elems, s); break;
       case OP_PHILOX: launch_philox((const PhiloxDesc*)d, op.count, op.total, s); break;
       case OP_BF16GEMM: launch_gemm_bf16_tc((const Bf16GemmDesc*)d, op.count, op.total, s, c->d_flags, op.a != 0); break;
       case OP_ZEROCHK: launch_zerochk((const ZeroChkDesc*)d, op.count, s); break;
       case OP_PINV_SCALE: launch_pinv_scale((const PinvScaleDesc*)d, op.count, s); break;
-      case OP_FINAL: launch_final((const FinalDesc*)d, op.count, op.total, s); break;
+      case OP_FINAL: launch_final((const FinalDesc*)d, op.count, op.elems, s); break;
       case OP_SETRANK: launch_setrank((const SetRankDesc*)d, op.count, s); break;
-      case OP_CVT_BF16: launch_cvt_bf16((const CvtDesc*)d, op.count, op.total, s, op.a != 0); break;
+      case OP_CVT_BF16: launch_cvt_bf16((const CvtDesc*)d, op.count, op.elems, s, op.a != 0); break;
       case OP_STAGE: TTC_CUDA(cudaEventRecord(c->ev[op.a], s)); break;
     }
   }
@@ -501,28 +502,28 @@ void Builder::gemm32(std::vector<GemmDesc> v) {
 }
 void Builder::cvt_f32(const std::vector<CvtDesc>& v) {
   if (v.empty()) return;
-  long long mx = 0;
+  ElemCount e;
   for (auto& d : v) {
-    mx = std::max(mx, d.rows * d.cols);
+    e.add(d.rows * d.cols);
     if (wsbase) {
       region_check(d.src, 8 * (size_t)sp2(d.rows, d.ss_i, d.cols, d.ss_j), "cvt32 src");
       region_check(d.dst, 4 * (size_t)sp2(d.rows, d.ds_i, d.cols, d.ds_j), "cvt32 dst");
     }
   }
-  Op op; op.kind = OP_CVT32; op.off = plan->push(v); op.count = (int)v.size(); op.total = mx;
+  Op op; op.kind = OP_CVT32; op.off = plan->push(v); op.count = (int)v.size(); op.total = e.max; op.elems = e;
   plan->ops.push_back(op);
 }
 void Builder::widen(const std::vector<CvtDesc>& v) {
   if (v.empty()) return;
-  long long mx = 0;
+  ElemCount e;
   for (auto& d : v) {
-    mx = std::max(mx, d.rows * d.cols);
+    e.add(d.rows * d.cols);
     if (wsbase) {
       region_check(d.src, 4 * (size_t)sp2(d.rows, d.ss_i, d.cols, d.ss_j), "widen src");
       region_check(d.dst, 8 * (size_t)sp2(d.rows, d.ds_i, d.cols, d.ds_j), "widen dst");
     }
   }
-  Op op; op.kind = OP_WIDEN; op.off = plan->push(v); op.count = (int)v.size(); op.total = mx;
+  Op op; op.kind = OP_WIDEN; op.off = plan->push(v); op.count = (int)v.size(); op.total = e.max; op.elems = e;
   plan->ops.push_back(op);
 }
 void Builder::qr(const std::vector<QRDesc>& v, bool sequential) {
@@ -606,9 +607,11 @@ void Builder::trunc(const std::vector<TruncDesc>& v, double tol, long long rmax)
 void Builder::select(const std::vector<SelectDesc>& v) {
   if (v.empty()) return;
   int mr = 0, mc = 0;
+  ElemCount e;
   for (auto& d : v) {
     const int rows = std::max(d.rows, d.zrows);
     mr = std::max(mr, rows); mc = std::max(mc, d.cols);
+    e.add((long long)rows * d.cols);
     const bool on = wsbase != nullptr;
     chk(on, d.X, (long long)d.ldx * (d.src_cols - 1) + d.rows, 8, "select X");
     chk(on, d.sigma, d.src_cols, 8, "select sigma");
@@ -617,12 +620,12 @@ void Builder::select(const std::vector<SelectDesc>& v) {
     chk(on, d.U, (long long)d.ldu * (d.cols - 1) + rows, 8, "select U");
     TTC_REQUIRE(d.ldx >= d.rows && d.ldu >= rows, TTC_EINTERNAL, "select: leading dims");
   }
-  Op op; op.kind = OP_SELECT; op.off = plan->push(v); op.count = (int)v.size(); op.a = mr; op.b = mc;
+  Op op; op.kind = OP_SELECT; op.off = plan->push(v); op.count = (int)v.size(); op.a = mr; op.b = mc; op.elems = e;
   plan->ops.push_back(op);
 }
 void Builder::copy(const std::vector<CopyDesc>& v) {
   std::vector<CopyDesc> w;
-  long long mx = 0;
+  ElemCount e;
   for (auto& d : v) {
     const long long n = d.ext[0] * d.ext[1] * d.ext[2] * d.ext[3];
     if (n <= 0) continue;
@@ -630,22 +633,22 @@ void Builder::copy(const std::vector<CopyDesc>& v) {
       region_check(d.src, 8 * (size_t)span_elems(d.ext, d.ss, 4), "copy src");
       region_check(d.dst, 8 * (size_t)span_elems(d.ext, d.ds, 4), "copy dst");
     }
-    mx = std::max(mx, n);
+    e.add(n);
     w.push_back(d);
   }
   if (w.empty()) return;
-  Op op; op.kind = OP_COPY; op.off = plan->push(w); op.count = (int)w.size(); op.total = mx;
+  Op op; op.kind = OP_COPY; op.off = plan->push(w); op.count = (int)w.size(); op.total = e.max; op.elems = e;
   plan->ops.push_back(op);
 }
 void Builder::zero(const std::vector<ZeroDesc>& v) {
   std::vector<ZeroDesc> w;
-  long long mx = 0;
+  ElemCount e;
   for (auto& d : v) if (d.n > 0) {
     chk(wsbase != nullptr, d.p, d.n, 8, "zero");
-    w.push_back(d); mx = std::max(mx, d.n);
+    w.push_back(d); e.add(d.n);
   }
   if (w.empty()) return;
-  Op op; op.kind = OP_ZERO; op.off = plan->push(w); op.count = (int)w.size(); op.total = mx;
+  Op op; op.kind = OP_ZERO; op.off = plan->push(w); op.count = (int)w.size(); op.total = e.max; op.elems = e;
   plan->ops.push_back(op);
 }
 void Builder::sumsq(const std::vector<NormDesc>& v) {
@@ -718,15 +721,15 @@ void Builder::bf16gemm(std::vector<Bf16GemmDesc> v, bool tf32) {
 }
 void Builder::cvt_bf16(const std::vector<CvtDesc>& v, bool f32) {
   if (v.empty()) return;
-  long long mx = 0;
+  ElemCount e;
   for (auto& d : v) {
-    mx = std::max(mx, d.rows * d.cols);
+    e.add(d.rows * d.cols);
     if (wsbase) {
       region_check(d.src, 8 * (size_t)sp2(d.rows, d.ss_i, d.cols, d.ss_j), "cvt src");
       region_check(d.dst, (f32 ? 4 : 2) * (size_t)sp2(d.rows, d.ds_i, d.cols, d.ds_j), "cvt dst");
     }
   }
-  Op op; op.kind = OP_CVT_BF16; op.off = plan->push(v); op.count = (int)v.size(); op.total = mx; op.a = f32;
+  Op op; op.kind = OP_CVT_BF16; op.off = plan->push(v); op.count = (int)v.size(); op.total = e.max; op.elems = e; op.a = f32;
   plan->ops.push_back(op);
 }
 void Builder::pinv_scale(const std::vector<PinvScaleDesc>& v) {
@@ -746,16 +749,16 @@ void Builder::zerochk(const std::vector<ZeroChkDesc>& v) {
 }
 void Builder::finalize(const std::vector<FinalDesc>& v) {
   if (v.empty()) return;
-  long long mx = 0;
+  ElemCount e;
   for (auto& d : v) {
-    mx = std::max(mx, d.n);
+    e.add(d.n);
     const bool on = wsbase != nullptr;
     chk(on, d.cores, d.n, 8, "final cores");
     chk(on, d.rks, d.nrks, 4, "final rks");
     chk(on, d.rks_restore, d.nrks, 4, "final rks src");
     chk(on, d.flag, 1, 4, "final flag");
   }
-  Op op; op.kind = OP_FINAL; op.off = plan->push(v); op.count = (int)v.size(); op.total = mx;
+  Op op; op.kind = OP_FINAL; op.off = plan->push(v); op.count = (int)v.size(); op.total = e.max; op.elems = e;
   plan->ops.push_back(op);
 }
 void Builder::setrank(const std::vector<SetRankDesc>& v) {

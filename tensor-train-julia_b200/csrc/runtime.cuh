@@ -32,7 +32,8 @@ struct Op {
   OpKind kind;
   size_t off = 0;      // byte offset of the descriptors in the plan blob
   int count = 0;       // number of descriptors
-  long long total = 0; // tiles (GEMM) or max elements (streaming kernels)
+  long long total = 0; // tiles (GEMM), or elements of the largest problem
+  ElemCount elems;     // streaming kernels
   int a = 0, b = 0;    // kernel-specific (max_m, max_n, stage id ...)
   double tol = 0.0;
   long long rmax = 0;
@@ -59,15 +60,15 @@ struct CvtDesc { const double* src; void* dst; long long rows, cols, ss_i, ss_j,
 struct PinvScaleDesc { double* X; int ldx; int m, n; const double* sigma; double eps; };
 void launch_pinv_scale(const PinvScaleDesc* d, int count, cudaStream_t s);
 void launch_zerochk(const ZeroChkDesc* d, int count, cudaStream_t s);
-void launch_final(const FinalDesc* d, int count, long long max_n, cudaStream_t s);
+void launch_final(const FinalDesc* d, int count, const ElemCount& e, cudaStream_t s);
 void launch_setrank(const SetRankDesc* d, int count, cudaStream_t s);
 // FP64 -> BF16 (f32 = false) or FP64 -> FP32 rounded to TF32 (f32 = true), same index map.
-void launch_cvt_bf16(const CvtDesc* d, int count, long long max_elems, cudaStream_t s, bool f32 = false);
+void launch_cvt_bf16(const CvtDesc* d, int count, const ElemCount& e, cudaStream_t s, bool f32 = false);
 // FP64 -> FP32 (round to nearest), same index map.
-void launch_cvt_f32(const CvtDesc* d, int count, long long max_elems, cudaStream_t s);
+void launch_cvt_f32(const CvtDesc* d, int count, const ElemCount& e, cudaStream_t s);
 // FP32 -> FP64: dst (double) from src holding floats, same index map (CvtDesc with the roles of the
 // pointers swapped: `src` points to floats, `dst` to doubles).
-void launch_widen(const CvtDesc* d, int count, long long max_elems, cudaStream_t s);
+void launch_widen(const CvtDesc* d, int count, const ElemCount& e, cudaStream_t s);
 
 struct Plan {
   std::vector<unsigned char> blob;

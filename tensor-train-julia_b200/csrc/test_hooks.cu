@@ -89,6 +89,14 @@ int ttc_test_set_tc_wait_limit(ttc_context* c, long long polls) {
   return hook(c, [&] { set_tc_wait_limit(polls); });
 }
 
+// Blocks per problem of an element-wise launch (host only).
+int ttc_test_elem_blocks(long long max_elems, long long total_elems, int per_block, int count, int nsm) {
+  ElemCount e;
+  e.max = max_elems;
+  e.total = total_elems;
+  return (int)elem_blocks(e, per_block, count, nsm);
+}
+
 // rs[i] = rsqrt_normal(x[i]), rc[i] = rcp_normal(x[i]).
 int ttc_test_reciprocals(ttc_context* c, int n, const double* x, double* rs, double* rc) {
   return hook(c, [&] {

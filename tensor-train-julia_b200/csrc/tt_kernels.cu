@@ -70,10 +70,10 @@ __global__ void __launch_bounds__(NT) copy4_kernel(const CopyDesc* __restrict__ 
   }
 }
 
-void launch_copy(const CopyDesc* d, int count, long long max_elems, cudaStream_t s) {
-  if (count <= 0 || max_elems <= 0) return;
+void launch_copy(const CopyDesc* d, int count, const ElemCount& e, cudaStream_t s) {
+  if (count <= 0 || e.max <= 0) return;
   // about four elements per thread; with `count` copies in the grid's y dimension
-  dim3 grid(elem_blocks(max_elems, 4 * NT, count), (unsigned)count);
+  dim3 grid(elem_blocks(e, 4 * NT, count, current_sm_count()), (unsigned)count);
   launch_dep(copy4_kernel, grid, NT, 0, s, d);
   TTC_CHECK_LAUNCH();
 }
@@ -89,9 +89,9 @@ __global__ void zero_kernel(const ZeroDesc* __restrict__ descs) {
   }
 }
 
-void launch_zero(const ZeroDesc* d, int count, long long max_n, cudaStream_t s) {
-  if (count <= 0 || max_n <= 0) return;
-  launch_dep(zero_kernel, dim3(elem_blocks(max_n, 4 * NT, count), (unsigned)count), NT, 0, s, d);
+void launch_zero(const ZeroDesc* d, int count, const ElemCount& e, cudaStream_t s) {
+  if (count <= 0 || e.max <= 0) return;
+  launch_dep(zero_kernel, dim3(elem_blocks(e, 4 * NT, count, current_sm_count()), (unsigned)count), NT, 0, s, d);
   TTC_CHECK_LAUNCH();
 }
 
@@ -197,10 +197,9 @@ __global__ void select_kernel(const SelectDesc* __restrict__ descs) {
   }
 }
 
-void launch_select(const SelectDesc* d, int count, int max_rows, int max_cols, cudaStream_t s) {
+void launch_select(const SelectDesc* d, int count, const ElemCount& e, cudaStream_t s) {
   if (count <= 0) return;
-  const long long total = (long long)max_rows * max_cols;
-  launch_dep(select_kernel, dim3(elem_blocks(total, NT, count), (unsigned)count), NT, 0, s, d);
+  launch_dep(select_kernel, dim3(elem_blocks(e, NT, count, current_sm_count()), (unsigned)count), NT, 0, s, d);
   TTC_CHECK_LAUNCH();
 }
 
