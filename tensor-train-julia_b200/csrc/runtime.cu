@@ -859,12 +859,21 @@ void block_trim(ttc_context* c) noexcept {
   c->blocks.held = 0;
 }
 
+// cudaMalloc, or the out-of-memory status that a test has asked for
+static cudaError_t try_malloc(ttc_context* c, void** p, size_t bytes) {
+  if (c->fail_count > 0 && --c->fail_after < 0) {
+    --c->fail_count;
+    return cudaErrorMemoryAllocation;
+  }
+  return cudaMalloc(p, bytes);
+}
+
 cudaError_t dev_malloc(ttc_context* c, void** p, size_t bytes) {
-  cudaError_t e = cudaMalloc(p, bytes);
+  cudaError_t e = try_malloc(c, p, bytes);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
     block_trim(c);
-    e = cudaMalloc(p, bytes);
+    e = try_malloc(c, p, bytes);
   }
   if (e != cudaSuccess) { cudaGetLastError(); *p = nullptr; }
   return e;
@@ -967,7 +976,8 @@ void check_device_flags(ttc_context* c) {
 // ---------------------------------------------------------------- batches
 ttc_batch* batch_create(ttc_context* c, int count, int N, const long long* dims, const int* cap, bool pooled) {
   TTC_REQUIRE(count > 0 && N > 0, TTC_EARG, "batch: count and N must be positive");
-  std::unique_ptr<ttc_batch> b(new ttc_batch());
+  // destroyed, with what it holds by then, when a later step fails
+  std::unique_ptr<ttc_batch, void (*)(ttc_batch*)> b(new ttc_batch(), batch_destroy);
   b->ctx = c; b->count = count; b->N = N;
   b->pooled = pooled;
   b->dims.assign(dims, dims + N);

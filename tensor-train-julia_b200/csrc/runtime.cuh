@@ -130,6 +130,7 @@ struct ttc_context {
   // batch identity, replay the captured plan
   std::vector<std::pair<std::string, ttc_batch*>> oneshot;
   ttc::BlockPool blocks;
+  int fail_after = 0, fail_count = 0;   // set by tests: fail_count allocation attempts fail, fail_after from now
   size_t grad_keep = 0;              // bytes up to which a gradient keeps every site's environments
 };
 

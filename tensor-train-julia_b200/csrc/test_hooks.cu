@@ -83,6 +83,21 @@ int ttc_test_grad_keep(ttc_context* c, long long bytes, long long* ws_bytes) {
   });
 }
 
+// Lets `count` attempts of the context to allocate device memory fail (a status on the host; nothing is
+// allocated), the first one after `after` others.
+int ttc_test_fail_alloc(ttc_context* c, int after, int count) {
+  return hook(c, [&] { c->fail_after = after; c->fail_count = count; });
+}
+
+// Device blocks of the one-shot calls: bytes idle, and blocks in use.
+int ttc_test_blocks(ttc_context* c, long long* idle_bytes, int* in_use) {
+  return hook(c, [&] {
+    std::lock_guard<std::mutex> lk(c->blocks.mu);
+    *idle_bytes = (long long)c->blocks.held;
+    *in_use = (int)c->blocks.cap.size();
+  });
+}
+
 // Sets the poll limit of the tensor-core GEMM's bounded mbarrier waits on the context's device
 // (default 2^24), so that a test can make the waits run out on purpose.
 int ttc_test_set_tc_wait_limit(ttc_context* c, long long polls) {
