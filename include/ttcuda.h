@@ -141,6 +141,10 @@ int ttc_set_profiling(ttc_context* ctx, int on);
 int ttc_create(ttc_context** ctx, int device);
 int ttc_destroy(ttc_context* ctx);
 int ttc_set_stream(ttc_context* ctx, void* cuda_stream);
+/* Gives the device memory that the context keeps between one-shot calls (at most 512 MiB of idle
+ * blocks) back to the driver.  Allocations of any context on the device do so by themselves when
+ * memory runs out; other users of the device in the process (a CUDA.jl or torch pool) cannot. */
+int ttc_trim(ttc_context* ctx);
 const char* ttc_last_error(const ttc_context* ctx);
 int ttc_get_stats(const ttc_context* ctx, ttc_stats* out);
 int ttc_synchronize(ttc_context* ctx);

@@ -67,13 +67,17 @@ Plan* get_plan(ttc_context* c, const std::string& key, const std::function<void(
 size_t plan_workspace(ttc_context* c, const std::function<void(Builder&)>& fn);
 void run_plan(ttc_context* c, Plan& p);
 void ensure_workspace(ttc_context* c, size_t bytes);
-// cudaMalloc that gives the context's idle blocks back and tries once more when memory runs out.
+// cudaMalloc that gives the idle blocks of every context on the device back and tries once more when memory
+// runs out.
 cudaError_t dev_malloc(ttc_context* c, void** p, size_t bytes);
 // A device block for the duration of one call, from the context's idle blocks where one fits, and its
 // return (waits for the context's stream).  block_trim frees every idle block.
 cudaError_t block_get(ttc_context* c, void** p, size_t bytes);
 void block_put(ttc_context* c, void* p) noexcept;
 void block_trim(ttc_context* c) noexcept;
+// The contexts whose idle blocks dev_malloc can give back: from creation to destruction.
+void context_add(ttc_context* c);
+void context_remove(ttc_context* c) noexcept;
 void check_device_flags(ttc_context* c);
 
 ttc_batch* batch_create(ttc_context* c, int count, int N, const long long* dims, const int* cap, bool pooled = true);

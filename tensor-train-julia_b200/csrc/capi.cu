@@ -458,6 +458,7 @@ int ttc_create(ttc_context** out, int device) {
     size_t free_bytes = 0, total_bytes = 0;
     TTC_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
     c->grad_keep = total_bytes / 8;
+    context_add(c);
   });
   if (st != TTC_OK) {
     g_err_noctx = c->err;
@@ -470,6 +471,7 @@ int ttc_create(ttc_context** out, int device) {
 
 int ttc_destroy(ttc_context* c) {
   if (!c) return TTC_OK;
+  context_remove(c);
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   c->plans.clear();
@@ -489,6 +491,11 @@ int ttc_destroy(ttc_context* c) {
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return TTC_OK;
+}
+
+int ttc_trim(ttc_context* c) {
+  if (!c) return TTC_EARG;
+  return guard(c, [&] { block_trim(c); });
 }
 
 int ttc_set_stream(ttc_context* c, void* stream) {

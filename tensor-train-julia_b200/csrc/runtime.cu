@@ -846,10 +846,23 @@ Plan* get_plan(ttc_context* c, const std::string& key, const std::function<void(
 // of a block of a megabyte or more map and unmap memory, 100 to 300 us a pair and tens of milliseconds
 // where the driver gives back a large mapping: of a dot and a partial contraction at ranks 128 x 77
 // (6.2 ms) they took 2.7 ms, of a gradient at r 192 (20 ms at best, 60 at times) 5 to 50.  Blocks of that
-// size are kept by their context, up to kPoolBytes together, and freed with it or when memory runs out;
-// smaller ones come out of the driver's own 2 MB slabs at 2 us and stay with cudaMalloc.
+// size are kept by their context, up to kPoolBytes together, and freed with it, by ttc_trim, or when memory runs
+// out for any context on the device; smaller ones come out of the driver's own 2 MB slabs at 2 us and stay with
+// cudaMalloc.
 namespace {
 constexpr size_t kPoolMin = 1u << 20, kPoolBytes = 512u << 20;
+std::mutex g_contexts_mu;
+std::vector<ttc_context*> g_contexts;        // those that may hold idle blocks
+}
+
+void context_add(ttc_context* c) {
+  std::lock_guard<std::mutex> lk(g_contexts_mu);
+  g_contexts.push_back(c);
+}
+
+void context_remove(ttc_context* c) noexcept {
+  std::lock_guard<std::mutex> lk(g_contexts_mu);
+  g_contexts.erase(std::remove(g_contexts.begin(), g_contexts.end(), c), g_contexts.end());
 }
 
 void block_trim(ttc_context* c) noexcept {
@@ -872,7 +885,11 @@ cudaError_t dev_malloc(ttc_context* c, void** p, size_t bytes) {
   cudaError_t e = try_malloc(c, p, bytes);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    block_trim(c);
+    {
+      std::lock_guard<std::mutex> lk(g_contexts_mu);
+      for (ttc_context* o : g_contexts)
+        if (o->device == c->device) block_trim(o);
+    }
     e = try_malloc(c, p, bytes);
   }
   if (e != cudaSuccess) { cudaGetLastError(); *p = nullptr; }

@@ -154,6 +154,10 @@ class Context:
     def synchronize(self):
         self.check(lib.ttc_synchronize(self.h))
 
+    def trim(self):
+        """Give the device memory kept between one-shot calls (at most 512 MiB) back to the driver."""
+        self.check(lib.ttc_trim(self.h))
+
     def set_stream(self, cuda_stream_handle: int):
         """Run subsequent calls on an existing CUDA stream (e.g. torch's cuda_stream handle)."""
         self.check(lib.ttc_set_stream(self.h, C.c_void_p(cuda_stream_handle)))

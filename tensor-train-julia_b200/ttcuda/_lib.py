@@ -64,6 +64,7 @@ _SIGS = {
     "ttc_get_stats": (i32, [vp, C.POINTER(Stats)]),
     "ttc_set_profiling": (i32, [vp, C.c_int]),
     "ttc_synchronize": (i32, [vp]),
+    "ttc_trim": (i32, [vp]),
     "ttc_batch_create": (i32, [vp, i32, i32, P_i64, P_i64, C.POINTER(vp)]),
     "ttc_batch_destroy": (i32, [vp]),
     "ttc_batch_upload": (i32, [vp, i32, C.POINTER(TTV)]),

@@ -38,3 +38,36 @@ def test_failed_call_gives_its_blocks_back(after, monkeypatch):
     ctx.check(lib.ttc_test_fail_alloc(ctx.h, 0, 0))
     assert blocks(ctx)[1] == in_use
     assert ttcuda.dot(x, y) == want
+
+
+def idle_context(monkeypatch, ranks=(300,)):
+    ctx = ttcuda.Context(0)
+    monkeypatch.setattr(ttcuda, "_CTX", ctx)
+    for r in ranks:
+        ttcuda.dot(train(r), train(r + 10))
+    assert blocks(ctx)[0] > 0
+    return ctx
+
+
+def test_idle_blocks_of_every_context_go_when_memory_runs_out(monkeypatch):
+    """One attempt of another context to allocate fails: the call succeeds at the second one, and no context of
+    the device holds an idle block from before it."""
+    a, b, c = idle_context(monkeypatch), idle_context(monkeypatch), idle_context(monkeypatch)
+    x, y = train(500), train(510)                      # larger than any idle block
+    c.check(lib.ttc_test_fail_alloc(c.h, 0, 1))
+    got = ttcuda.dot(x, y)
+    assert blocks(a) == (0, 0) and blocks(b) == (0, 0)
+    assert got == ttcuda.dot(x, y)
+
+
+def test_trim(monkeypatch):
+    ctx = idle_context(monkeypatch)
+    ctx.trim()
+    assert blocks(ctx) == (0, 0)
+    assert np.isfinite(ttcuda.dot(train(300), train(310)))
+
+
+def test_idle_blocks_stay_within_their_bound(monkeypatch):
+    """0.8 GB of operands of growing size, none of which fits a block that is idle."""
+    ctx = idle_context(monkeypatch, range(300, 1000, 70))
+    assert blocks(ctx)[0] <= 512 << 20
