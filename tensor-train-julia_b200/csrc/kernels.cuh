@@ -77,7 +77,9 @@ struct QRDesc {
   double* Rt; int ldrt;   // optional second copy of R, transposed: R^T[j][i] at Rt[i*ldrt + j]
 };
 constexpr int QR_MAX_M = 1536;
-void launch_qr(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, int* d_flags);
+// dependent: as a plan's launches (launch_dep); false on a caller's stream, whose capture would take the
+// programmatic edge that this makes into the caller's graph, and then cannot list its edges (cuGraphGetEdges).
+void launch_qr(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, int* d_flags, bool dependent = true);
 // The same factorisation with every sum over all rows in one order (qr_sequential.cu).
 void launch_qr_seq(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, int* d_flags);
 

@@ -97,7 +97,7 @@ extern "C" int ttc_qr_noalloc(int32_t m, int32_t n, const double* A, int64_t lda
     ttc::QRDesc d{m, n, work, m, Q, (int)ldq, R, (int)ldr, tws};
     qrna_prepare<<<1, 32, 0, s>>>(d, ddesc, flag);
     TTC_CHECK_LAUNCH();
-    ttc::launch_qr(ddesc, 1, m, s, flag);
+    ttc::launch_qr(ddesc, 1, m, s, flag, false);
     return TTC_OK;
   } catch (const ttc::Error& e) {
     ttc::set_noctx_error(e.what());

@@ -656,7 +656,7 @@ void launch_qr_apply_t(const QApplyDesc* d_descs, int count, int max_m, cudaStre
 }
 
 template <int NW>
-void launch_qr_t(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, int* d_flags) {
+void launch_qr_t(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, int* d_flags, bool dependent) {
   constexpr int lim = NW <= 8 ? kSmallM : QR_MAX_M;
   const size_t smem = qr_smem<NW>(max_m);
   static PerDeviceOnce attr_once;
@@ -689,7 +689,7 @@ void launch_qr_t(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, in
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = dependent ? 2 : 1;
   TTC_CUDA(cudaLaunchKernelEx(&cfg, householder_qr_kernel<NW>, d_descs, csize, d_flags));
   TTC_CHECK_LAUNCH();
 }
@@ -702,14 +702,14 @@ void launch_qr_apply(const QApplyDesc* d_descs, int count, int max_m, cudaStream
   else launch_qr_apply_t<16>(d_descs, count, max_m, s);
 }
 
-void launch_qr(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, int* d_flags) {
+void launch_qr(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, int* d_flags, bool dependent) {
   if (count <= 0) return;
   TTC_REQUIRE(max_m <= QR_MAX_M, TTC_EDIM, "qr: row count exceeds the supported maximum (1536)");
   // Launches of few problems (every CTA has an SM to itself) and panels beyond 256 rows take sixteen
   // warps: one problem 512 x 256 with Q 468 us (584 with eight), 276 x 138 203 (213), 256 x 256 363 (320)
   const bool alone = max_m > 256 && 8LL * count <= current_sm_count();
-  if (max_m <= kSmallM && !alone) launch_qr_t<8>(d_descs, count, max_m, s, d_flags);
-  else launch_qr_t<16>(d_descs, count, max_m, s, d_flags);
+  if (max_m <= kSmallM && !alone) launch_qr_t<8>(d_descs, count, max_m, s, d_flags, dependent);
+  else launch_qr_t<16>(d_descs, count, max_m, s, d_flags, dependent);
 }
 
 }  // namespace ttc
