@@ -292,6 +292,36 @@ int ttc_test_qr_seq(ttc_context* c, int m, int n, const double* A, double* Q, do
   return test_qr(c, m, n, A, Q, R, true);
 }
 
+// `count` problems of ttc_test_qr, one after another in A, Q and R, in one launch; mb, nb >= 0: rows from mult * mb
+// and columns from mult * nb on are zero, which the kernel reads from the device; tall > 0: beside one
+// more problem, of zeros, of that many rows.
+int ttc_test_qr_many(ttc_context* c, int count, int m, int n, const double* A, double* Q, double* R, int mb, int nb, int mult,
+                     int sequential, int tall) {
+  return hook(c, [&] {
+    const int K = std::min(m, n), Kt = std::min(tall, n);
+    const size_t a = (size_t)m * n, q = (size_t)m * K, r = (size_t)K * n, tw = (size_t)((std::max(K, Kt) + 15) / 16 + 1) * 256;
+    DevBuf dA(a * count * 8), dQ(q * count * 8), dR(r * count * 8), dT(tw * (count + 1) * 8), dB(8);
+    DevBuf tA((size_t)tall * n * 8), tQ((size_t)tall * Kt * 8), tR((size_t)Kt * n * 8);
+    TTC_CUDA(cudaMemcpy(dA.p, A, a * count * 8, cudaMemcpyHostToDevice));
+    const int bounds[2] = {mb, nb};
+    TTC_CUDA(cudaMemcpy(dB.p, bounds, 8, cudaMemcpyHostToDevice));
+    run_plan_once(c, [&](Builder& B) {
+      std::vector<QRDesc> v;
+      for (int i = 0; i < count; ++i) {
+        QRDesc d{m, n, dA.as<double>() + a * i, m, dQ.as<double>() + q * i, m, dR.as<double>() + r * i, K, dT.as<double>() + tw * i};
+        if (mb >= 0) { d.m_dev = dB.as<int>(); d.m_mult = mult; }
+        if (nb >= 0) { d.n_dev = dB.as<int>() + 1; d.n_mult = mult; }
+        v.push_back(d);
+      }
+      if (tall > 0)
+        v.push_back({tall, n, tA.as<double>(), tall, tQ.as<double>(), tall, tR.as<double>(), Kt, dT.as<double>() + tw * count});
+      B.qr(v, sequential != 0);
+    });
+    TTC_CUDA(cudaMemcpy(Q, dQ.p, q * count * 8, cudaMemcpyDeviceToHost));
+    TTC_CUDA(cudaMemcpy(R, dR.p, r * count * 8, cudaMemcpyDeviceToHost));
+  });
+}
+
 // One-sided Jacobi of X (m x n): X <- X W (orthogonal columns), sigma, perm; W if accw.
 // *sweeps receives the sweeps used (negative when the cap was hit; not raised as an error here).
 int ttc_test_jacobi(ttc_context* c, int m, int n, double* X, int accw, double* W, double* sigma, int* perm,
