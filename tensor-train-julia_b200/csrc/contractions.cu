@@ -1026,10 +1026,10 @@ void rayleigh_grad_host(ttc_context* c, const ttc_tto* Hh, const ttc_ttv* x, int
   };
   // What the first plan leaves lies in the workspace, which therefore has to be large enough for both before
   // the first one runs: the second one's K splits can need more of it (d 32, r 132, R 8: 94 MB against 88).
-  ensure_workspace(c, std::max(plan_workspace(c, chains), plan_workspace(c, products)));
+  ensure_workspace(c, plan_workspace(c, products));
   ensure_stage(c, sizeof(double) * gsz + 256);        // the gradient in the caller's layout
-  const size_t ws_bytes = c->ws_bytes;
   run_once(c, chains);
+  const size_t ws_bytes = c->ws_bytes;
   double hv[2];
   TTC_CUDA(cudaMemcpy(hv, dval, 2 * sizeof(double), cudaMemcpyDeviceToHost));
   nn = hv[1];
