@@ -42,13 +42,13 @@ METRIC = "TT roundings/s at d=32,r=256: mixed vs FP64 GPU at 1e-8 rel err; % roo
 # (dram__bytes_read.sum + dram__bytes_write.sum) of smaller cases of the same kernels, scaled to a
 # 64-TT launch by the problems it holds (the factors stay in L2 within a launch, so a launch reads
 # its inputs once and traffic grows with the problem count):
-#  * householder_qr_kernel: 7.57 MB for a 32-TT orthogonalisation-sweep launch at bond 12
-#    (unfoldings up to 512 x 256) -> 15.1 MB for 64 TTs;
-#  * jacobi_svd (the Gram-block kernel): 33.75 MB for 64 preconditioned 256 x 256 factors
+#  * householder_qr_kernel: 7.90 MB for a 32-TT orthogonalisation-sweep launch at bond 12
+#    (unfoldings up to 512 x 256) -> 15.8 MB for 64 TTs;
+#  * jacobi_svd (the Gram-block kernel): 34.37 MB for 64 preconditioned 256 x 256 factors
 #    (bench.py --jacobi-bench), the largest launch of the SVD sweep.
 DOMINANT_DRAM_BYTES_PER_LAUNCH_64TT = {
-    "householder_qr": (15.1e6, "ncu capture of a 32-TT orthogonalisation-sweep QR launch (bond 12), x2 for 64 TTs"),
-    "jacobi_svd": (33.75e6, "ncu capture of a 64-problem 256 x 256 launch (bench.py --jacobi-bench), the largest"),
+    "householder_qr": (15.8e6, "ncu capture of a 32-TT orthogonalisation-sweep QR launch (bond 12), x2 for 64 TTs"),
+    "jacobi_svd": (34.37e6, "ncu capture of a 64-problem 256 x 256 launch (bench.py --jacobi-bench), the largest"),
 }
 
 

@@ -27,8 +27,9 @@
 // the scalars of a reflector (one reciprocal square root and one reciprocal, no branch) are computed
 // while the dot products are reduced.  Cycles per column step on one SM, with a square root and two
 // divisions in every warp and the columns in shared memory before: 64 rows 2020, now 790; 256 rows
-// 2290 and 1020; 512 rows 5600 and 1600.  One problem with Q: 128 x 64 126 us before and 69 now,
-// 256 x 256 530 and 320, 512 x 256 870 and 468; the QRs of a 60-TT rounding 36.7 and 24.6 ms.
+// 2290 and 1020; 512 rows 5600 and 1600.  One problem with Q: 128 x 64 126 us before and 65 now,
+// 256 x 256 530 and 293, 512 x 256 870 and 446; the QR family of a 64-TT rounding 32.9
+// and 20.7 ms.
 // The rest is the trailing update and the Q formation, on 8-column octets held in registers from the
 // first product to the second (read and written once; 0.33 and 0.52 of 2.5 M cycles for 512 x 256
 // before, 0.14 and 0.17 now).
@@ -706,7 +707,7 @@ void launch_qr(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, int*
   if (count <= 0) return;
   TTC_REQUIRE(max_m <= QR_MAX_M, TTC_EDIM, "qr: row count exceeds the supported maximum (1536)");
   // Launches of few problems (every CTA has an SM to itself) and panels beyond 256 rows take sixteen
-  // warps: one problem 512 x 256 with Q 468 us (584 with eight), 276 x 138 203 (213), 256 x 256 363 (320)
+  // warps: one problem 512 x 256 with Q 446 us (454 with eight), 276 x 138 184 (183), 256 x 256 316 (293)
   const bool alone = max_m > 256 && 8LL * count <= current_sm_count();
   if (max_m <= kSmallM && !alone) launch_qr_t<8>(d_descs, count, max_m, s, d_flags, dependent);
   else launch_qr_t<16>(d_descs, count, max_m, s, d_flags, dependent);

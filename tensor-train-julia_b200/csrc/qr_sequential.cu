@@ -7,7 +7,7 @@
 // sites), and its trailing Q columns follow the rounding of every sum to eight digits.  The kernel of
 // qr_householder.cu, which shares a column's rows between warps, gives there another, equally accurate
 // basis (1.7e-8 from the 64-bit result's either way, 1e-8 from each other); this one returns the basis
-// that results of these roundings were stored with.  It costs 243 us for 276 x 138 with Q, the other 203.
+// that results of these roundings were stored with.  It costs 243 us for 276 x 138 with Q, the other 184.
 //
 // Every sum keeps its order whatever the split of the work: a change of the kernel must not move a bit.
 // What bounds it: the 16 column steps of a panel, 1300 cycles each at 276 rows (a barrier, a warp's sum over
