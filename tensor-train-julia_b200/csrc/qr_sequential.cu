@@ -55,7 +55,7 @@ constexpr int kTop = kG + NB * NB;       // NB*NB  R's part of the panel, top[co
 constexpr int kW = kTop + NB * NB;       // NW/2*256  the W of the octets in work
 constexpr int kU = kW + NW / 2 * 256;    // NW/2*128  and their -U
 constexpr int kP = kU + NW / 2 * 128;    // panel, panel_ld x NB
-extern __shared__ double sm[];
+extern __shared__ __align__(16) double sm[];   // T is read in pairs
 
 // Block-wide sum; `red` holds NW doubles.  All threads get the result.
 __device__ double block_sum(double v, double* red) {
