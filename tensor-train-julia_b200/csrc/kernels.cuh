@@ -58,6 +58,11 @@ __device__ __forceinline__ int dev_bound(int cap, const int* p, int mult) {
 
 // Dynamic shared memory that keeps a second CTA off an SM (227 KB at most per SM and CTA).
 constexpr size_t kLoneCtaSmem = 116 * 1024;
+// Clusters of csize CTAs of that size which the current device holds at once.  Fewer than its SMs have room for:
+// a cluster lies within one group of SMs, and what is left over of a group goes unused (of 148 SMs 15 clusters of
+// eight, 33 of four).  A launch of more clusters would run in two turns where CTAs share SMs in one: 16 Jacobi
+// problems of 256 x 256 2.43 ms alone on their SMs, 1.73 sharing, 35 of 128 x 128 0.96 and 0.65.
+int lone_clusters(int csize);
 
 // ---- batched Householder QR (qr_householder.cu)
 // A (m x n, col-major, lda) is overwritten.  Q (m x K, ldq) and R (K x n, ldr),

@@ -679,8 +679,8 @@ void launch_qr_t(const QRDesc* d_descs, int count, int max_m, cudaStream_t s, in
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(count * csize));
   cfg.blockDim = dim3(NW * 32);
-  // one CTA per SM while there are SMs for all
-  cfg.dynamicSmemBytes = count * csize <= current_sm_count() ? std::max(smem, kLoneCtaSmem) : smem;
+  // one CTA per SM while all clusters have room so
+  cfg.dynamicSmemBytes = count <= lone_clusters(csize) ? std::max(smem, kLoneCtaSmem) : smem;
   cfg.stream = s;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;

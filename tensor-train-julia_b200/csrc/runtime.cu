@@ -977,6 +977,36 @@ int current_sm_count() {
   return count[dev];
 }
 
+namespace {
+__global__ void lone_probe_kernel() {}
+}  // namespace
+
+int lone_clusters(int csize) {
+  static std::mutex mu;
+  static int held[kMaxDevices][9] = {};
+  int dev = 0;
+  TTC_CUDA(cudaGetDevice(&dev));
+  TTC_REQUIRE(dev >= 0 && dev < kMaxDevices && csize >= 1 && csize <= 8, TTC_EARG, "lone_clusters: device or cluster size");
+  std::lock_guard<std::mutex> lk(mu);
+  int& n = held[dev][csize];
+  if (n == 0) {
+    TTC_CUDA(cudaFuncSetAttribute(lone_probe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLoneCtaSmem));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)csize);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = kLoneCtaSmem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)csize;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    TTC_CUDA(cudaOccupancyMaxActiveClusters(&n, lone_probe_kernel, &cfg));
+  }
+  return n;
+}
+
 void check_device_flags(ttc_context* c) {
   int f = 0;
   TTC_CUDA(cudaMemcpyAsync(&f, c->d_flags, sizeof(int), cudaMemcpyDeviceToHost, c->stream));

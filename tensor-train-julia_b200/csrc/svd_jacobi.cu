@@ -1231,7 +1231,7 @@ static void launch_jacobi_block(const JacobiDesc* d_descs, int count, int max_m,
   // Launches that leave every CTA an SM of its own ask for more than half of an SM's shared memory:
   // otherwise two CTAs of a cluster may land on one SM and share its tensor cores (one 248 x 248 problem
   // 1.37 ms, 1.30 apart)
-  cfg.dynamicSmemBytes = (size_t)count * csize <= (size_t)current_sm_count() ? std::max(smem, kLoneCtaSmem) : smem;
+  cfg.dynamicSmemBytes = count <= lone_clusters(csize) ? std::max(smem, kLoneCtaSmem) : smem;
   cfg.stream = s;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;

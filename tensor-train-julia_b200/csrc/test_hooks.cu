@@ -112,6 +112,14 @@ int ttc_test_elem_blocks(long long max_elems, long long total_elems, int per_blo
   return (int)elem_blocks(e, per_block, count, nsm);
 }
 
+// lone_clusters(csize), and the SMs of the context's device.
+int ttc_test_lone_clusters(ttc_context* c, int csize, int* clusters, int* sms) {
+  return hook(c, [&] {
+    *clusters = lone_clusters(csize);
+    *sms = current_sm_count();
+  });
+}
+
 // rs[i] = rsqrt_normal(x[i]), rc[i] = rcp_normal(x[i]).
 int ttc_test_reciprocals(ttc_context* c, int n, const double* x, double* rs, double* rc) {
   return hook(c, [&] {
