@@ -215,17 +215,23 @@ __global__ void __launch_bounds__(WM * WN * 32, MINB) gemm_f64_grouped_kernel(co
     __syncthreads();
     if (!s_last) return;
     __threadfence();
+    // a row of fragments at a time, the loads of several splits in flight (its own partial is read back as well)
 #pragma unroll
-    for (int i = 0; i < FM; ++i)
+    for (int i = 0; i < FM; ++i) {
+      double v[FN][2] = {};
+#pragma unroll 4
+      for (int s2 = 0; s2 < ks; ++s2) {
+        const double* from = slots + (long long)s2 * (BM * BN) + i * FN * 2 * NT;
+#pragma unroll
+        for (int j = 0; j < FN; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) v[j][e] += __ldcg(from + (j * 2 + e) * NT);
+      }
 #pragma unroll
       for (int j = 0; j < FN; ++j)
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int o = ((i * FN + j) * 2 + e) * NT;
-          double v = 0.0;
-          for (int s2 = 0; s2 < ks; ++s2) v += (s2 == split) ? acc[i][j][e] : __ldcg(slots + (long long)s2 * (BM * BN) + o);
-          acc[i][j][e] = v;
-        }
+        for (int e = 0; e < 2; ++e) acc[i][j][e] = v[j][e];
+    }
     if (tid == 0) D.cnt[lt] = 0u;   // zero again for the next launch of the plan
   }
   if (!busy) return;
