@@ -35,8 +35,10 @@ constexpr int BK = 16;
 // the tile that the K splits are counted in
 constexpr int REF_BM = 64, REF_BN = 64;
 
-struct TileShape { int bm, bn; };
-constexpr TileShape kTiles[kGemmTiles] = {{64, 64}, {64, 32}, {32, 32}, {16, 16}};
+// bm x bn, the CTAs that an SM holds, and what a turn of n CTAs on an SM costs: once + n each (gemm_pick_tile)
+struct TileShape { int bm, bn, per_sm; double once, each; };
+constexpr TileShape kTiles[kGemmTiles] = {{64, 64, 3, 0.52, 1.0}, {64, 32, 3, 0.29, 0.55}, {32, 32, 6, 0.30, 0.35},
+                                          {16, 16, 8, 0.092, 0.18}};
 
 // 8 bytes global -> shared; zero when !on (the address is not read)
 __device__ __forceinline__ void cp8(unsigned dst, const double* src, bool on) {
@@ -314,27 +316,22 @@ long long gemm_split_ws_doubles(const GemmDesc& d, int tile) {
 }
 
 int gemm_pick_tile(const GemmDesc* d, int nd, int nsm) {
-  // The shape with the least time at one tile per SM and turn.  The costs are the times per output element
-  // of a launch that fills the chip, measured at 4096 x 4096 x 1024: 28.0, 26.5 and 20.5 TFLOP/s (a smaller
-  // tile loads more fragments and copies per product).  Sums over whole roundings, all launches at one
-  // shape against this rule (ms): operator rounding r 320 x R 64 16.8 / 18.1 / 20.5 against 15.9, r 128 x R 6
-  // 4.3 / 3.1 / 3.0 against 3.0, gradient 14.6 / 11.9 / 11.7 against 11.6, 60 ragged trains 6.2 / 5.6 / 5.7
-  // against 5.6.
-  constexpr double cost[3] = {1.0, 1.05, 1.3};
+  // The shape with the least time, for as many turns as the SMs' CTAs need.  A turn's time per K step grows with
+  // the CTAs on an SM, but from a part that one CTA alone pays as well (four warps do not fill an SM's tensor
+  // cores): fitted to 160 launches, 1 to 840 tiles of 64 x 64, K 64 to 10240, all four layouts, each shape timed.
+  // The choice is 1.2 % above the best shape on average and nowhere above the time of 64 x 64 tiles of eight
+  // warps; counting turns of one tile per SM by area alone was 3.8 % above it, 20 to 37 % for 112 to 148 tiles
+  // (700^3 55 -> 45 us, transposed 66 -> 48; eight 1000 x 60 x 1000 88 -> 71).
   int best = 0;
   double best_t = 0.0;
-  long long tiles = 0;
-  for (int t = 0; t < 3; ++t) {
-    tiles = 0;
+  for (int t = 0; t < kGemmTiles; ++t) {
+    const TileShape& T = kTiles[t];
+    long long tiles = 0;
     for (int i = 0; i < nd; ++i) tiles += gemm_tiles(d[i], t);
-    const double turns = (double)((tiles + nsm - 1) / nsm) * kTiles[t].bm * kTiles[t].bn * cost[t];
-    if (t == 0 || turns < best_t) { best = t; best_t = turns; }
+    const long long per = (tiles + nsm - 1) / nsm, rest = per % T.per_sm;
+    const double time = (double)(per / T.per_sm) * (T.once + T.per_sm * T.each) + (rest ? T.once + (double)rest * T.each : 0.0);
+    if (t == 0 || time < best_t) { best = t; best_t = time; }
   }
-  // Launches of at most one 32 x 32 tile per SM wait for the instructions of the one warp on each scheduler
-  // (170 per K step, 6 cycles each), of which a 16 x 16 tile has half: operator rounding at r 128, R 6 8.40 ->
-  // 8.12 ms, a dot and a partial contraction 2.57 -> 2.39, three rank-5 trains rounded 1.370 -> 1.338.  Eight
-  // warps per tile 8.23, 2.51, 1.355; 16 x 32 tiles 8.25, 2.44, 1.362; up to two tiles per SM the same.
-  if (best == 2 && tiles <= nsm) best = 3;
   return best;
 }
 

@@ -112,6 +112,14 @@ int ttc_test_elem_blocks(long long max_elems, long long total_elems, int per_blo
   return (int)elem_blocks(e, per_block, count, nsm);
 }
 
+// The tile shape that a launch of `count` equal FP64 problems takes on nsm SMs (host only).
+int ttc_test_gemm_tile(int m, int n, int k, int batch, int count, int nsm) {
+  GemmDesc d{};
+  d.m = m; d.n = n; d.k = k; d.batch = batch;
+  d.ksplit = gemm_pick_ksplit(d, gemm_tiles(d, kGemmRefTile) * count, nsm);
+  return gemm_pick_tile(std::vector<GemmDesc>((size_t)count, d).data(), count, nsm);
+}
+
 // lone_clusters(csize), and the SMs of the context's device.
 int ttc_test_lone_clusters(ttc_context* c, int csize, int* clusters, int* sms) {
   return hook(c, [&] {
