@@ -847,10 +847,11 @@ Plan* get_plan(ttc_context* c, const std::string& key, const std::function<void(
 // where the driver gives back a large mapping: of a dot and a partial contraction at ranks 128 x 77
 // (6.2 ms) they took 2.7 ms, of a gradient at r 192 (20 ms at best, 60 at times) 5 to 50.  Blocks of that
 // size are kept by their context, up to kPoolBytes together, and freed with it, by ttc_trim, or when memory runs
-// out for any context on the device; smaller ones come out of the driver's own 2 MB slabs at 2 us and stay with
-// cudaMalloc.
+// out for any context on the device.  Smaller ones come out of the driver's own 2 MB slabs at 2 us, but a slab
+// whose last block is freed is unmapped, and mapped again by the next call (a sum of two trains of 16 sites and
+// rank 48 after other calls: 1.1 ms a call, 0.4 with the slab held), so blocks from 32 KB on are kept as well.
 namespace {
-constexpr size_t kPoolMin = 1u << 20, kPoolBytes = 512u << 20;
+constexpr size_t kPoolMin = 32u << 10, kPoolLarge = 1u << 20, kPoolBytes = 512u << 20, kPoolBlocks = 128;
 std::mutex g_contexts_mu;
 std::vector<ttc_context*> g_contexts;        // those that may hold idle blocks
 }
@@ -901,7 +902,8 @@ cudaError_t block_get(ttc_context* c, void** p, size_t bytes) {
   *p = nullptr;
   size_t cap = std::max<size_t>(bytes, 16);
   if (cap >= kPoolMin) {
-    cap = (cap + (2u << 20) - 1) / (2u << 20) * (2u << 20);
+    const size_t unit = cap >= kPoolLarge ? 2u << 20 : kPoolMin;
+    cap = (cap + unit - 1) / unit * unit;
     std::lock_guard<std::mutex> lk(P.mu);
     auto best = P.idle.end();                  // the smallest that fits and wastes at most a quarter
     for (auto it = P.idle.begin(); it != P.idle.end(); ++it)
@@ -929,16 +931,22 @@ void block_put(ttc_context* c, void* p) noexcept {
   if (!p) return;
   BlockPool& P = c->blocks;
   region_remove(p);
-  const bool idle = cudaStreamSynchronize(c->stream) == cudaSuccess;   // nothing of the call still uses it
-  std::lock_guard<std::mutex> lk(P.mu);
-  auto it = P.cap.find(p);
-  const size_t cap = it == P.cap.end() ? 0 : it->second;
-  if (it != P.cap.end()) P.cap.erase(it);
-  if (!idle || cap == 0 || cap > kPoolBytes) {
+  size_t cap = 0;                              // 0: not one to be kept
+  {
+    std::lock_guard<std::mutex> lk(P.mu);
+    auto it = P.cap.find(p);
+    if (it != P.cap.end()) {
+      cap = it->second;
+      P.cap.erase(it);
+    }
+  }
+  // nothing of the call still uses a block that is kept
+  if (cap == 0 || cap > kPoolBytes || cudaStreamSynchronize(c->stream) != cudaSuccess) {
     cudaFree(p);
     return;
   }
-  while (P.held + cap > kPoolBytes) {
+  std::lock_guard<std::mutex> lk(P.mu);
+  while (P.held + cap > kPoolBytes || P.idle.size() >= kPoolBlocks) {
     P.held -= P.idle.front().cap;
     cudaFree(P.idle.front().p);
     P.idle.pop_front();

@@ -71,3 +71,20 @@ def test_idle_blocks_stay_within_their_bound(monkeypatch):
     """0.8 GB of operands of growing size, none of which fits a block that is idle."""
     ctx = idle_context(monkeypatch, range(300, 1000, 70))
     assert blocks(ctx)[0] <= 512 << 20
+
+
+def test_blocks_below_a_megabyte_are_kept(monkeypatch):
+    """Two operands of 213 KB: left to the driver, they may be the last of a slab, which each call then maps and
+    unmaps."""
+    ctx = ttcuda.Context(0)
+    monkeypatch.setattr(ttcuda, "_CTX", ctx)
+    x = train(48, 16)
+    size = sum(c.nbytes for c in x.ttv_vec)
+    assert 100 << 10 < size < 1 << 20
+    ttcuda.dot(x, x)
+    assert blocks(ctx)[0] >= 2 * size and blocks(ctx)[1] == 0
+    for r in range(8, 200, 2):
+        ttcuda.norm(train(r, 4))
+    held = blocks(ctx)[0]
+    ctx.trim()
+    assert 0 < held <= 512 << 20 and blocks(ctx) == (0, 0)
